@@ -107,7 +107,6 @@ struct Carver
 void drop_eam(fmdg_sys_t *s)
 {
     Geo &g = s->g;
-    g.eF = g.eFDD = g.erho = g.erhoDD = g.ephi = g.ephiDD = nullptr;
     g.pk_rho = g.pk_phi = g.pk_F = nullptr;
     g.pkf_rho = g.pkf_phi = g.pkf_F = g.pkf_pr = nullptr;
     g.pkd_rho = g.pkd_phi = nullptr;
@@ -283,8 +282,6 @@ extern "C" void fmdg_destroy(fmdg_sys_t *s)
     if (s->eam_borrowed) drop_eam(s);
     dfree(s, (void *)s->g.pairs); dfree(s, (void *)s->g.mass); dfree(s, (void *)s->g.eam_elem);
     dfree(s, (void *)s->g.pairf); dfree(s, (void *)s->g.paird);
-    dfree(s, (void *)s->g.eF); dfree(s, (void *)s->g.eFDD); dfree(s, (void *)s->g.erho);
-    dfree(s, (void *)s->g.erhoDD); dfree(s, (void *)s->g.ephi); dfree(s, (void *)s->g.ephiDD);
     dfree(s, (void *)s->g.pk_rho); dfree(s, (void *)s->g.pk_phi); dfree(s, (void *)s->g.pk_F);
     dfree(s, (void *)s->g.pkf_rho); dfree(s, (void *)s->g.pkf_phi); dfree(s, (void *)s->g.pkf_F);
     dfree(s, (void *)s->g.pkf_pr); dfree(s, (void *)s->g.pkd_rho); dfree(s, (void *)s->g.pkd_phi);
@@ -406,7 +403,9 @@ int fmdg_skin_scale(fmdg_sys_t *s)
     if (s->rsk > 0.0)
     {
         g.rskin2 = (float)(s->rsk * xs * s->rsk * xs);
-        g.half_skin2 = (float)(0.25 * s->skin * s->skin * xs * xs);
+        g.half_skin2 = (float)(0.25 * s->skin_used * s->skin_used * xs * xs);
+        const double rc = (s->rsk - s->skin_used) * xs;
+        g.rcut2 = (float)(rc * rc * (1.0 + 2e-5));
     }
     const int nk2 = s->nkinds * s->nkinds;
     if (nk2 > 0 && g.pairf)
@@ -444,20 +443,7 @@ extern "C" int fmdg_set_eam(fmdg_sys_t *s, int nelem, int Nrho, double drho, int
     if (nelem < 1 || nelem > FMDG_MAXE || Nrho < 3 || Nr2 < 3) return fmdg_set_error("fmdg_set_eam: bad sizes");
     Geo &g = s->g;
     if (s->eam_borrowed) drop_eam(s);
-    dfree(s, (void *)g.eF); dfree(s, (void *)g.eFDD); dfree(s, (void *)g.erho);
-    dfree(s, (void *)g.erhoDD); dfree(s, (void *)g.ephi); dfree(s, (void *)g.ephiDD);
-    const size_t nF = (size_t)nelem * Nrho, nR = (size_t)nelem * Nr2, nP = (size_t)nelem * nelem * Nr2;
     int rc;
-    if ((rc = dalloc(s, (double **)&g.eF, nF)) || (rc = dalloc(s, (double **)&g.eFDD, nF)) ||
-        (rc = dalloc(s, (double **)&g.erho, nR)) || (rc = dalloc(s, (double **)&g.erhoDD, nR)) ||
-        (rc = dalloc(s, (double **)&g.ephi, nP)) || (rc = dalloc(s, (double **)&g.ephiDD, nP)))
-        return rc;
-    FMDG_CK(cudaMemcpyAsync((void *)g.eF, F, nF * 8, cudaMemcpyHostToDevice, s->stream));
-    FMDG_CK(cudaMemcpyAsync((void *)g.eFDD, F_DD, nF * 8, cudaMemcpyHostToDevice, s->stream));
-    FMDG_CK(cudaMemcpyAsync((void *)g.erho, rho, nR * 8, cudaMemcpyHostToDevice, s->stream));
-    FMDG_CK(cudaMemcpyAsync((void *)g.erhoDD, rhoDD, nR * 8, cudaMemcpyHostToDevice, s->stream));
-    FMDG_CK(cudaMemcpyAsync((void *)g.ephi, phi, nP * 8, cudaMemcpyHostToDevice, s->stream));
-    FMDG_CK(cudaMemcpyAsync((void *)g.ephiDD, phiDD, nP * 8, cudaMemcpyHostToDevice, s->stream));
     g.nelem = nelem; g.Nrho = Nrho; g.Nr2 = Nr2; g.drho = drho; g.dr2 = dr2;
     g.inv_dr2 = 1.0 / dr2;
     g.inv_drho = 1.0 / drho;
@@ -557,7 +543,7 @@ int fmdg_list_capacity(const fmdg_sys_t *s, const int *cell_count, int ncell)
         const double hmin = fmin(g.cellh[0], fmin(g.cellh[1], g.cellh[2]));
         rc2max = hmin * hmin;
     }
-    const double rlist = sqrt(rc2max) + (s->skin > 0.0 ? s->skin : 1e-2);
+    const double rlist = sqrt(rc2max) + (s->skin_used > 0.0 ? s->skin_used : 1e-2);
     if (s->list_capacity > 0) return s->list_capacity;
     return fmdg_capacity_estimate(cell_count, ncell, g.cellh[0] * g.cellh[1] * g.cellh[2], rlist);
 }
@@ -596,12 +582,35 @@ int fmdg_capacity_estimate(const int *cell_count, int ncell, double cell_volume,
     return maxnb;
 }
 
+// the thinnest default skin (A) a skin list is kept for
+static constexpr double MIN_SKIN = 0.02;
+
+// log2 of the shares V of a slot's list walk in the skin-list density and
+// force kernels: as many as keep n V within the thread target.  One thread
+// per slot leaves the chip idle below ~10^5 atoms, and its whole list is one
+// serial chain; beyond the target the lanes' sums and the extra blocks cost
+// more than they hide.  Measured on one GB300, us per step with 1 share ->
+// with V: single systems in binary64, argon 4000 atoms 146 -> 50 (V 16),
+// Morse 4004 320 -> 84 (16), EAM 2048 200 -> 64 (16), the 160 000-atom TTM
+// slab 820 -> 760 (2: 1250 blocks were 1.17 waves), EAM 256 000 580 at 1,
+// 640 at 2; single systems in mixed precision, argon 32 000 98 -> 93 (2),
+// 134 at 8; served jobs are bounded lower, as other jobs fill the chip.
+int fmdg_share_log(const fmdg_sys_t *s, int n)
+{
+    int target = s->g.prec == FMDG_PREC_FP64 ? 400000 : 1 << 16;
+    if (s->served) target = s->g.prec == FMDG_PREC_FP64 ? 1 << 14 : 1 << 13;
+    int l = 0;
+    while (l < 4 && ((long long)n << (l + 1)) <= target) l++;
+    return l;
+}
+
 // device bytes of a system with n atoms, ncell cells and list capacity maxnb
-size_t fmdg_bytes_estimate(int n, int ncell, int maxnb)
+size_t fmdg_bytes_estimate(int n, int ncell, int maxnb, int prec)
 {
     const size_t cap = n > 0 ? n : 1;
     const size_t per_atom = 2 * (48 + 16) + 32 + 7 * 4 + 16 + 4 + 4 * (size_t)maxnb + 9 * 8 / 64 + 8 + 24 +
-                            32;   // binary64 position rows (xdf)
+                            32 +  // binary64 position rows (xdf)
+                            (prec == FMDG_PREC_FP64 ? 4 * (size_t)maxnb + 64 : 0);   // pruned lists
     const size_t per_cell = 2 * 4 + 5 * 4 + 32;
     return cap * per_atom + (size_t)ncell * per_cell + 64 * 1024;
 }
@@ -631,14 +640,11 @@ extern "C" int fmdg_share_eam(fmdg_sys_t *s, const fmdg_sys_t *owner)
     Geo &g = s->g;
     if (!s->eam_borrowed)
     {
-        dfree(s, (void *)g.eF); dfree(s, (void *)g.eFDD); dfree(s, (void *)g.erho);
-        dfree(s, (void *)g.erhoDD); dfree(s, (void *)g.ephi); dfree(s, (void *)g.ephiDD);
         dfree(s, (void *)g.pk_rho); dfree(s, (void *)g.pk_phi); dfree(s, (void *)g.pk_F);
         dfree(s, (void *)g.pkf_rho); dfree(s, (void *)g.pkf_phi); dfree(s, (void *)g.pkf_F);
         dfree(s, (void *)g.pkf_pr); dfree(s, (void *)g.pkd_rho); dfree(s, (void *)g.pkd_phi);
     }
     const Geo &o = owner->g;
-    g.eF = o.eF; g.eFDD = o.eFDD; g.erho = o.erho; g.erhoDD = o.erhoDD; g.ephi = o.ephi; g.ephiDD = o.ephiDD;
     g.pk_rho = o.pk_rho; g.pk_phi = o.pk_phi; g.pk_F = o.pk_F;
     g.pkf_rho = o.pkf_rho; g.pkf_phi = o.pkf_phi; g.pkf_F = o.pkf_F; g.pkf_pr = o.pkf_pr;
     g.pkd_rho = o.pkd_rho; g.pkd_phi = o.pkd_phi;
@@ -695,29 +701,45 @@ extern "C" int fmdg_upload(fmdg_sys_t *s, int n, const int *cell_count, const do
     }
     const double rlist = sqrt(rc2max) + 1e-2;
     g.rlist2 = (float)(rlist * rlist);
-    const int maxnb = fmdg_list_capacity(s, cell_count, ncell);
-    g.maxnb = maxnb;
     for (int d3 = 0; d3 < 3; d3++)
     {
         g.cellh_f[d3] = (float)g.cellh[d3];
     }
     // a skin list needs the list radius below half of every periodic box
     // length (one image inside it) and within two cells; otherwise the
-    // exact stencil list is rebuilt every step
-    // (default: mixed precision only -- in binary64 mode the double-float
-    // pair arithmetic costs more on the longer list than the rebuilds save:
-    // EAM 256k 3.0e8 vs 3.5e8 atom-steps/s; LJ and Morse gain 7-8%)
-    g.skin_on = 0;
-    if (s->skin > 0.0 && cap < (1 << 25) && (s->skin_set || g.prec == FMDG_PREC_MIXED))
+    // exact stencil list is rebuilt every step.  The default skin shrinks to
+    // fit a short box (a thinner skin is rebuilt more often, which still
+    // costs less than the exact list of every step); a caller's is taken as
+    // it is.  Binary64 systems of several kinds keep the exact list, on which
+    // a list that overflows gives the same bits as one that does not.
+    double skin = s->skin;
+    if (!s->skin_set)
     {
-        const double rsk = sqrt(rc2max) + s->skin;
+        if (g.prec == FMDG_PREC_FP64 && s->nkinds > 1) skin = 0.0;
+        for (int d3 = 0; d3 < 3; d3++)
+            if (g.pbc[d3]) skin = fmin(skin, 0.9 * (0.5 * g.l[d3] - sqrt(rc2max)));
+        if (skin < MIN_SKIN) skin = 0.0;
+    }
+    g.skin_on = 0;
+    if (skin > 0.0 && cap < (1 << 25))
+    {
+        const double rsk = sqrt(rc2max) + skin;
         bool ok = rsk <= 2.0 * fmin(g.cellh[0], fmin(g.cellh[1], g.cellh[2]));
         for (int d3 = 0; d3 < 3; d3++)
             if (g.pbc[d3] && !(g.l[d3] > 2.0 * rsk)) ok = false;
         g.skin_on = ok;
     }
+    s->skin_used = g.skin_on ? skin : 0.0;
+    const int maxnb = fmdg_list_capacity(s, cell_count, ncell);
+    g.maxnb = maxnb;
     // partials for the smallest block size the tuner may pick (64)
-    const int nb = fmdg_grid(cap, 64);
+    g.share_log = g.lane_log = g.skin_on ? fmdg_share_log(s, cap) : 0;
+    const int nb = fmdg_grid(cap << g.share_log, 64);
+    // words of the pruned lists (binary64 mode; a single system may change
+    // its precision between runs)
+    const size_t shares = (size_t)1 << g.share_log;
+    const size_t pruned = (g.skin_on && !(s->served && g.prec == FMDG_PREC_MIXED))
+                        ? (size_t)cap * shares * 4 * fmdg_grid((maxnb + 3) / 4, (int)shares) : 0;
     auto layout = [&](Carver &c) {
         for (int k = 0; k < 2; k++)
         {
@@ -740,6 +762,7 @@ extern "C" int fmdg_upload(fmdg_sys_t *s, int n, const int *cell_count, const do
             c.take(g.pos, cap); c.take(g.cb, cap); c.take(g.xl, cap); c.take(g.xb, cap);
             c.take(g.xd, cap); c.take(g.gslot, cap); c.take(g.fpb, cap); c.take(g.fpd, cap);
             c.take(g.xll, cap);
+            c.take(g.nbc, pruned); c.take(g.nbc_count, pruned ? (size_t)cap * shares : 0);
         }
     };
     Carver measure{nullptr, 0};
@@ -760,7 +783,7 @@ extern "C" int fmdg_upload(fmdg_sys_t *s, int n, const int *cell_count, const do
         FMDG_CK(cudaMemcpyAsync(g.pos, iota.data(), (size_t)cap * 4, cudaMemcpyHostToDevice, st));
         // build cells: valid cell indexes before the first build writes them
         FMDG_CK(cudaMemsetAsync(g.cb, 0, (size_t)cap * 4, st));
-        const double rsk = sqrt(rc2max) + s->skin;
+        const double rsk = sqrt(rc2max) + s->skin_used;
         s->rsk = rsk;
         g.srad = 1;
         for (int d3 = 0; d3 < 3; d3++)

@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density(__gri
             else g.fpdf[i] = make_float2(0.f, 0.f);
         }
     }
-    block_reduce_store<1>(acc, g.partials + (size_t)nb * 8 + bx);
+    block_reduce_store<1>(acc, g.partials + (size_t)nb * 8 + bx, blockDim.x);
 }
 
 __global__ void k_reduce_final(Geo g, int nblocks, int keep_pe, int with_emb, int thermostat,
@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_force(__grid_
     }
     __shared__ double blk[7];
     __shared__ unsigned ticket;
-    block_reduce_store<7>(acc, blk);
+    block_reduce_store<7>(acc, blk, blockDim.x);
     if (threadIdx.x == 0)
     {
         for (int k = 0; k < 7; k++) g.partials[(size_t)k * nb + bx] = blk[k];
@@ -575,14 +575,17 @@ __global__ void __launch_bounds__(128) k_thermo(Geo g, int group)
         acc[5] = 1.0;
     }
     __shared__ double blk[6];
-    block_reduce_store<6>(acc, blk);
+    block_reduce_store<6>(acc, blk, blockDim.x);
     if (threadIdx.x == 0)
         for (int k = 0; k < 6; k++) g.partials[(size_t)k * gridDim.x + blockIdx.x] = blk[k];
 }
 
 } // namespace
 
-int fmdg_force_blocks(const fmdg_sys_t *s) { return fmdg_grid(s->g.cap > 0 ? s->g.cap : 1, s->fblk); }
+int fmdg_force_blocks(const fmdg_sys_t *s) 
+{
+    return fmdg_grid(s->g.cap > 0 ? s->g.cap << s->g.lane_log : 1, s->fblk);
+}
 
 namespace {
 
@@ -677,7 +680,7 @@ int fmdg_launch_forces(fmdg_sys_t *s, int group, int finish, double dt, int ther
 int fmdg_launch_thermo(fmdg_sys_t *s, int group, int thermostat, double dt, double tau, double T0)
 {
     Geo &g = s->g;
-    const int nb = fmdg_force_blocks(s);
+    const int nb = fmdg_grid(g.cap, 128);
     k_thermo<<<nb, 128, 0, s->stream>>>(g, group);
     k_reduce_final<<<1, 256, 0, s->stream>>>(g, nb, 1, 0, thermostat, dt, tau, T0);
     s->launches += 2;

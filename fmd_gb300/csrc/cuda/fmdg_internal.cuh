@@ -77,6 +77,7 @@ struct Geo   // passed by value to kernels
     int *nbr;          // nbr[k*cap + i] = j | (stencil offset code << 26)
     int *nbr_count;    // true count (entries beyond maxnb are not stored)
     int maxnb;
+    unsigned char share_log, lane_log;   // skin lists: log2 of the shares of a slot's walk and of its lanes (fmdg_skin.cu)
     float rlist2;      // binary32 prefilter radius^2 (largest cutoff + margin)
     float cellh_f[3];  // binary32 cell widths (remainders cellh - cellh_f formed per block)
     // packed spline tables: per interval k {y_k, y_k+1, y''_k, y''_k+1}
@@ -110,7 +111,6 @@ struct Geo   // passed by value to kernels
     const int *eam_elem;          // nkinds
     int nelem, Nrho, Nr2;
     double drho, dr2;
-    const double *eF, *eFDD, *erho, *erhoDD, *ephi, *ephiDD;
     int has_eam;
     int prec;
     // TTM friction term (src/forces.c:292-330), 1-D along z
@@ -139,8 +139,11 @@ struct Geo   // passed by value to kernels
     int *gslot;            // by slot: group
     float *fpb;            // by slot: F'(rho) binary32
     double *fpd;           // by slot: F'(rho) binary64
+    unsigned *nbc;         // binary64 mode: the entries within the cutoff, per share (prune_share)
+    int *nbc_count;        // by slot and share
     int srad;              // stencil radius in cells of the list build
     float rskin2;          // (largest cutoff + skin)^2, scaled units (xs)
+    float rcut2;           // (largest cutoff)^2, scaled units, widened by 2e-5 relative
     float half_skin2;      // (skin/2)^2, scaled units: displacement that triggers a rebuild
     // Scaled frame of the skin-list binary32 coordinates (xl, xb, xf4 of a
     // skin system): x' = xs x with xs = binary32(cellh[0]) / cellh[0] in
@@ -190,12 +193,14 @@ struct fmdg_sys
     int graph_mode;               // 0 velocity Verlet, 1 symplectic Euler
     int fblk;                     // threads per block of the list/density/force kernels
     bool eam_borrowed;            // EAM tables belong to another system
+    bool served;                  // a served job: its precision is fixed at the upload
     char *arena;                  // one device allocation holding the per-atom and per-cell buffers
     bool skin_set;                // skin chosen by the caller (any precision)
     int list_capacity;            // neighbour-list entries per atom; 0: estimated at upload
     int build_lanes;              // threads per atom of a skin-list build; 0: by size
     double rsk;                   // skin-list radius (largest cutoff + skin), real units
-    double skin;                  // Verlet skin of the neighbour list (A), 0: exact per-step list
+    double skin;                  // Verlet skin asked for (A), 0: exact per-step list
+    double skin_used;             // the skin of the list in use, 0: exact per-step list
 };
 
 // the skin kernels' binary32 pair parameters in the scaled frame: the
@@ -235,6 +240,8 @@ struct LocOne
     static constexpr int max_threads = 128;
     static constexpr int min_blocks = 0;      // 0: register count left to the compiler
     static constexpr int lean_min_blocks = 7; // lean force kernels: 7 blocks of 128 (72 registers), measured best
+    static constexpr bool one_lane = false;     // lanes by Geo::lane_log
+    static constexpr bool split_shares = false; // every share has its lane
     static constexpr bool renumbered = false;  // skin-list slots stay the upload positions
     Geo g;
 };
@@ -244,12 +251,21 @@ struct LocPack
     static constexpr int max_threads = 256;
     static constexpr int min_blocks = 0;
     static constexpr int lean_min_blocks = 0; // packed lean force kernels: compiler's choice, measured best
+    static constexpr bool one_lane = true;      // one share, one lane per slot
+    static constexpr bool split_shares = false;
     static constexpr bool renumbered = true;   // slot = index whenever a list is built
     int nsys;
     int bstart[FMDG_PACK_MAX + 1];
     Geo geos[FMDG_PACK_MAX];
 };
-static_assert(sizeof(LocPack) < 32000, "a packed launch's parameters exceed the 32 KB limit");
+// a pack of small systems, whose list walks are split into shares
+// (fmdg_skin.cu): the kernels of the others keep their code free of it
+struct LocPackShares : LocPack
+{
+    static constexpr bool one_lane = false;
+    static constexpr bool split_shares = true;  // a lane may walk several shares
+};
+static_assert(sizeof(LocPack) <= 32704, "a packed launch's parameters exceed the 32 KB limit");
 
 __device__ __forceinline__ const Geo &loc_geo(const LocOne &L, int &bx, int &nb)
 {
@@ -292,6 +308,7 @@ struct fmdg_pack_launch
     int cats;                   // bit mask (1 << FMDG_POT_*) of the members' pair categories
     int mixed;
     int lean;                   // every member has one kind (lean binary32 kernels)
+    int shares;                 // the members' list walks are split into shares (small systems)
     int fblk;                   // threads per block of the list/density/force kernels
     LocPack la;                 // 128-thread atom blocks
     LocPack lc;                 // 128-thread cell blocks
@@ -327,8 +344,9 @@ int fmdg_launch_pair_forces(fmdg_sys_t *s, int group, int finish, double dt, int
 int fmdg_launch_thermo(fmdg_sys_t *s, int group, int thermostat, double dt, double tau, double T0);
 int fmdg_force_blocks(const fmdg_sys_t *s);
 int fmdg_capacity_estimate(const int *cell_count, int ncell, double cell_volume, double rlist);
+int fmdg_share_log(const fmdg_sys_t *s, int n);
 int fmdg_list_capacity(const fmdg_sys_t *s, const int *cell_count, int ncell);
-size_t fmdg_bytes_estimate(int n, int ncell, int maxnb);
+size_t fmdg_bytes_estimate(int n, int ncell, int maxnb, int prec);
 int fmdg_set_steps_left(fmdg_sys_t *s, int steps);
 // single-system path on a skin list (fmdg_skin.cu)
 int fmdg_skin_launch_nlist(fmdg_sys_t *s);

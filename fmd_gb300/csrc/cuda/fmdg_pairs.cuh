@@ -309,13 +309,16 @@ __device__ __forceinline__ double warp_sum_transposed(const double (&v)[NV], int
     return d;
 }
 
-// Deterministic block reduction of NV doubles; thread 0 writes out[0..NV).
+// Deterministic block reduction of NV doubles of the block's first
+// `threads` threads (the others hold zeros); thread 0 writes out[0..NV).
 template <int NV>
-__device__ __forceinline__ void block_reduce_store(double (&v)[NV], double *out)
+__device__ __forceinline__ void block_reduce_store(double (&v)[NV], double *out, int threads)
 {
     __shared__ double red[32][NV];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (NV >= 3)
+    if (w * 32 >= threads)
+        ;
+    else if (NV >= 3)
     {
         const double s = warp_sum_transposed<NV>(v, lane);
         const int k = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
@@ -331,7 +334,7 @@ __device__ __forceinline__ void block_reduce_store(double (&v)[NV], double *out)
     __syncthreads();
     if (threadIdx.x == 0)
     {
-        const int nw = (blockDim.x + 31) >> 5;
+        const int nw = (threads + 31) >> 5;
         for (int k = 0; k < NV; k++)
         {
             double t = 0.0;

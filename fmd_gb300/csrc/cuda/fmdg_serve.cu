@@ -102,6 +102,7 @@ struct Pack
 {
     int cls = 0, mixed = 0;
     int lean = 0;       // one-kind jobs (lean binary32 kernels); a job's variant never depends on the mix
+    int shares = 0;     // small jobs, whose list walks are split into shares (Geo::share_log > 0)
     cudaStream_t stream = nullptr;
     std::vector<Job *> members;
     bool dirty = true;
@@ -225,15 +226,16 @@ int want_fblk(const fmdg_server_t *S, const Pack &p)
 
 int pack_class(int cats) { return __builtin_popcount(cats) > 1 ? 0 : __builtin_ctz(cats); }
 
-// a pack of (class, mixed, lean) with room for one more system
-Pack *pack_for(fmdg_server_t *S, int cls, int mixed, int lean)
+// a pack of (class, mixed, lean, shares) with room for one more system
+Pack *pack_for(fmdg_server_t *S, int cls, int mixed, int lean, int shares)
 {
     for (Pack *p : S->packs[cls][mixed])
-        if (p->lean == lean && p->active() < FMDG_PACK_MAX) return p;
+        if (p->lean == lean && p->shares == shares && p->active() < FMDG_PACK_MAX) return p;
     Pack *p = new Pack();
     p->cls = cls;
     p->mixed = mixed;
     p->lean = lean;
+    p->shares = shares;
     if (cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking) != cudaSuccess)
     {
         delete p;
@@ -288,6 +290,7 @@ int setup_job(fmdg_server_t *S, Job *j)
         if ((rc = fmdg_share_eam(s, it->second))) return rc;
     }
     if ((rc = fmdg_set_precision(s, j->prec))) return rc;
+    s->served = true;
     std::vector<double> hx(3 * (size_t)j->n), hv(3 * (size_t)j->n);
     std::vector<unsigned> hk(j->n), hid(j->n);
     std::vector<int> hg(j->n, 0);
@@ -361,7 +364,8 @@ int admit(fmdg_server_t *S, double budget_s)
             retire(S, j);
             continue;
         }
-        Pack *p = pack_for(S, pack_class(j->cats), j->prec == FMDG_PREC_MIXED, j->nkinds == 1);
+        Pack *p = pack_for(S, pack_class(j->cats), j->prec == FMDG_PREC_MIXED, j->nkinds == 1,
+                           j->sys->g.share_log > 0);
         if (!p)
         {
             fail_job(S, j, fmdg_set_error("fmdg_srv: cannot create a pack stream"), true);
@@ -371,6 +375,26 @@ int admit(fmdg_server_t *S, double budget_s)
         p->dirty = true;
     }
     return FMDG_OK;
+}
+
+// How many halvings of the lanes (Geo::lane_log) keep the threads of every
+// running job within LANE_THREADS: with few atoms running each share of a
+// list walk gets its own lane, with many each lane walks more of them.  The
+// shares, and so the results, stay the same.
+constexpr double LANE_THREADS = 1 << 18;
+int lane_level(fmdg_server_t *S)
+{
+    int level = 0;
+    for (; level < 5; level++)
+    {
+        double threads = 0.0;
+        each_pack(S, [&](Pack &p) {
+            for (const Job *j : p.members)
+                if (j->left > 0) threads += (double)j->n * (1 << std::max(0, j->sys->g.share_log - level));
+        });
+        if (threads <= LANE_THREADS) break;
+    }
+    return level;
 }
 
 // Geo table, block maps and the captured chunk of the current membership.
@@ -394,6 +418,7 @@ int rebuild(fmdg_server_t *S, Pack &p)
     P.cats = 0;
     for (const Job *j : p.members) P.cats |= j->cats;
     P.lean = p.lean;
+    P.shares = p.shares;
     P.mixed = p.mixed;
     P.fblk = fblk;
     LocPack *locs[4] = {&P.la, &P.lc, &P.lf, &P.ls};
@@ -402,14 +427,16 @@ int rebuild(fmdg_server_t *S, Pack &p)
         L->nsys = P.nsys;
         L->bstart[0] = 0;
     }
+    const int level = lane_level(S);
     for (int k = 0; k < P.nsys; k++)
     {
         fmdg_sys_t *s = p.members[k]->sys;
         s->fblk = fblk;
+        s->g.lane_log = (unsigned char)std::max(0, s->g.share_log - level);
         for (LocPack *L : locs) L->geos[k] = s->g;
         P.la.bstart[k + 1] = P.la.bstart[k] + fmdg_grid(s->g.cap, 128);
         P.lc.bstart[k + 1] = P.lc.bstart[k] + fmdg_grid(s->g.ncell, 128);
-        P.lf.bstart[k + 1] = P.lf.bstart[k] + fmdg_grid(s->g.cap, fblk);
+        P.lf.bstart[k + 1] = P.lf.bstart[k] + fmdg_grid(s->g.cap << s->g.lane_log, fblk);
         P.ls.bstart[k + 1] = k + 1;
     }
     // members set up on their own streams must be ready before the chunk
@@ -800,7 +827,7 @@ extern "C" int fmdg_srv_submit(fmdg_server_t *S, const fmdg_job_desc_t *d, long 
     const int maxnb = j->list_capacity > 0 ? j->list_capacity
                                            : fmdg_capacity_estimate(j->cell_count.data(), ncell,
                                                                     j->cellh[0] * j->cellh[1] * j->cellh[2], rl);
-    j->bytes = fmdg_bytes_estimate(d->n, ncell, maxnb);
+    j->bytes = fmdg_bytes_estimate(d->n, ncell, maxnb, d->precision);
     j->id = S->next_id++;
     j->t_submit = wall_s() - S->t0;
     S->jobs[j->id] = j;

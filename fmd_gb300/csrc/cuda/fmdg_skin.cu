@@ -37,6 +37,7 @@
 // Pair arithmetic and precision modes are those of the per-step kernels
 // (fmdg_force.cu); the lean variants (one kind, no group) are described at
 // k_force_skin.
+#include <algorithm>
 #include <type_traits>
 
 #include "fmdg_pairs.cuh"
@@ -236,10 +237,6 @@ struct NoRound
     __device__ __forceinline__ void operator()(int) const {}
 };
 
-// List walk of slot t (four entries per round): f(neighbour slot, its
-// binary32 position, image offset); r(k) after every k entries visited (a
-// round of four, or one).  PF: the next round's list rows are prefetched
-// into L1 while this round is processed (the rows stream from DRAM).
 // An atom whose list overflowed scans the stencil of its cell directly:
 // positions are the current binary64 ones relative to the cells of the
 // last refresh (packed systems refresh their cells only at a rebuild; an
@@ -247,19 +244,47 @@ struct NoRound
 // list radius), and of the occurrences of a neighbour (a cell recurs in the
 // stencil when an axis has fewer than 2R + 1 cells) only the image within
 // the list radius is passed on.
+template <typename F, bool DF>
+__device__ __forceinline__ void for_each_slot_overflow(const Geo &g, const Side &S, const SkinOffT<DF> &so, int t,
+                                                       int i, float4 &xi, F &&f)
+{
+    const double4_32a xdi = g.xd[t], oi = g.corig[S.cell_of[i]];
+    const double xs = g.xs;
+    xi = make_float4((float)((xdi.x - oi.x) * xs), (float)((xdi.y - oi.y) * xs), (float)((xdi.z - oi.z) * xs), xi.w);
+    const float lim2 = g.rskin2 * 1.0001f;
+    for_each_candidate(g, S, i, xi, [&](int j, int code) {
+        const int js = S.slot[j];
+        const double4_32a xdj = g.xd[js], oj = g.corig[S.cell_of[j]];
+        const float4 xj = make_float4((float)((xdj.x - oj.x) * xs), (float)((xdj.y - oj.y) * xs),
+                                      (float)((xdj.z - oj.z) * xs), g.xf4[j].w);
+        float4 o = so.off[code];
+        const float3 d = rv_of(xi, xj, o);
+        if (d.x * d.x + d.y * d.y + d.z * d.z > lim2) return;
+        o.w = __int_as_float(-1 - code);    // current-cell frame, not the build frame
+        f(js, xj, o);
+    });
+}
+
+// Share v of V of the list walk of slot t (rounds of four entries; share v
+// takes rounds v, v + V, ...): f(neighbour slot, its binary32 position,
+// image offset); r(k) after every k entries visited (a round of four, or
+// one).  PF: the next round's list rows are prefetched into L1 while this
+// round is processed (the rows stream from DRAM).
+// An atom whose list overflowed is share 0's alone (for_each_slot_overflow).
 template <bool PF = false, typename F, typename R, bool DF>
 __device__ __forceinline__ void for_each_slot_pair(const Geo &g, const Side &S, const SkinOffT<DF> &so, int t, int i,
-                                                   float4 &xi, F &&f, R &&r)
+                                                   int v, int V, float4 &xi, F &&f, R &&r)
 {
     const int cnt = g.nbr_count[t];
     if (cnt <= g.maxnb)
     {
-        const int cap = g.cap;
+        const int cap = g.cap, step = 4 * V;
         const int4 *col = reinterpret_cast<const int4 *>(g.nbr) + t;
-        int k = 0;
-        for (; k + 4 <= cnt; k += 4)
+        int k = 4 * v;
+        for (; k + 4 <= cnt; k += step)
         {
-            if (PF && k + 8 <= cnt) asm volatile("prefetch.global.L1 [%0];" ::"l"(col + (size_t)((k >> 2) + 1) * cap));
+            if (PF && k + step + 4 <= cnt)
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(col + (size_t)((k + step) >> 2) * cap));
             const int4 e4 = __ldg(col + (size_t)(k >> 2) * cap);
             const int e0 = e4.x, e1 = e4.y, e2 = e4.z, e3 = e4.w;
             const float4 x0 = g.xl[e0 & SLOT_MASK], x1 = g.xl[e1 & SLOT_MASK];
@@ -283,33 +308,87 @@ __device__ __forceinline__ void for_each_slot_pair(const Geo &g, const Side &S, 
             }
         }
     }
-    else
-    {
-        const double4_32a xdi = g.xd[t], oi = g.corig[S.cell_of[i]];
-        const double xs = g.xs;
-        xi = make_float4((float)((xdi.x - oi.x) * xs), (float)((xdi.y - oi.y) * xs), (float)((xdi.z - oi.z) * xs),
-                         xi.w);
-        const float lim2 = g.rskin2 * 1.0001f;
-        for_each_candidate(g, S, i, xi, [&](int j, int code) {
-            const int js = S.slot[j];
-            const double4_32a xdj = g.xd[js], oj = g.corig[S.cell_of[j]];
-            const float4 xj = make_float4((float)((xdj.x - oj.x) * xs), (float)((xdj.y - oj.y) * xs),
-                                          (float)((xdj.z - oj.z) * xs), g.xf4[j].w);
-            float4 o = so.off[code];
-            const float3 d = rv_of(xi, xj, o);
-            if (d.x * d.x + d.y * d.y + d.z * d.z > lim2) return;
-            o.w = __int_as_float(-1 - code);    // current-cell frame, not the build frame
+    else if (v == 0)
+        for_each_slot_overflow(g, S, so, t, i, xi, [&](int js, float4 xj, float4 o) {
             f(js, xj, o);
             r(1);
         });
-    }
 }
 
 template <typename F, bool DF>
 __device__ __forceinline__ void for_each_slot_pair(const Geo &g, const Side &S, const SkinOffT<DF> &so, int t, int i,
-                                                   float4 &xi, F &&f)
+                                                   int v, int V, float4 &xi, F &&f)
 {
-    for_each_slot_pair(g, S, so, t, i, xi, f, NoRound{});
+    for_each_slot_pair(g, S, so, t, i, v, V, xi, f, NoRound{});
+}
+
+// The double-float kernels' walk.  Their pair arithmetic costs hundreds of
+// instructions, and a list entry out of range (a fifth to a third of a skin
+// list) would idle its lane for all of them, as the lanes of a warp hardly
+// ever agree.  So share v of V of slot t's list is first pruned: rounds of
+// four entries tested in binary32 against the largest cutoff (widened by
+// 2e-5 relative, far above the binary32 error), the entries in range
+// written to the share's own compact list (entry m at nbc[m cap V + t V + v]:
+// a row over consecutive shares), which the double-float loop then walks.
+// The EAM force pass reuses the density pass's compact lists.
+__device__ __forceinline__ int prune_share(const Geo &g, const SkinOffT<true> &so, int cnt, int t, int v, int V,
+                                           float4 ih)
+{
+    const int cap = g.cap;
+    const size_t row = (size_t)cap * V;
+    const float lim = g.rcut2;
+    const int4 *col = reinterpret_cast<const int4 *>(g.nbr) + t;
+    unsigned *out = g.nbc + (size_t)t * V + v;
+    int m = 0;
+    for (int k = 4 * v; k < cnt; k += 4 * V)
+    {
+        const int4 e4 = __ldg(col + (size_t)(k >> 2) * cap);
+        const int left = cnt - k;
+        // (the words behind a list's last entry are not defined)
+        const unsigned e[4] = {(unsigned)e4.x, left > 1 ? (unsigned)e4.y : (unsigned)e4.x,
+                               left > 2 ? (unsigned)e4.z : (unsigned)e4.x, left > 3 ? (unsigned)e4.w : (unsigned)e4.x};
+        float4 x[4];
+        for (int w = 0; w < 4; w++) x[w] = g.xl[e[w] & SLOT_MASK];
+        for (int w = 0; w < 4; w++)
+        {
+            const float3 d = rv_of(ih, x[w], so.off[e[w] >> SLOT_BITS]);
+            if (w < left && d.x * d.x + d.y * d.y + d.z * d.z < lim)
+            {
+                *out = e[w];
+                out += row;
+                m++;
+            }
+        }
+    }
+    return m;
+}
+
+// f(neighbour slot, position, image offset) for the m entries of a share's
+// compact list
+template <typename F>
+__device__ __forceinline__ void for_each_pruned(const Geo &g, const SkinOffT<true> &so, int m, int t, int v, int V, F &&f)
+{
+    const size_t row = (size_t)g.cap * V;
+    const unsigned *p = g.nbc + (size_t)t * V + v;
+    unsigned next = m > 0 ? *p : 0u;
+    for (int k = 0; k < m; k++)
+    {
+        const unsigned e = next;
+        p += row;
+        if (k + 1 < m) next = *p;
+        f((int)(e & SLOT_MASK), g.xl[e & SLOT_MASK], so.off[e >> SLOT_BITS]);
+    }
+}
+
+// sum over the lanes of a group of G (every lane of the warp takes part)
+__device__ __forceinline__ dfl group_sum(dfl v, int G)
+{
+    for (int o = G >> 1; o > 0; o >>= 1)
+    {
+        const dfl w = {__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)};
+        v = df_add(v, w);
+    }
+    return v;
 }
 
 // ---------------------------------------------------------------- kernels
@@ -617,8 +696,97 @@ __global__ void __launch_bounds__(128) k_nlist_skin_grp(__grid_constant__ const 
     finish_build(dyn, gridDim.x);
 }
 
-// EAM pass 1 + embedding (src/eam.h:270-406, src/eam.c:160-179), one
-// thread per slot.  LEAN (binary32, one kind, no group): the pair's table
+// Shares and lanes.  A slot's list walk is split into V = 2^share_log shares
+// whose partial sums meet in a fixed binary tree (share v with v + V/2
+// first), so the result depends on V alone, and V on the system's size alone
+// (fmdg_share_log).  A slot is given G = 2^lane_log <= V lanes, each of
+// which walks V / G shares: single systems G = V, packed ones fewer while
+// enough other atoms run (a served job's arithmetic must not depend on the
+// mix).  part_tree: the part of the tree inside one lane; share_log -
+// lane_log levels over the lane's M = V / G partial sums.
+constexpr int MAX_SHARES = 16;
+template <int NV>
+__device__ __forceinline__ void part_tree(dfl (&part)[MAX_SHARES][NV], int M, int nv, dfl (&sum)[NV])
+{
+    for (int h = M >> 1; h > 0; h >>= 1)
+        for (int m = 0; m < h; m++)
+            for (int q = 0; q < nv; q++) part[m][q] = df_add(part[m][q], part[m + h][q]);
+    for (int q = 0; q < nv; q++) sum[q] = part[0][q];
+}
+
+// The per-slot epilogues (embedding; finish step and block sums) are
+// binary64 work, which issues at 1/64 of the binary32 rate: run by every
+// group's first lane they would cost one warp's issue per 32 / G slots.  The
+// groups' sums go through shared memory instead (rows of blockDim / G) and
+// the block's first blockDim / G threads take one slot each, full warps
+// again.  Every thread of the block calls these; the sums meet in a fixed
+// tree over the lanes.
+extern __shared__ double stage[];
+
+// the slot whose epilogue this thread runs, -1: none
+__device__ __forceinline__ int slot_of_thread(const Geo &g, int bx, int gl)
+{
+    const int apb = blockDim.x >> gl;
+    const int t = bx * apb + threadIdx.x;
+    return ((int)threadIdx.x < apb && t < g.cap) ? t : -1;
+}
+
+// one value per slot: that of this thread's slot
+__device__ __forceinline__ double group_value(dfl v, int gl)
+{
+    if (gl == 0) return df_to_double(v);
+    v = group_sum(v, 1 << gl);
+    if ((threadIdx.x & ((1 << gl) - 1)) == 0) stage[threadIdx.x >> gl] = df_to_double(v);
+    __syncthreads();
+    return (int)threadIdx.x < (int)(blockDim.x >> gl) ? stage[threadIdx.x] : 0.0;
+}
+
+// The force (3 values), and with `thermo` energy and virial, of this
+// thread's slot.  The force values are summed by a transposing butterfly: an
+// exchange halves the values a lane carries, 2 + 1 + 1 + ... double-float
+// additions instead of three per level.
+__device__ __forceinline__ void group_forces(const dfl (&v)[5], int gl, bool thermo, double (&out)[5])
+{
+    if (gl == 0)
+    {
+        for (int q = 0; q < 5; q++) out[q] = df_to_double(v[q]);
+        return;
+    }
+    const int G = 1 << gl, lane = threadIdx.x & (G - 1), apb = blockDim.x >> gl, row = threadIdx.x >> gl;
+    auto take = [](dfl keep, dfl give, int o) {
+        const dfl w = {__shfl_xor_sync(0xffffffffu, give.hi, o), __shfl_xor_sync(0xffffffffu, give.lo, o)};
+        return df_add(keep, w);
+    };
+    int o = G >> 1;
+    const bool up = (lane & o) != 0;     // keeps values 2, 3 (else 0, 1); 3: the energy
+    const dfl k0 = take(up ? v[2] : v[0], up ? v[0] : v[2], o);
+    dfl k1 = take(up ? v[3] : v[1], up ? v[1] : v[3], o);
+    o >>= 1;
+    if (o == 0)
+    {
+        stage[(up ? 2 : 0) * apb + row] = df_to_double(k0);
+        stage[(up ? 3 : 1) * apb + row] = df_to_double(k1);
+    }
+    else
+    {
+        const bool up2 = (lane & o) != 0;
+        dfl r = take(up2 ? k1 : k0, up2 ? k0 : k1, o);
+        const int q = (up ? 2 : 0) + (up2 ? 1 : 0), low = o - 1;
+        for (o >>= 1; o > 0; o >>= 1) r = take(r, r, o);
+        if ((lane & low) == 0) stage[q * apb + row] = df_to_double(r);
+    }
+    if (thermo)
+    {
+        const dfl e = group_sum(v[4], G);
+        if (lane == 0) stage[4 * apb + row] = df_to_double(e);
+    }
+    __syncthreads();
+    const int mine = (int)threadIdx.x < apb ? threadIdx.x : 0;
+    for (int q = 0; q < 5; q++) out[q] = (q < 4 || thermo) ? stage[q * apb + mine] : 0.0;
+}
+
+// EAM pass 1 + embedding (src/eam.h:270-406, src/eam.c:160-179), a group of
+// 2^lane_log lanes per slot (see k_force_skin).  LEAN (binary32, one kind, no group): the pair's table
 // row and cutoff in registers, no per-entry kind or group lookups.
 template <class L, bool MIXED, bool HYBRID, bool LEAN>
 __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density_skin(__grid_constant__ const L loc)
@@ -633,27 +801,32 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density_skin(
     load_offsets(g, so);
     Dyn *dyn = g.dyn;
     const Side S = g.side[dyn->cur];
-    const int t = bx * blockDim.x + threadIdx.x;
+    const int gl = L::one_lane ? 0 : g.lane_log, lane = threadIdx.x & ((1 << gl) - 1);
     double acc[1] = {0.0};
-    const int i = (t < g.cap) ? g.pos[t] : -1;
-    if (i >= 0)
+    dfl dens[1] = {{0.f, 0.f}};    // this lane's shares of the density
+    auto is_active = [&](int t, int ki) {
+        return (group < 0 || g.gslot[t] == group) && sp.elem[ki] >= 0;   // hybrid: EAM kinds only
+    };
     {
-        float4 xi = g.xl[t];
-        const int ki = __float_as_int(xi.w);
-        const int ei = sp.elem[ki];
-        const bool active = (group < 0 || g.gslot[t] == group) && ei >= 0;   // hybrid: EAM kinds only
+        const int t = (bx * blockDim.x + threadIdx.x) >> gl;
+        const int i = (t < g.cap) ? g.pos[t] : -1;
+        float4 xi = i >= 0 ? g.xl[t] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const int ki = (LEAN || i < 0) ? 0 : __float_as_int(xi.w);
         const int nk = g.nkinds, nint = g.Nr2 - 1;
-        double rho = 0.0;
-        if (active)
+        const bool on = i >= 0 && is_active(t, ki);
+        const int V = L::one_lane ? 1 : 1 << g.share_log, M = L::split_shares ? V >> gl : 1;
+        dfl part[L::split_shares ? MAX_SHARES : 1][1];
+        for (int m = 0; m < M; m++)
         {
-            if (!MIXED)
+            const int v = lane + (m << gl);
+            dfl acc_rho = {0.f, 0.f};
+            if constexpr (!MIXED)
             {
                 // double-float pair arithmetic (fmdg_df.cuh)
-                const float4 ih = g.xl[t], il = g.xll[t];
+                const float4 ih = on ? xi : make_float4(0.f, 0.f, 0.f, 0.f), il = on ? g.xll[t] : ih;
                 const dfl inv_h = df_of(df_split(g.inv_dr2));
                 const float kmax = (float)(nint - 1);
-                dfl acc_rho = {0.f, 0.f};
-                for_each_slot_pair(g, S, so, t, i, xi, [&](int js, float4 xjf, float4 o) {
+                auto pair = [&](int js, float4 xjf, float4 o) {
                     if (group >= 0 && g.gslot[js] != group) return;
                     const int pidx = ki * nk + __float_as_int(xjf.w);
                     const fmdg_pair_t &pp = sp.pairs[pidx];
@@ -661,9 +834,15 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density_skin(
                     const GeomDF p = skin_geom_df(g, so, t, ih, il, js, xjf, o);
                     if (within_cut_df_mi(g, t, js, p.r2, sp.pf[pidx][2], pp.p[2]))
                         acc_rho = df_add(acc_rho, df_rho(g, pp, p, inv_h, kmax, nint));
-                });
-                rho = df_to_double(acc_rho);
+                };
+                const int cnt = on ? g.nbr_count[t] : 0;
+                const int m_in = prune_share(g, so, cnt <= g.maxnb ? cnt : 0, t, v, V, ih);
+                if (on) g.nbc_count[(size_t)t * V + v] = m_in;
+                for_each_pruned(g, so, m_in, t, v, V, pair);
+                if (cnt > g.maxnb && v == 0) for_each_slot_overflow(g, S, so, t, i, xi, pair);
             }
+            else if (!on)
+                ;
             else if constexpr (LEAN)
             {
                 // branch-free walk (table rows read for every entry, entries
@@ -677,7 +856,7 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density_skin(
                 Acc32<1> ac;
                 int npend = 0, pend = 0;
                 float pr2 = 0.f;
-                for_each_slot_pair<true>(g, S, so, t, i, xi, [&](int js, float4 xj, float4 o) {
+                for_each_slot_pair<true>(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
                     const float3 rv = rv_of(xi, xj, o);
                     const float r2 = rv.x * rv.x + rv.y * rv.y + rv.z * rv.z;
                     const bool near = fabsf(r2 - rc2f) <= band;
@@ -703,7 +882,7 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density_skin(
                 }
                 else if (npend > 1)
                 {
-                    for_each_slot_pair<false>(g, S, so, t, i, xi, [&](int js, float4 xj, float4 o) {
+                    for_each_slot_pair<false>(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
                         const float3 rv = rv_of(xi, xj, o);
                         const float r2 = rv.x * rv.x + rv.y * rv.y + rv.z * rv.z;
                         if (!(fabsf(r2 - rc2f) <= band)) return;
@@ -714,14 +893,14 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density_skin(
                     }, [&](int k) { ac.entries(k); });
                     ac.flush();
                 }
-                rho = ac.total(0);
+                acc_rho = {ac.hi[0], ac.lo[0]};
             }
             else
             {
                 const float inv_h = scaled_index_factor(g);   // (scaled r^2: index only)
                 const float kmax = (float)(nint - 1);
                 Acc32<1> ac;
-                for_each_slot_pair(g, S, so, t, i, xi, [&](int js, float4 xj, float4 o) {
+                for_each_slot_pair(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
                     if (group >= 0 && g.gslot[js] != group) return;
                     const int pidx = ki * nk + __float_as_int(xj.w);
                     const fmdg_pair_t &pp = sp.pairs[pidx];
@@ -737,8 +916,24 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density_skin(
                     ac.tick();
                 });
                 ac.flush();
-                rho = ac.total(0);
+                acc_rho = {ac.hi[0], ac.lo[0]};
             }
+            if (L::split_shares && M > 1) part[m][0] = acc_rho;
+            else dens[0] = acc_rho;
+        }
+        if constexpr (L::split_shares)
+            if (M > 1) part_tree(part, M, 1, dens);
+    }
+    // embedding, one thread per slot
+    const double rho = group_value(dens[0], gl);
+    const int t = slot_of_thread(g, bx, gl);
+    const int i = (t >= 0) ? g.pos[t] : -1;
+    if (i >= 0)
+    {
+        const int ki = LEAN ? 0 : (int)S.kind[i];
+        if (is_active(t, ki))
+        {
+            const int ei = sp.elem[ki];
             const double qr = rho * g.inv_drho;
             int irho = (int)qr;
             if (irho >= g.Nrho - 1 || irho < 0)
@@ -782,12 +977,12 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density_skin(
             if (!MIXED) g.fpdf[t] = make_float2(0.f, 0.f);
         }
     }
-    if (loc_thermo(loc, g)) block_reduce_store<1>(acc, g.partials + (size_t)nb * 8 + bx);
+    if (loc_thermo(loc, g)) block_reduce_store<1>(acc, g.partials + (size_t)nb * 8 + bx, blockDim.x >> gl);
 }
 
 // Pair forces + velocity-Verlet finish step (src/integrators.c:94-126) and
-// the thermo record, one thread per slot; the forces are stored in the
-// current order for the next start step.  LEAN (binary32, one kind, no
+// the thermo record, 2^lane_log lanes per slot (shares and lanes, above);
+// the forces are stored in the current order for the next start step.  LEAN (binary32, one kind, no
 // group): pair parameters in registers, no per-entry kind or group
 // lookups, hardware exp2 / rsqrt / rcp approximations.
 template <class L, int CAT, bool MIXED, bool LEAN>
@@ -805,32 +1000,35 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
     Dyn *dyn = g.dyn;
     const Side S = g.side[dyn->cur];
     const int cap = g.cap;
-    const int t = bx * blockDim.x + threadIdx.x;
+    const int gl = L::one_lane ? 0 : g.lane_log, lane = threadIdx.x & ((1 << gl) - 1);
     const bool thermo = loc_thermo(loc, g);
     // pe, m v^2, m v (3), count, pair virial
     double acc[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    const int i = (t < cap) ? g.pos[t] : -1;
-    if (i >= 0)
+    // this lane's shares of the force (3), energy and virial
+    dfl sum[5] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
     {
-        float4 xi = g.xl[t];
+        const int t = (bx * blockDim.x + threadIdx.x) >> gl;
+        const int i = (t < cap) ? g.pos[t] : -1;
+        float4 xi = i >= 0 ? g.xl[t] : make_float4(0.f, 0.f, 0.f, 0.f);
         const int ki = LEAN ? 0 : __float_as_int(xi.w);   // (lean EAM: w holds F'(rho))
-        const bool active = (group < 0 || g.gslot[t] == group);
         const int nk = g.nkinds;
-        double f[3] = {0.0, 0.0, 0.0};
-        double pe = 0.0, vir = 0.0;
-        if (active)
+        const int nint = g.Nr2 - 1;
+        const size_t ne = g.nelem;
+        const bool on = i >= 0 && (group < 0 || g.gslot[t] == group);
+        const int V = L::one_lane ? 1 : 1 << g.share_log, M = L::split_shares ? V >> gl : 1;
+        dfl part[L::split_shares ? MAX_SHARES : 1][5];
+        for (int m = 0; m < M; m++)
         {
-            const int nint = g.Nr2 - 1;
-            const size_t ne = g.nelem;
-            if (!MIXED)
+            const int v = lane + (m << gl);
+            for (int q = 0; q < 5; q++) sum[q] = {0.f, 0.f};
+            if constexpr (!MIXED)
             {
                 // double-float pair arithmetic (fmdg_df.cuh, df_pair)
-                const float4 ih = g.xl[t], il = g.xll[t];
-                const dfl fpi = (CAT == CAT_EAM || CAT == CAT_HYBRID) ? df_of(g.fpdf[t]) : dfl{0.f, 0.f};
+                const float4 ih = on ? xi : make_float4(0.f, 0.f, 0.f, 0.f), il = on ? g.xll[t] : ih;
+                const dfl fpi = ((CAT == CAT_EAM || CAT == CAT_HYBRID) && on) ? df_of(g.fpdf[t]) : dfl{0.f, 0.f};
                 const dfl inv_h = df_of(df_split(g.inv_dr2));
                 const float kmax = (float)(nint - 1);
-                dfl fs[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}}, pes = {0.f, 0.f}, virs = {0.f, 0.f};
-                for_each_slot_pair(g, S, so, t, i, xi, [&](int js, float4 xjf, float4 o) {
+                auto pair = [&](int js, float4 xjf, float4 o) {
                     if (group >= 0 && g.gslot[js] != group) return;
                     const int pidx = ki * nk + __float_as_int(xjf.w);
                     const fmdg_pair_t &pp = sp.pairs[pidx];
@@ -841,14 +1039,18 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
                     dfl fa, eh;
                     df_pair(g, sp, pidx, pp, cat, p, fpi, inv_h, kmax, nint, ne, [&]() { return df_of(g.fpdf[js]); },
                             fa, eh);
-                    for (int d = 0; d < 3; d++) fs[d] = df_add(fs[d], df_mul(fa, p.rv[d]));
-                    pes = df_add(pes, eh);
-                    virs = df_add(virs, df_mul(fa, p.r2));     // rv . (fa rv), both sides of the pair
-                });
-                for (int d = 0; d < 3; d++) f[d] = df_to_double(fs[d]);
-                pe = df_to_double(pes);
-                vir = 0.5 * df_to_double(virs);
+                    for (int d = 0; d < 3; d++) sum[d] = df_add(sum[d], df_mul(fa, p.rv[d]));
+                    sum[3] = df_add(sum[3], eh);
+                    sum[4] = df_add(sum[4], df_mul(fa, p.r2));     // rv . (fa rv), both sides of the pair
+                };
+                const int cnt = on ? g.nbr_count[t] : 0;
+                const int m_in = (CAT == CAT_EAM) ? (on ? g.nbc_count[(size_t)t * V + v] : 0)
+                                                  : prune_share(g, so, cnt <= g.maxnb ? cnt : 0, t, v, V, ih);
+                for_each_pruned(g, so, m_in, t, v, V, pair);
+                if (cnt > g.maxnb && v == 0) for_each_slot_overflow(g, S, so, t, i, xi, pair);
             }
+            else if (!on)
+                ;
             else if constexpr (LEAN)
             {
                 const float4 pq = make_float4(sp.pf[0][0], sp.pf[0][1], sp.pf[0][2], sp.pf[0][3]);
@@ -888,18 +1090,18 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
                         e = 0.5f * (pq.x * (e2 - 2.f * e1));
                     }
                 };
-                // E: the walk sums the energy, V: the pair virial (rv . F =
+                // E: the walk sums the energy, W: the pair virial (rv . F =
                 // fa r^2); both on steps that form the thermo record only
                 // (the EAM walk keeps its energy term on every step)
                 auto walk = [&](auto with_e, auto with_v) {
                     constexpr bool E = decltype(with_e)::value;
-                    constexpr bool V = decltype(with_v)::value;
-                    constexpr int NA = V ? 5 : (E ? 4 : 3);
+                    constexpr bool W = decltype(with_v)::value;
+                    constexpr int NA = W ? 5 : (E ? 4 : 3);
                     Acc32<NA> ac;
                     if constexpr (CAT == CAT_EAM)
                     {
                         const float band = 1e-4f * rc2f;
-                        for_each_slot_pair<false>(g, S, so, t, i, xi, [&](int js, float4 xj, float4 o) {
+                        for_each_slot_pair<false>(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
                             const float3 rv = rv_of(xi, xj, o);
                             const float r2 = rv.x * rv.x + rv.y * rv.y + rv.z * rv.z;
                             bool in = r2 < rc2f;
@@ -919,7 +1121,7 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
                             ac.part[1] += fa * rv.y;
                             ac.part[2] += fa * rv.z;
                             if constexpr (E) ac.part[3] += 0.5f * spl_val(tph, b);
-                            if constexpr (V) ac.part[NA - 1] += fa * r2;
+                            if constexpr (W) ac.part[NA - 1] += fa * r2;
                         }, [&](int k) { ac.entries(k); });
                         ac.flush();
                     }
@@ -935,7 +1137,7 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
                         const float band = 2e-5f * rc2f;
                         int npend = 0, pend = 0;
                         float3 prv = make_float3(0.f, 0.f, 0.f);
-                        for_each_slot_pair<true>(g, S, so, t, i, xi, [&](int js, float4 xj, float4 o) {
+                        for_each_slot_pair<true>(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
                             const float3 rv = rv_of(xi, xj, o);
                             const float r2 = rv.x * rv.x + rv.y * rv.y + rv.z * rv.z;
                             const bool near = fabsf(r2 - rc2f) <= band;
@@ -951,7 +1153,7 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
                             ac.part[1] += fa * rv.y;
                             ac.part[2] += fa * rv.z;
                             if constexpr (E) ac.part[3] += e;
-                            if constexpr (V) ac.part[NA - 1] += fa * r2;
+                            if constexpr (W) ac.part[NA - 1] += fa * r2;
                         }, [&](int k) { ac.entries(k); });
                         ac.flush();
                         if (npend == 1)
@@ -965,13 +1167,13 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
                                 ac.part[1] += fa * prv.y;
                                 ac.part[2] += fa * prv.z;
                                 if constexpr (E) ac.part[3] += e;
-                                if constexpr (V) ac.part[NA - 1] += fa * r2;
+                                if constexpr (W) ac.part[NA - 1] += fa * r2;
                                 ac.flush();
                             }
                         }
                         else if (npend > 1)
                         {
-                            for_each_slot_pair<false>(g, S, so, t, i, xi, [&](int js, float4 xj, float4 o) {
+                            for_each_slot_pair<false>(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
                                 const float3 rv = rv_of(xi, xj, o);
                                 const float r2 = rv.x * rv.x + rv.y * rv.y + rv.z * rv.z;
                                 if (!(fabsf(r2 - rc2f) <= band)) return;
@@ -982,14 +1184,14 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
                                 ac.part[1] += fa * rv.y;
                                 ac.part[2] += fa * rv.z;
                                 if constexpr (E) ac.part[3] += e;
-                                if constexpr (V) ac.part[NA - 1] += fa * r2;
+                                if constexpr (W) ac.part[NA - 1] += fa * r2;
                             }, [&](int k) { ac.entries(k); });
                             ac.flush();
                         }
                     }
-                    for (int d = 0; d < 3; d++) f[d] = ac.total(d);
-                    if constexpr (E) pe = ac.total(3);
-                    if constexpr (V) vir = 0.5 * ac.total(NA - 1);
+                    for (int d = 0; d < 3; d++) sum[d] = {ac.hi[d], ac.lo[d]};
+                    if constexpr (E) sum[3] = {ac.hi[3], ac.lo[3]};
+                    if constexpr (W) sum[4] = {ac.hi[NA - 1], ac.lo[NA - 1]};
                 };
                 // (the EAM walk keeps its energy term: dropping it measured
                 // slower for that kernel)
@@ -1008,7 +1210,7 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
                 const float kmax = (float)(nint - 1);
                 const float xs2 = scaled_xs2(g);
                 Acc32<5> ac;
-                for_each_slot_pair(g, S, so, t, i, xi, [&](int js, float4 xj, float4 o) {
+                for_each_slot_pair(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
                     if (group >= 0 && g.gslot[js] != group) return;
                     const int pidx = ki * nk + __float_as_int(xj.w);
                     const fmdg_pair_t &pp = sp.pairs[pidx];
@@ -1066,11 +1268,29 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
                     ac.tick();
                 });
                 ac.flush();
-                for (int d = 0; d < 3; d++) f[d] = ac.total(d);
-                pe = ac.total(3);
-                vir = 0.5 * ac.total(4);
+                for (int q = 0; q < 5; q++) sum[q] = {ac.hi[q], ac.lo[q]};
+            }
+            if (L::split_shares && M > 1)
+            {
+                for (int q = 0; q < 3; q++) part[m][q] = sum[q];
+                if (thermo)
+                    for (int q = 3; q < 5; q++) part[m][q] = sum[q];
             }
         }
+        if constexpr (L::split_shares)
+            if (M > 1) part_tree(part, M, thermo ? 5 : 3, sum);
+    }
+    // the group's sums, then one thread per slot
+    double fin[5];
+    group_forces(sum, gl, thermo, fin);
+    const int t = slot_of_thread(g, bx, gl);
+    const int i = (t >= 0) ? g.pos[t] : -1;
+    if (i >= 0)
+    {
+        const int ki = LEAN ? 0 : (int)S.kind[i];
+        const bool active = (group < 0 || g.gslot[t] == group);
+        double f[3] = {fin[0], fin[1], fin[2]};
+        double pe = fin[3], vir = 0.5 * fin[4];
         if (MIXED)
         {
             // binary32 pairs were summed in the scaled frame (Geo::xs): the
@@ -1123,7 +1343,7 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
     }
     __shared__ double blk[7];
     __shared__ unsigned ticket;
-    if (thermo) block_reduce_store<7>(acc, blk);
+    if (thermo) block_reduce_store<7>(acc, blk, blockDim.x >> gl);
     if (threadIdx.x == 0)
     {
         if (thermo)
@@ -1145,35 +1365,47 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
 }
 
 // lean: one kind and no group (used in binary32 only)
+// dynamic shared bytes of slot_of_thread for NV values per slot
+size_t stage_bytes(const LocOne &L, int blk, int nv) { return L.g.lane_log ? (size_t)nv * 8 * (blk >> L.g.lane_log) : 0; }
+size_t stage_bytes(const LocPack &L, int blk, int nv)
+{
+    size_t most = 0;
+    for (int k = 0; k < L.nsys; k++)
+        if (const int gl = L.geos[k].lane_log) most = std::max(most, (size_t)nv * 8 * (blk >> gl));
+    return most;
+}
+
 template <class L, bool MIXED>
 void launch_force_skin(const L &loc, int cats, int finish, int nb, int blk, cudaStream_t st, bool lean)
 {
+    const size_t sh = stage_bytes(loc, blk, 5);
     const int ncat = __builtin_popcount(cats);
-    if (ncat > 1) k_force_skin<L, CAT_HYBRID, MIXED, false><<<nb, blk, 0, st>>>(loc, finish);
+    if (ncat > 1) k_force_skin<L, CAT_HYBRID, MIXED, false><<<nb, blk, sh, st>>>(loc, finish);
     else if (MIXED && lean)
     {
-        if (cats == (1 << FMDG_POT_LJ)) k_force_skin<L, CAT_LJ, true, true><<<nb, blk, 0, st>>>(loc, finish);
-        else if (cats == (1 << FMDG_POT_MORSE)) k_force_skin<L, CAT_MORSE, true, true><<<nb, blk, 0, st>>>(loc, finish);
-        else k_force_skin<L, CAT_EAM, true, true><<<nb, blk, 0, st>>>(loc, finish);
+        if (cats == (1 << FMDG_POT_LJ)) k_force_skin<L, CAT_LJ, true, true><<<nb, blk, sh, st>>>(loc, finish);
+        else if (cats == (1 << FMDG_POT_MORSE)) k_force_skin<L, CAT_MORSE, true, true><<<nb, blk, sh, st>>>(loc, finish);
+        else k_force_skin<L, CAT_EAM, true, true><<<nb, blk, sh, st>>>(loc, finish);
     }
-    else if (cats == (1 << FMDG_POT_LJ)) k_force_skin<L, CAT_LJ, MIXED, false><<<nb, blk, 0, st>>>(loc, finish);
-    else if (cats == (1 << FMDG_POT_MORSE)) k_force_skin<L, CAT_MORSE, MIXED, false><<<nb, blk, 0, st>>>(loc, finish);
-    else k_force_skin<L, CAT_EAM, MIXED, false><<<nb, blk, 0, st>>>(loc, finish);
+    else if (cats == (1 << FMDG_POT_LJ)) k_force_skin<L, CAT_LJ, MIXED, false><<<nb, blk, sh, st>>>(loc, finish);
+    else if (cats == (1 << FMDG_POT_MORSE)) k_force_skin<L, CAT_MORSE, MIXED, false><<<nb, blk, sh, st>>>(loc, finish);
+    else k_force_skin<L, CAT_EAM, MIXED, false><<<nb, blk, sh, st>>>(loc, finish);
 }
 
 template <class L>
 void launch_density_skin(const L &loc, bool mixed, bool hyb, int nb, int blk, cudaStream_t st, bool lean)
 {
+    const size_t sh = stage_bytes(loc, blk, 1);
     if (mixed)
     {
-        if (hyb) k_density_skin<L, true, true, false><<<nb, blk, 0, st>>>(loc);
-        else if (lean) k_density_skin<L, true, false, true><<<nb, blk, 0, st>>>(loc);
-        else k_density_skin<L, true, false, false><<<nb, blk, 0, st>>>(loc);
+        if (hyb) k_density_skin<L, true, true, false><<<nb, blk, sh, st>>>(loc);
+        else if (lean) k_density_skin<L, true, false, true><<<nb, blk, sh, st>>>(loc);
+        else k_density_skin<L, true, false, false><<<nb, blk, sh, st>>>(loc);
     }
     else
     {
-        if (hyb) k_density_skin<L, false, true, false><<<nb, blk, 0, st>>>(loc);
-        else k_density_skin<L, false, false, false><<<nb, blk, 0, st>>>(loc);
+        if (hyb) k_density_skin<L, false, true, false><<<nb, blk, sh, st>>>(loc);
+        else k_density_skin<L, false, false, false><<<nb, blk, sh, st>>>(loc);
     }
 }
 
@@ -1198,17 +1430,24 @@ int fmdg_pack_launch_forces(const fmdg_pack_launch &P, int phases)
     if (phases & 1)
     {
         k_prep_skin<<<nab, 128, 0, st>>>(P.la, 1);
-        k_nlist_skin<<<nfb, P.fblk, 0, st>>>(P.lf);
+        k_nlist_skin<<<nab, 128, 0, st>>>(P.la);
         n += 2;
     }
     if ((phases & 2) && (P.cats & (1 << FMDG_POT_EAM)))
     {
-        launch_density_skin(P.lf, P.mixed != 0, __builtin_popcount(P.cats) > 1, nfb, P.fblk, st, P.lean != 0);
+        if (P.shares) launch_density_skin(LocPackShares{P.lf}, P.mixed != 0, __builtin_popcount(P.cats) > 1, nfb, P.fblk, st, P.lean != 0);
+        else launch_density_skin(P.lf, P.mixed != 0, __builtin_popcount(P.cats) > 1, nfb, P.fblk, st, P.lean != 0);
         n++;
     }
     if (phases & 4)
     {
-        if (P.mixed) launch_force_skin<LocPack, true>(P.lf, P.cats, 1, nfb, P.fblk, st, P.lean != 0);
+        if (P.shares)
+        {
+            const LocPackShares L{P.lf};
+            if (P.mixed) launch_force_skin<LocPackShares, true>(L, P.cats, 1, nfb, P.fblk, st, P.lean != 0);
+            else launch_force_skin<LocPackShares, false>(L, P.cats, 1, nfb, P.fblk, st, false);
+        }
+        else if (P.mixed) launch_force_skin<LocPack, true>(P.lf, P.cats, 1, nfb, P.fblk, st, P.lean != 0);
         else launch_force_skin<LocPack, false>(P.lf, P.cats, 1, nfb, P.fblk, st, false);
         n++;
     }
@@ -1240,7 +1479,7 @@ int fmdg_skin_launch_nlist(fmdg_sys_t *s)
     case 8: k_nlist_skin_grp<8><<<nbg, 128, 0, s->stream>>>(L); break;
     case 16: k_nlist_skin_grp<16><<<nbg, 128, 0, s->stream>>>(L); break;
     case 32: k_nlist_skin_grp<32><<<nbg, 128, 0, s->stream>>>(L); break;
-    default: k_nlist_skin<<<fmdg_force_blocks(s), s->fblk, 0, s->stream>>>(L); break;
+    default: k_nlist_skin<<<nbg, 128, 0, s->stream>>>(L); break;
     }
     s->launches += 2;
     FMDG_CK(cudaGetLastError());

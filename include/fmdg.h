@@ -107,9 +107,9 @@ int fmdg_set_precision(fmdg_sys_t *s, int mode);
    and is rebuilt on the device once an atom has moved more than skin/2.
    Used when every periodic box length exceeds twice the list radius and
    the radius spans at most two cells; otherwise (and with skin 0) the
-   exact stencil list is rebuilt every step.  Default: 0.5 A for systems in
-   mixed precision at upload (environment FMD_SKIN overrides), none in
-   binary64 unless set here. */
+   exact stencil list is rebuilt every step.  Default: 0.5 A (environment
+   FMD_SKIN overrides), less where a periodic box is too short for it, none
+   for binary64 systems of several kinds. */
 int fmdg_set_skin(fmdg_sys_t *s, double skin);
 /* Neighbour-list entries per atom (before fmdg_upload; 0, the default:
    1.3 x the count at the fullest cell's density + 16).  A multiple of 8 up
