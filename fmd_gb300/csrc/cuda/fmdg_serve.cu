@@ -910,6 +910,10 @@ extern "C" int fmdg_srv_release(fmdg_server_t *S, long long id)
     if (it == S->jobs.end()) return fmdg_set_error("fmdg_srv_release: unknown job");
     Job *j = it->second;
     if (j->state != JOB_DONE && j->state != JOB_FAILED) return FMDG_E_STATE;
+    // a pack keeps its finished members until its next rebuild
+    each_pack(S, [&](Pack &p) {
+        p.members.erase(std::remove(p.members.begin(), p.members.end(), j), p.members.end());
+    });
     delete j;
     S->jobs.erase(it);
     return FMDG_OK;

@@ -74,3 +74,21 @@ def test_lanes_change_nothing(L, eam, pot, n, precision):
         srv.close()
     for a, b in zip(*got):
         np.testing.assert_array_equal(a, b)
+
+
+def test_release_between_batches(L, eam):
+    """Jobs released as soon as a batch is done, batch after batch on one
+    server: a released job is gone from its pack too."""
+    x, v, l = _cube("lj", 6, 99)
+    srv = serve.Server(L, budget_bytes=8 << 30, max_jobs=64, chunk_steps=8, eam=eam)
+    first = None
+    for _ in range(6):
+        ids = [srv.submit("lj", x, v, l, 16, precision=p, keep_state=True) for p in (0, 1, 0, 1, 0)]
+        srv.drain()
+        got = [srv.state(j, len(x))[0] for j in ids]
+        for j in ids:
+            srv.release(j)
+        first = first or got
+        for a, b in zip(first, got):
+            np.testing.assert_array_equal(a, b)
+    srv.close()
