@@ -29,41 +29,42 @@
 //      key of the pass sequence read from the last hop backwards.
 // Each destination cell sorts its (few) arrivals by that key, after which
 // every atom knows its new index and one scatter writes the next side.
-#include "fmdg_internal.cuh"
+//
+// Kernels.  A single system of more than CLUSTER_ATOMS atoms runs the phases
+// as grid kernels (k_bin_classify, k_bin_scan, k_bin_cells, k_bin_arrivals,
+// k_bin_place).  A smaller one, and every packed system on the steps that
+// rebuild its list, runs all of them in one kernel: one cluster of blocks
+// per system, a cluster barrier between the phases (k_refresh_cluster) --
+// launches and their gaps were most of a small system's step.
+#include <cooperative_groups.h>
+
+#include "fmdg_prep.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace {
+
+// Measured on one GB300, us per step of the whole refresh: 256 atoms 21 (eight
+// launches) -> 11 (one cluster kernel), 4000 atoms 24 -> 14, but 32 000 atoms
+// 26 (five grid kernels) against 61.
+constexpr int CLUSTER_ATOMS = 1 << 13;
 
 __device__ __forceinline__ int cell_flat(const Geo &g, int x, int y, int z)
 {
     return z + g.nc[2] * (y + g.nc[1] * x);
 }
 
-// Start-of-step update fused with the binning decision.
+// Phase 1, one atom: start-of-step update fused with the binning decision.
 //  mode VV: src/integrators.c:40-75 (v *= lambda; v += dt*0.5/m*F; x += dt*v)
 //  mode SE: src/integrators.c:129-152 (v += dt*F/m; x += dt*v)
 // Explicit _rn intrinsics keep the reference's operation order with no
 // fused multiply-add, so positions and velocities match bit for bit given
-// the same forces.  lazy (packed systems, mode REFRESH_ONLY): the cells are
-// refreshed only on a step that rebuilds the skin list.
-template <class L>
-__global__ void k_bin_classify(__grid_constant__ const L loc, int mode, int lazy)
+// the same forces.  hk: half kick dt * 0.5 / m per kind, formed on the host
+// (set_step_dt) with the reference's operations.
+__device__ __forceinline__ void classify_atom(const Geo &g, Dyn *dyn, const Side &S, int i, int mode, const double *hk)
 {
-    int bx, nb;
-    const Geo &g = loc_geo(loc, bx, nb);
-    if (loc_idle(loc, g)) return;
-    if (lazy && !g.dyn->rebuild) return;
     const double dt = g.st.dt;
     const int group = g.st.group, thermostat = g.st.thermostat;
-    // half kick dt * 0.5 / m per kind, formed on the host (set_step_dt):
-    // the reference's operations, so the same bits as per atom
-    __shared__ double hk[FMDG_MAXK];
-    if (threadIdx.x < g.nkinds) hk[threadIdx.x] = g.st.hk[threadIdx.x];
-    __syncthreads();
-    Dyn *dyn = g.dyn;
-    const int n = dyn->n;
-    const int i = bx * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const Side S = g.side[dyn->cur];
     const int cap = g.cap;
 
     double x[3], v[3];
@@ -170,53 +171,98 @@ __global__ void k_bin_classify(__grid_constant__ const L loc, int mode, int lazy
     if (nq == 0 && c < D) atomicAdd(&g.arr_lower[D], 1);
 }
 
-// Exclusive scans over cells (one block): arrival bases and the next side's
-// cell_start, plus the atom count after the refresh.
-template <class L>
-__global__ void k_bin_scan(__grid_constant__ const L loc)
+// Exclusive scans over the cells by the blocks of one cluster: arrival bases
+// and the next side's cell_start, plus the atom count after the refresh.
+// Each block takes a run of cells: first its totals, which the blocks read
+// from one another's shared memory, then tiles of blockDim cells scanned by
+// warp shuffles on top of the totals before them.  Coalesced: the 17 576
+// cells of the 256 000-atom EAM system take 9.8 us (launch included), a
+// single block with consecutive cells per thread took 36.
+struct ScanSmem
 {
-    int bx, nb;
-    const Geo &g = loc_geo(loc, bx, nb);
-    if (loc_idle(loc, g)) return;
-    Dyn *dyn = g.dyn;
-    if (!dyn->any_move) return;
-    const Side S = g.side[dyn->cur];
-    const Side T = g.side[dyn->cur ^ 1];
-    const int nc = g.ncell;
-    __shared__ int sa[1024], sn[1024];
-    const int tid = threadIdx.x, nt = blockDim.x;
-    const int per = (nc + nt - 1) / nt;
-    const int lo = min(nc, tid * per), hi = min(nc, lo + per);
-    int ta = 0, tn = 0;
-    for (int c = lo; c < hi; c++)
+    int2 total;          // this block's sums
+    int2 warp[32];
+};
+
+__device__ __forceinline__ int2 warp_inclusive(int2 v, int lane)
+{
+    for (int o = 1; o < 32; o <<= 1)
     {
-        ta += g.arr_total[c];
-        tn += S.cell_start[c + 1] - S.cell_start[c] - g.dep_count[c] + g.arr_total[c];
+        const int a = __shfl_up_sync(0xffffffffu, v.x, o), b = __shfl_up_sync(0xffffffffu, v.y, o);
+        if (lane >= o) { v.x += a; v.y += b; }
     }
-    sa[tid] = ta; sn[tid] = tn;
+    return v;
+}
+
+// inclusive scan over the block; every thread must call it
+__device__ __forceinline__ int2 block_inclusive(int2 v, ScanSmem &sm, int2 &sum)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    v = warp_inclusive(v, lane);
+    if (lane == 31) sm.warp[w] = v;
     __syncthreads();
-    for (int off = 1; off < nt; off <<= 1)
+    if (w == 0)
     {
-        int va = 0, vn = 0;
-        if (tid >= off) { va = sa[tid - off]; vn = sn[tid - off]; }
-        __syncthreads();
-        sa[tid] += va; sn[tid] += vn;
-        __syncthreads();
+        const int2 t = warp_inclusive(lane < nw ? sm.warp[lane] : make_int2(0, 0), lane);
+        __syncwarp();
+        if (lane < nw) sm.warp[lane] = t;
     }
-    int ra = sa[tid] - ta, rn = sn[tid] - tn;
-    for (int c = lo; c < hi; c++)
+    __syncthreads();
+    if (w > 0) { v.x += sm.warp[w - 1].x; v.y += sm.warp[w - 1].y; }
+    sum = sm.warp[nw - 1];
+    __syncthreads();
+    return v;
+}
+
+__device__ __forceinline__ void scan_cells(const Geo &g, Dyn *dyn, const Side &S, const Side &T, ScanSmem &sm,
+                                           cg::cluster_group &cl)
+{
+    const int nc = g.ncell, rank = cl.block_rank(), nblk = cl.num_blocks();
+    const int per = (nc + nblk - 1) / nblk;
+    const int lo = min(nc, rank * per), hi = min(nc, lo + per);
+    auto cell = [&](int c) {
+        if (c >= hi) return make_int2(0, 0);
+        const int a = g.arr_total[c];
+        return make_int2(a, S.cell_start[c + 1] - S.cell_start[c] - g.dep_count[c] + a);
+    };
+    int2 sum = make_int2(0, 0), tile;
+    for (int c = lo + threadIdx.x; c < hi; c += blockDim.x)
     {
-        g.arr_base[c] = ra;
-        T.cell_start[c] = rn;
-        ra += g.arr_total[c];
-        rn += S.cell_start[c + 1] - S.cell_start[c] - g.dep_count[c] + g.arr_total[c];
+        const int2 v = cell(c);
+        sum.x += v.x;
+        sum.y += v.y;
     }
-    if (tid == nt - 1)
+    block_inclusive(sum, sm, tile);
+    if (threadIdx.x == 0) sm.total = tile;
+    cl.sync();
+    int2 base = make_int2(0, 0);
+    for (int r = 0; r < rank; r++)
     {
-        g.arr_base[nc] = sa[tid];
-        T.cell_start[nc] = sn[tid];
-        dyn->n_next = sn[tid];
+        const int2 t = cl.map_shared_rank(&sm, r)->total;
+        base.x += t.x;
+        base.y += t.y;
     }
+    for (int c0 = lo; c0 < hi; c0 += blockDim.x)
+    {
+        const int c = c0 + threadIdx.x;
+        const int2 v = cell(c);
+        const int2 in = block_inclusive(v, sm, tile);
+        if (c < hi)
+        {
+            g.arr_base[c] = base.x + in.x - v.x;
+            T.cell_start[c] = base.y + in.y - v.y;
+        }
+        base.x += tile.x;
+        base.y += tile.y;
+    }
+    if (rank == nblk - 1 && threadIdx.x == 0)
+    {
+        g.arr_base[nc] = base.x;
+        T.cell_start[nc] = base.y;
+        dyn->n_next = base.y;
+    }
+    // (no block leaves while another still reads its totals)
+    cl.sync();
 }
 
 // Replay of the swap-remove walk of one source cell (src/misc.c:276-303)
@@ -224,17 +270,8 @@ __global__ void k_bin_scan(__grid_constant__ const L loc)
 // cells.  Emits the departure rank of each leaving atom (and queues it in
 // its destination's bucket), the final slot of each stayer, and the slot of
 // each placeholder.
-template <class L>
-__global__ void k_bin_cells(__grid_constant__ const L loc)
+__device__ __forceinline__ void replay_cell(const Geo &g, const Side &S, int c)
 {
-    int bx, nb;
-    const Geo &g = loc_geo(loc, bx, nb);
-    if (loc_idle(loc, g)) return;
-    Dyn *dyn = g.dyn;
-    if (!dyn->any_move) return;
-    const int c = bx * blockDim.x + threadIdx.x;
-    if (c >= g.ncell) return;
-    const Side S = g.side[dyn->cur];
     const int start = S.cell_start[c];
     const int n0 = S.cell_start[c + 1] - start;
     const int A = g.arr_lower[c];
@@ -273,21 +310,11 @@ __global__ void k_bin_cells(__grid_constant__ const L loc)
     }
 }
 
-// Order the arrivals of each destination cell and give them new indexes.
-template <class L>
-__global__ void k_bin_arrivals(__grid_constant__ const L loc)
+// Order the arrivals of destination cell D and give them new indexes.
+__device__ __forceinline__ void order_arrivals(const Geo &g, const Side &S, const Side &T, int D)
 {
-    int bx, nb;
-    const Geo &g = loc_geo(loc, bx, nb);
-    if (loc_idle(loc, g)) return;
-    Dyn *dyn = g.dyn;
-    if (!dyn->any_move) return;
-    const int D = bx * blockDim.x + threadIdx.x;
-    if (D >= g.ncell) return;
     const int total = g.arr_total[D];
     if (total == 0) return;
-    const Side S = g.side[dyn->cur];
-    const Side T = g.side[dyn->cur ^ 1];
     const int base = g.arr_base[D];
     int *b = g.bucket + base;
     auto key = [&](int a) -> unsigned long long {
@@ -313,60 +340,63 @@ __global__ void k_bin_arrivals(__grid_constant__ const L loc)
     }
 }
 
-template <class L>
-__global__ void k_bin_scatter(__grid_constant__ const L loc)
+// Last phase, one atom: its place on the next side (moved: some atom moved,
+// so the sides are swapped after this), and the per-atom tables the force
+// kernels read, formed from the position in hand.  PACK: the slots are
+// renumbered in the new order -- slot = index, so a list build walks and
+// writes consecutive atoms of a cell together, and until the next rebuild
+// (no refresh in between) every slot-to-index map is the identity.
+template <bool PACK>
+__device__ __forceinline__ void place_atom(const Geo &g, Dyn *dyn, const Side &S, const Side &T, int i, bool moved,
+                                           int n_next)
 {
-    int bx, nb;
-    const Geo &g = loc_geo(loc, bx, nb);
-    if (loc_idle(loc, g)) return;
-    Dyn *dyn = g.dyn;
-    if (!dyn->any_move) return;
-    const int i = bx * blockDim.x + threadIdx.x;
-    if (i >= dyn->n) return;
-    const int d = g.bdest[i];
-    if (d == -1) return;
-    const Side S = g.side[dyn->cur];
-    const Side T = g.side[dyn->cur ^ 1];
-    const int c = S.cell_of[i];
-    int idx, D;
-    if (d == -2)
-    {
-        D = c;
-        idx = T.cell_start[c] + (g.dep_count[c] == 0 ? (i - S.cell_start[c]) : g.bslot[i]);
-    }
-    else
-    {
-        D = d;
-        idx = g.bnewidx[i];
-    }
-    if (idx < 0 || idx >= dyn->n_next)
-    {
-        // cannot happen for a consistent refresh; recorded instead of writing
-        atomic_or_err(dyn, FMDG_ERRBIT_INTERNAL);
-        return;
-    }
     const int cap = g.cap;
-    for (int k = 0; k < 3; k++)
+    const int c = S.cell_of[i];
+    int idx = i, D = c;
+    if (moved)
     {
-        T.x[k * cap + idx] = S.x[k * cap + i];
-        T.v[k * cap + idx] = S.v[k * cap + i];
+        const int d = g.bdest[i];
+        if (d == -1) return;
+        if (d == -2) idx = T.cell_start[c] + (g.dep_count[c] == 0 ? (i - S.cell_start[c]) : g.bslot[i]);
+        else
+        {
+            D = d;
+            idx = g.bnewidx[i];
+        }
+        if (idx < 0 || idx >= n_next)
+        {
+            // cannot happen for a consistent refresh; recorded instead of writing
+            atomic_or_err(dyn, FMDG_ERRBIT_INTERNAL);
+            return;
+        }
     }
-    T.kind[idx] = S.kind[i];
-    T.group[idx] = S.group[i];
-    T.atomid[idx] = S.atomid[i];
-    T.cell_of[idx] = D;
-    if (g.skin_on) T.slot[idx] = S.slot[i];
+    const double x[3] = {S.x[i], S.x[cap + i], S.x[2 * (size_t)cap + i]};
+    const unsigned kind = S.kind[i];
+    const int group = S.group[i];
+    const int t = PACK ? idx : (g.skin_on ? S.slot[i] : 0);
+    if (moved)
+    {
+        for (int k = 0; k < 3; k++)
+        {
+            T.x[k * cap + idx] = x[k];
+            T.v[k * cap + idx] = S.v[k * cap + i];
+        }
+        T.kind[idx] = kind;
+        T.group[idx] = group;
+        T.atomid[idx] = S.atomid[i];
+        T.cell_of[idx] = D;
+        if (g.skin_on) T.slot[idx] = t;
+    }
+    else if (PACK)
+        S.slot[i] = t;
+    if (g.skin_on) prep_skin_atom(g, dyn, idx, t, D, (int)kind, group, x, !PACK && !dyn->rebuild);
+    else prep_local_atom(g, idx, D, (int)kind, x);
 }
 
 // swaps sides after a refresh that moved atoms; advances the device copy of
 // the simulation time by one step (src/integrators.c:203, :256)
-template <class L>
-__global__ void k_bin_flip(__grid_constant__ const L loc, int mode)
+__device__ __forceinline__ void flip_sides(const Geo &g, Dyn *dyn, int mode)
 {
-    int bx, nb;
-    const Geo &g = loc_geo(loc, bx, nb);
-    if (loc_idle(loc, g) || threadIdx.x != 0) return;
-    Dyn *dyn = g.dyn;
     dyn->time += (mode == FMDG_REFRESH_ONLY) ? 0.0 : g.st.dt;
     if (dyn->any_move)
     {
@@ -376,26 +406,153 @@ __global__ void k_bin_flip(__grid_constant__ const L loc, int mode)
     }
 }
 
-// per-cell binning counters of every system of a pack that refreshes its
-// cells this step
-__global__ void k_bin_clear(__grid_constant__ const LocPack loc)
+__device__ __forceinline__ void load_half_kicks(const Geo &g, double *hk)
 {
-    int bx, nb;
-    const Geo &g = loc_geo(loc, bx, nb);
+    if (threadIdx.x < g.nkinds) hk[threadIdx.x] = g.st.hk[threadIdx.x];
+    __syncthreads();
+}
+
+// ------------------------------------------------- grid kernels (one system)
+
+__global__ void __launch_bounds__(256) k_bin_classify(__grid_constant__ const LocOne loc, int mode)
+{
+    const Geo &g = loc.g;
+    __shared__ double hk[FMDG_MAXK];
+    load_half_kicks(g, hk);
+    Dyn *dyn = g.dyn;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < dyn->n) classify_atom(g, dyn, g.side[dyn->cur], i, mode, hk);
+}
+
+// (one cluster)
+__global__ void __launch_bounds__(1024) k_bin_scan(__grid_constant__ const LocOne loc)
+{
+    const Geo &g = loc.g;
+    Dyn *dyn = g.dyn;
+    if (!dyn->any_move) return;
+    __shared__ ScanSmem sm;
+    cg::cluster_group cl = cg::this_cluster();
+    scan_cells(g, dyn, g.side[dyn->cur], g.side[dyn->cur ^ 1], sm, cl);
+}
+
+__global__ void __launch_bounds__(128) k_bin_cells(__grid_constant__ const LocOne loc)
+{
+    const Geo &g = loc.g;
+    const Dyn *dyn = g.dyn;
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (dyn->any_move && c < g.ncell) replay_cell(g, g.side[dyn->cur], c);
+}
+
+__global__ void __launch_bounds__(128) k_bin_arrivals(__grid_constant__ const LocOne loc)
+{
+    const Geo &g = loc.g;
+    const Dyn *dyn = g.dyn;
+    const int D = blockIdx.x * blockDim.x + threadIdx.x;
+    if (dyn->any_move && D < g.ncell) order_arrivals(g, g.side[dyn->cur], g.side[dyn->cur ^ 1], D);
+}
+
+// the last block to finish swaps the sides
+__global__ void __launch_bounds__(256) k_bin_place(__grid_constant__ const LocOne loc, int mode)
+{
+    const Geo &g = loc.g;
+    Dyn *dyn = g.dyn;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int cur = dyn->cur;
+    if (i < dyn->n) place_atom<false>(g, dyn, g.side[cur], g.side[cur ^ 1], i, dyn->any_move != 0, dyn->n_next);
+    __shared__ unsigned ticket;
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        __threadfence();
+        ticket = atomicAdd(&dyn->place_done, 1u);
+        if (ticket == gridDim.x - 1)
+        {
+            dyn->place_done = 0;
+            flip_sides(g, dyn, mode);
+        }
+    }
+}
+
+// ----------------------------------------------------------- cluster kernel
+
+__device__ __forceinline__ const Geo &cluster_geo(const LocOne &L, int) { return L.g; }
+__device__ __forceinline__ const Geo &cluster_geo(const LocPack &L, int s) { return L.geos[s]; }
+
+// All phases of one system's refresh by one cluster.  Packed systems
+// (LocPack): only on a step that rebuilds the system's skin list (between
+// rebuilds an atom stays within skin/2 of its build position, less than a
+// cell, and the packed kernels address atoms by slot); the conditions are
+// uniform over a cluster.
+template <class L>
+__global__ void __launch_bounds__(512) k_refresh_cluster(__grid_constant__ const L loc, int mode)
+{
+    constexpr bool PACK = L::renumbered;
+    cg::cluster_group cl = cg::this_cluster();
+    const int nblk = cl.num_blocks(), rank = cl.block_rank();
+    const Geo &g = cluster_geo(loc, blockIdx.x / nblk);
     if (loc_idle(loc, g)) return;
-    if (!g.dyn->rebuild) return;
-    const int c = bx * blockDim.x + threadIdx.x;
-    if (c >= g.ncell) return;
-    g.dep_count[c] = 0;
-    g.arr_lower[c] = 0;
-    g.arr_total[c] = 0;
-    g.bucket_fill[c] = 0;
+    Dyn *dyn = g.dyn;
+    if (PACK && !dyn->rebuild) return;
+    __shared__ double hk[FMDG_MAXK];
+    __shared__ ScanSmem sm;
+    load_half_kicks(g, hk);
+    const int n = dyn->n, cur = dyn->cur, ncell = g.ncell;
+    const Side S = g.side[cur], T = g.side[cur ^ 1];
+    const int tid = rank * blockDim.x + threadIdx.x, nt = nblk * blockDim.x;
+    // (dep_count, arr_lower, arr_total, bucket_fill are contiguous)
+    for (int c = tid; c < 4 * ncell; c += nt) g.dep_count[c] = 0;
+    cl.sync();
+    for (int i = tid; i < n; i += nt) classify_atom(g, dyn, S, i, mode, hk);
+    cl.sync();
+    const bool moved = *(volatile int *)&dyn->any_move != 0;
+    int n_next = n;
+    if (moved)
+    {
+        scan_cells(g, dyn, S, T, sm, cl);
+        for (int c = tid; c < ncell; c += nt) replay_cell(g, S, c);
+        cl.sync();
+        for (int c = tid; c < ncell; c += nt) order_arrivals(g, S, T, c);
+        cl.sync();
+        n_next = *(volatile int *)&dyn->n_next;
+    }
+    for (int i = tid; i < n; i += nt) place_atom<PACK>(g, dyn, S, T, i, moved, n_next);
+    if (PACK)
+        for (int i = n_next + tid; i < g.cap; i += nt) g.pos[i] = -1;
+    cl.sync();
+    if (tid == 0) flip_sides(g, dyn, mode);
+}
+
+// grid: blocks of `threads` in clusters of `cluster`
+template <class L>
+cudaError_t launch_cluster(void (*kernel)(L, int), const L &loc, int mode, int blocks, int threads, int cluster, cudaStream_t st)
+{
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, loc, mode);
+}
+
+// blocks of 512 in the cluster that refreshes a system of n atoms: one
+// thread per atom up to the portable cluster size
+int refresh_blocks(int n)
+{
+    int b = 1;
+    while (b < 8 && b * 512 < n) b <<= 1;
+    return b;
 }
 
 } // namespace
 
-// One refresh: optional integrator start step, then re-binning.  All
-// launches go to the system's stream; graph-capturable (no host reads).
+// One refresh: optional integrator start step, then re-binning and the
+// per-atom tables.  All launches go to the system's stream; graph-capturable
+// (no host reads).
 int fmdg_launch_refresh(fmdg_sys_t *s, int mode, double dt, int group, int thermostat)
 {
     Geo &g = s->g;
@@ -404,39 +561,50 @@ int fmdg_launch_refresh(fmdg_sys_t *s, int mode, double dt, int group, int therm
     g.st.group = group;
     g.st.thermostat = thermostat;
     const LocOne L{g};
+    if (g.cap <= CLUSTER_ATOMS)
+    {
+        const int b = refresh_blocks(g.cap);
+        FMDG_CK(launch_cluster(k_refresh_cluster<LocOne>, L, mode, b, 512, b, st));
+        s->launches++;
+        return FMDG_OK;
+    }
     // dep_count, arr_lower, arr_total, bucket_fill are contiguous
     FMDG_CK(cudaMemsetAsync(g.dep_count, 0, sizeof(int) * 4 * (size_t)g.ncell, st));
-    k_bin_classify<<<fmdg_grid(g.cap, 256), 256, 0, st>>>(L, mode, 0);
-    k_bin_scan<<<1, 1024, 0, st>>>(L);
+    k_bin_classify<<<fmdg_grid(g.cap, 256), 256, 0, st>>>(L, mode);
+    {
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = 8;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(8);
+        cfg.blockDim = dim3(1024);
+        cfg.stream = st;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        FMDG_CK(cudaLaunchKernelEx(&cfg, k_bin_scan, L));
+    }
     k_bin_cells<<<fmdg_grid(g.ncell, 128), 128, 0, st>>>(L);
     k_bin_arrivals<<<fmdg_grid(g.ncell, 128), 128, 0, st>>>(L);
-    k_bin_scatter<<<fmdg_grid(g.cap, 256), 256, 0, st>>>(L);
-    k_bin_flip<<<1, 32, 0, st>>>(L, mode);
-    s->launches += 6;
+    k_bin_place<<<fmdg_grid(g.cap, 256), 256, 0, st>>>(L, mode);
+    s->launches += 5;
     FMDG_CK(cudaGetLastError());
     return FMDG_OK;
 }
 
 // Step start of every system of a pack: velocity-Verlet start step, slot
-// tables and displacement test (fmdg_skin_launch_start), then the cell
-// refresh of the systems that rebuild their skin list this step (between
-// rebuilds an atom stays within skin/2 of its build position, less than a
-// cell, and the packed kernels address atoms by slot, not by cell).
-// Returns the kernels launched, or minus a status.
+// tables and displacement test (k_skin_start), then the cell refresh of the
+// systems that rebuild their skin list this step.  Returns the kernels
+// launched, or minus a status.
 int fmdg_pack_launch_refresh(const fmdg_pack_launch &P)
 {
     cudaStream_t st = P.stream;
-    const int nab = P.la.bstart[P.nsys], ncb = P.lc.bstart[P.nsys];
     int n = fmdg_pack_launch_start(P);
     if (n < 0) return n;
-    k_bin_clear<<<ncb, 128, 0, st>>>(P.lc);
-    k_bin_classify<<<nab, 128, 0, st>>>(P.la, FMDG_REFRESH_ONLY, 1);
-    k_bin_scan<<<P.nsys, 1024, 0, st>>>(P.ls);
-    k_bin_cells<<<ncb, 128, 0, st>>>(P.lc);
-    k_bin_arrivals<<<ncb, 128, 0, st>>>(P.lc);
-    k_bin_scatter<<<nab, 128, 0, st>>>(P.la);
-    k_bin_flip<<<P.nsys, 32, 0, st>>>(P.ls, FMDG_REFRESH_ONLY);
-    cudaError_t e = cudaGetLastError();
+    int most = 1;
+    for (int k = 0; k < P.nsys; k++) most = P.la.geos[k].cap > most ? P.la.geos[k].cap : most;
+    const int b = refresh_blocks(most);
+    const cudaError_t e = launch_cluster(k_refresh_cluster<LocPack>, P.la, FMDG_REFRESH_ONLY, b * P.nsys, 512, b, st);
     if (e != cudaSuccess) return -fmdg_fail("pack refresh", e);
-    return n + 7;
+    return n + 1;
 }

@@ -917,7 +917,7 @@ extern "C" int fmdg_refresh(fmdg_sys_t *s)
 extern "C" int fmdg_compute_forces(fmdg_sys_t *s, int active_group)
 {
     if (!s->atoms || !s->cats) return FMDG_E_STATE;
-    return fmdg_launch_forces(s, active_group, 0, 0.0, 0, 1.0, 0.0);
+    return fmdg_launch_forces(s, active_group, 0, 0.0, 0, 1.0, 0.0, false);
 }
 
 extern "C" int fmdg_thermo(fmdg_sys_t *s, int active_group, fmdg_thermo_t *out)
@@ -932,7 +932,7 @@ static int vv_step_launches(fmdg_sys_t *s, double dt, int group, int thermostat,
 {
     int rc = fmdg_launch_refresh(s, FMDG_REFRESH_VV, dt, group, thermostat);
     if (rc) return rc;
-    rc = fmdg_launch_forces(s, group, 1, dt, thermostat, tau, T0);
+    rc = fmdg_launch_forces(s, group, 1, dt, thermostat, tau, T0, true);
     if (rc) return rc;
     // fields of every turi after the step (src/integrators.c:258-259)
     for (int k = 0; k < s->nturi; k++)
@@ -947,7 +947,7 @@ static int se_step_launches(fmdg_sys_t *s, double dt, int group)
     if (rc) return rc;
     for (int k = 0; k < s->nturi; k++)
         if ((rc = fmdg_launch_turi(s, k, dt))) return rc;
-    return fmdg_launch_forces(s, group, 0, dt, 0, 1.0, 0.0);
+    return fmdg_launch_forces(s, group, 0, dt, 0, 1.0, 0.0, true);
 }
 
 // Before the first step of a run the caller computes the forces of the
@@ -975,7 +975,7 @@ extern "C" int fmdg_vv_steps(fmdg_sys_t *s, int nsteps, double dt, int active_gr
             int rc = fmdg_launch_refresh(s, FMDG_REFRESH_VV, dt, active_group, thermostat);
             if (rc) return rc;
             FMDG_CK(cudaEventRecord(s->pev[1], s->stream));
-            if ((rc = fmdg_launch_nlist(s))) return rc;
+            if ((rc = fmdg_launch_nlist(s, true))) return rc;
             FMDG_CK(cudaEventRecord(s->pev[2], s->stream));
             if ((rc = fmdg_launch_density(s, active_group))) return rc;
             FMDG_CK(cudaEventRecord(s->pev[3], s->stream));
@@ -1008,6 +1008,7 @@ extern "C" int fmdg_vv_steps(fmdg_sys_t *s, int nsteps, double dt, int active_gr
         cudaError_t e = cudaStreamEndCapture(s->stream, &graph);
         if (rc) return rc;
         if (e != cudaSuccess) return fmdg_fail("cudaStreamEndCapture", e);
+        s->graph_steps = (int)(s->launches - before);     // kernels of the captured step
         s->launches = before;
         e = cudaGraphInstantiate(&s->graph, graph, 0);
         cudaGraphDestroy(graph);
@@ -1016,14 +1017,9 @@ extern "C" int fmdg_vv_steps(fmdg_sys_t *s, int nsteps, double dt, int active_gr
         s->graph_dt = dt; s->graph_group = active_group; s->graph_thermo = thermostat;
         s->graph_tau = tau; s->graph_T0 = T0;
         s->graph_mode = 0;
-        // kernels per captured step
-        const bool eam = (s->cats & (1 << FMDG_POT_EAM)) != 0;
-        // memset node + 6 refresh kernels + 2 list kernels + density + force
-        s->graph_steps = 7 + 2 + (eam ? 1 : 0) + 1;
-        for (int k = 0; k < s->nturi; k++) s->graph_steps += 5 + (s->turi[k].ttm ? 1 : 0);
     }
     for (int k = 0; k < nsteps; k++) FMDG_CK(cudaGraphLaunch(s->graph, s->stream));
-    s->launches += (long long)nsteps * (s->graph_steps - 1);  // memset node is not a kernel
+    s->launches += (long long)nsteps * s->graph_steps;
     return FMDG_OK;
 }
 
@@ -1049,7 +1045,7 @@ extern "C" int fmdg_se_steps(fmdg_sys_t *s, int nsteps, double dt, int active_gr
             for (int q = 0; q < s->nturi; q++)
                 if ((rc = fmdg_launch_ttm_solve(s, q, dt))) return rc;
             FMDG_CK(cudaEventRecord(s->pev[3], s->stream));
-            if ((rc = fmdg_launch_forces(s, active_group, 0, dt, 0, 1.0, 0.0))) return rc;
+            if ((rc = fmdg_launch_forces(s, active_group, 0, dt, 0, 1.0, 0.0, true))) return rc;
             FMDG_CK(cudaEventRecord(s->pev[4], s->stream));
             FMDG_CK(cudaEventSynchronize(s->pev[4]));
             const int phase[4] = {0, 4, 5, 3};
@@ -1074,7 +1070,7 @@ extern "C" int fmdg_se_steps(fmdg_sys_t *s, int nsteps, double dt, int active_gr
         cudaError_t e = cudaStreamEndCapture(s->stream, &graph);
         if (rc) return rc;
         if (e != cudaSuccess) return fmdg_fail("cudaStreamEndCapture", e);
-        s->graph_steps = (int)(s->launches - before) + 1;
+        s->graph_steps = (int)(s->launches - before);
         s->launches = before;
         e = cudaGraphInstantiate(&s->graph, graph, 0);
         cudaGraphDestroy(graph);
@@ -1085,7 +1081,7 @@ extern "C" int fmdg_se_steps(fmdg_sys_t *s, int nsteps, double dt, int active_gr
         s->graph_group = active_group;
     }
     for (int k = 0; k < nsteps; k++) FMDG_CK(cudaGraphLaunch(s->graph, s->stream));
-    s->launches += (long long)nsteps * (s->graph_steps - 1);
+    s->launches += (long long)nsteps * s->graph_steps;
     return FMDG_OK;
 }
 

@@ -42,6 +42,7 @@
 // converted to binary64 per atom.  Pairs within 1e-4 relative of a cutoff
 // are re-tested in binary64 so both modes include exactly the same pairs.
 #include "fmdg_pairs.cuh"
+#include "fmdg_prep.cuh"
 
 namespace {
 
@@ -152,22 +153,9 @@ __global__ void k_prep_local(__grid_constant__ const L loc)
     const int i = bx * blockDim.x + threadIdx.x;
     if (i >= dyn->n) return;
     const Side S = g.side[dyn->cur];
-    const double4_32a oc = g.corig[S.cell_of[i]];
     const int cap = g.cap;
-    const double ux = S.x[i] - oc.x;
-    const double uy = S.x[cap + i] - oc.y;
-    const double uz = S.x[2 * (size_t)cap + i] - oc.z;
-    const float lx = (float)ux, ly = (float)uy, lz = (float)uz;
-    const float4 hi = make_float4(lx, ly, lz, __int_as_float((int)S.kind[i]));
-    g.xf4[i] = hi;
-    // binary64 mode: hi and the remainders side by side, the double-float
-    // cell-local position in one 32-byte row
-    if (g.prec == FMDG_PREC_FP64)
-    {
-        g.xdf[2 * (size_t)i] = hi;
-        g.xdf[2 * (size_t)i + 1] =
-            make_float4((float)(ux - (double)lx), (float)(uy - (double)ly), (float)(uz - (double)lz), 0.f);
-    }
+    const double x[3] = {S.x[i], S.x[cap + i], S.x[2 * (size_t)cap + i]};
+    prep_local_atom(g, i, S.cell_of[i], (int)S.kind[i], x);
 }
 
 template <class L>
@@ -592,7 +580,7 @@ namespace {
 template <class L>
 void launch_nlist_t(const L &loc, int n_prep, int prep_threads, int nb, int blk, cudaStream_t st)
 {
-    k_prep_local<<<n_prep, prep_threads, 0, st>>>(loc);
+    if (n_prep > 0) k_prep_local<<<n_prep, prep_threads, 0, st>>>(loc);
     k_nlist<<<nb, blk, 0, st>>>(loc);
 }
 
@@ -623,11 +611,12 @@ void launch_force_t(const L &loc, int cats, int finish, int nb, int blk, cudaStr
 
 } // namespace
 
-int fmdg_launch_nlist(fmdg_sys_t *s)
+// prepped: a refresh has just written the per-atom tables
+int fmdg_launch_nlist(fmdg_sys_t *s, bool prepped)
 {
-    if (s->g.skin_on) return fmdg_skin_launch_nlist(s);
-    launch_nlist_t(LocOne{s->g}, fmdg_grid(s->g.cap, 256), 256, fmdg_force_blocks(s), s->fblk, s->stream);
-    s->launches += 2;
+    if (s->g.skin_on) return fmdg_skin_launch_nlist(s, prepped);
+    launch_nlist_t(LocOne{s->g}, prepped ? 0 : fmdg_grid(s->g.cap, 256), 256, fmdg_force_blocks(s), s->fblk, s->stream);
+    s->launches += prepped ? 1 : 2;
     FMDG_CK(cudaGetLastError());
     return FMDG_OK;
 }
@@ -665,9 +654,10 @@ int fmdg_launch_pair_forces(fmdg_sys_t *s, int group, int finish, double dt, int
     return FMDG_OK;
 }
 
-int fmdg_launch_forces(fmdg_sys_t *s, int group, int finish, double dt, int thermostat, double tau, double T0)
+int fmdg_launch_forces(fmdg_sys_t *s, int group, int finish, double dt, int thermostat, double tau, double T0,
+                       bool prepped)
 {
-    int rc = fmdg_launch_nlist(s);
+    int rc = fmdg_launch_nlist(s, prepped);
     if (rc) return rc;
     if ((rc = fmdg_launch_density(s, group))) return rc;
     return fmdg_launch_pair_forces(s, group, finish, dt, thermostat, tau, T0);

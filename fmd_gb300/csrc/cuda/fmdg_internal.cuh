@@ -34,7 +34,7 @@ struct Dyn
     int steps_left;     // packed launches: steps this system still takes
     int rebuild;        // skin list: rebuild before the next force pass
     unsigned nl_done;   // ticket of the skin-list build's last block
-    int pad;
+    unsigned place_done;    // ticket of the refresh's last block
     double lambda;      // Berendsen scale for the next start step
     double time;        // simulation time (advanced by every step)
     double dt;          // time step of the current run (turi windows)
@@ -311,9 +311,7 @@ struct fmdg_pack_launch
     int shares;                 // the members' list walks are split into shares (small systems)
     int fblk;                   // threads per block of the list/density/force kernels
     LocPack la;                 // 128-thread atom blocks
-    LocPack lc;                 // 128-thread cell blocks
     LocPack lf;                 // force blocks of fblk threads
-    LocPack ls;                 // one block per system
 };
 // all three return the number of kernels launched, or minus a status
 int fmdg_pack_launch_start(const fmdg_pack_launch &P);
@@ -336,9 +334,10 @@ int fmdg_launch_turi(fmdg_sys_t *s, int k, double dt);
 // the two halves of fmdg_launch_turi: the field passes, then the TTM solver
 int fmdg_launch_turi_fields(fmdg_sys_t *s, int k, double dt);
 int fmdg_launch_ttm_solve(fmdg_sys_t *s, int k, double dt);
-int fmdg_launch_forces(fmdg_sys_t *s, int group, int finish, double dt, int thermostat, double tau, double T0);
+int fmdg_launch_forces(fmdg_sys_t *s, int group, int finish, double dt, int thermostat, double tau, double T0,
+                       bool prepped);
 int fmdg_launch_density(fmdg_sys_t *s, int group);
-int fmdg_launch_nlist(fmdg_sys_t *s);
+int fmdg_launch_nlist(fmdg_sys_t *s, bool prepped);
 int fmdg_pack_tables(fmdg_sys_t *s);
 int fmdg_launch_pair_forces(fmdg_sys_t *s, int group, int finish, double dt, int thermostat, double tau, double T0);
 int fmdg_launch_thermo(fmdg_sys_t *s, int group, int thermostat, double dt, double tau, double T0);
@@ -349,7 +348,7 @@ int fmdg_list_capacity(const fmdg_sys_t *s, const int *cell_count, int ncell);
 size_t fmdg_bytes_estimate(int n, int ncell, int maxnb, int prec);
 int fmdg_set_steps_left(fmdg_sys_t *s, int steps);
 // single-system path on a skin list (fmdg_skin.cu)
-int fmdg_skin_launch_nlist(fmdg_sys_t *s);
+int fmdg_skin_launch_nlist(fmdg_sys_t *s, bool prepped);
 int fmdg_skin_launch_density(fmdg_sys_t *s);
 int fmdg_skin_launch_pair_forces(fmdg_sys_t *s, int finish);
 

@@ -421,7 +421,7 @@ int rebuild(fmdg_server_t *S, Pack &p)
     P.shares = p.shares;
     P.mixed = p.mixed;
     P.fblk = fblk;
-    LocPack *locs[4] = {&P.la, &P.lc, &P.lf, &P.ls};
+    LocPack *locs[2] = {&P.la, &P.lf};
     for (LocPack *L : locs)
     {
         L->nsys = P.nsys;
@@ -435,9 +435,7 @@ int rebuild(fmdg_server_t *S, Pack &p)
         s->g.lane_log = (unsigned char)std::max(0, s->g.share_log - level);
         for (LocPack *L : locs) L->geos[k] = s->g;
         P.la.bstart[k + 1] = P.la.bstart[k] + fmdg_grid(s->g.cap, 128);
-        P.lc.bstart[k + 1] = P.lc.bstart[k] + fmdg_grid(s->g.ncell, 128);
         P.lf.bstart[k + 1] = P.lf.bstart[k] + fmdg_grid(s->g.cap << s->g.lane_log, fblk);
-        P.ls.bstart[k + 1] = k + 1;
     }
     // members set up on their own streams must be ready before the chunk
     for (Job *j : p.members)

@@ -41,6 +41,7 @@
 #include <type_traits>
 
 #include "fmdg_pairs.cuh"
+#include "fmdg_prep.cuh"
 
 namespace {
 
@@ -393,39 +394,6 @@ __device__ __forceinline__ dfl group_sum(dfl v, int G)
 
 // ---------------------------------------------------------------- kernels
 
-// Slot t's binary32 position relative to the cell it had at the last build
-// (unwrapped across periodic faces) and the displacement test against its
-// build position: sets the rebuild flag beyond skin/2.
-__device__ __forceinline__ void slot_rel_build(const Geo &g, Dyn *dyn, int t, const double (&x)[3], float kb)
-{
-    const double4_32a ob = g.corig[g.cb[t]];
-    const double o3[3] = {ob.x, ob.y, ob.z};
-    float l3[3];
-    double u3[3];
-    const double xs = g.xs;     // (1 in binary64 mode: xll below holds remainders of unscaled values)
-    for (int d = 0; d < 3; d++)
-    {
-        double u = x[d] - o3[d];
-        float uf = d2f_rn(u * xs);
-        // unwrap across a periodic face (binary64 test near half a box)
-        if (g.pbc[d] && fabsf(uf) > 0.49f * g.l_f[d])
-        {
-            if (u > 0.5 * g.l[d]) u -= g.l[d];
-            else if (u < -0.5 * g.l[d]) u += g.l[d];
-            uf = d2f_rn(u * xs);
-        }
-        l3[d] = uf;
-        u3[d] = u;
-    }
-    g.xl[t] = make_float4(l3[0], l3[1], l3[2], kb);
-    if (g.prec == FMDG_PREC_FP64)
-        g.xll[t] = make_float4((float)(u3[0] - (double)l3[0]), (float)(u3[1] - (double)l3[1]),
-                               (float)(u3[2] - (double)l3[2]), 0.f);
-    const float4 o = g.xb[t];
-    const float dx = l3[0] - o.x, dy = l3[1] - o.y, dz = l3[2] - o.z;
-    if (!(dx * dx + dy * dy + dz * dz <= g.half_skin2)) dyn->rebuild = 1;
-}
-
 // Packed systems, every step (one thread per current atom index): the
 // velocity-Verlet start step (src/integrators.c:40-75, the operations of
 // k_bin_classify), the slot tables that change every step and the
@@ -469,50 +437,18 @@ __global__ void k_skin_start(__grid_constant__ const L loc)
     slot_rel_build(g, dyn, t, x, __int_as_float(kind));
 }
 
-// one thread per current atom index.  lazy (packed systems): rebuild steps
-// only, after the cell refresh, and the slots are renumbered in the
-// current (cell) order -- slot = index, so the rebuild walks and writes
-// consecutive atoms of a cell together, and until the next rebuild (no
-// refresh in between) every slot-to-index map is the identity
-template <class L>
-__global__ void k_prep_skin(__grid_constant__ const L loc, int lazy)
+// The per-atom tables of the current positions (prep_atom), one thread per
+// atom, for a force evaluation without a refresh before it
+__global__ void __launch_bounds__(128) k_prep_skin(__grid_constant__ const LocOne loc)
 {
-    int bx, nb;
-    const Geo &g = loc_geo(loc, bx, nb);
-    if (loc_idle(loc, g)) return;
+    const Geo &g = loc.g;
     Dyn *dyn = g.dyn;
-    if (lazy && !dyn->rebuild) return;
-    const int i = bx * blockDim.x + threadIdx.x;
-    if (i >= dyn->n)
-    {
-        if (lazy && i < g.cap) g.pos[i] = -1;
-        return;
-    }
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= dyn->n) return;
     const Side S = g.side[dyn->cur];
     const int cap = g.cap;
-    const int t = lazy ? i : S.slot[i];
-    if (lazy) S.slot[i] = i;
     const double x[3] = {S.x[i], S.x[cap + i], S.x[2 * (size_t)cap + i]};
-    const int kind = (int)S.kind[i];
-    const float kb = __int_as_float(kind);
-    g.pos[t] = i;
-    g.xd[t] = make_double4_32a(x[0], x[1], x[2], 0.0);
-    g.gslot[t] = S.group[i];
-    // relative to the current cell (a rebuild starts from these)
-    const double4_32a oc = g.corig[S.cell_of[i]];
-    const double ux = x[0] - oc.x, uy = x[1] - oc.y, uz = x[2] - oc.z;
-    const double xs = g.xs;     // (1 in binary64 mode: the remainders below are of unscaled values)
-    const float lx = (float)(ux * xs), ly = (float)(uy * xs), lz = (float)(uz * xs);
-    g.xf4[i] = make_float4(lx, ly, lz, kb);
-    if (g.prec == FMDG_PREC_FP64)
-    {
-        g.xdf[2 * (size_t)i] = make_float4(lx, ly, lz, kb);
-        g.xdf[2 * (size_t)i + 1] =
-            make_float4((float)(ux - (double)lx), (float)(uy - (double)ly), (float)(uz - (double)lz), 0.f);
-    }
-    // (renumbered, or a rebuild already due: the build cell and position of
-    // slot t are rewritten by the list build that follows)
-    if (!lazy && !dyn->rebuild) slot_rel_build(g, dyn, t, x, kb);
+    prep_skin_atom(g, dyn, i, S.slot[i], S.cell_of[i], (int)S.kind[i], S.group[i], x, !dyn->rebuild);
 }
 
 // The stencil walk of a list build: f(code, c, ax, ay, az) for every cell
@@ -535,7 +471,13 @@ __device__ __forceinline__ void record_build(const Geo &g, const Side &S, int t,
     g.cb[t] = S.cell_of[i];
     g.xl[t] = xi;
     g.xb[t] = xi;
-    if (g.prec == FMDG_PREC_FP64) g.xll[t] = g.xdf[2 * (size_t)i + 1];
+    if (g.prec == FMDG_PREC_FP64)
+    {
+        // (xs is 1 in binary64 mode)
+        const double4_32a x = g.xd[t], o = g.corig[S.cell_of[i]];
+        g.xll[t] = make_float4((float)(x.x - o.x - (double)xi.x), (float)(x.y - o.y - (double)xi.y),
+                               (float)(x.z - o.z - (double)xi.z), 0.f);
+    }
 }
 
 // the last block of a build to finish clears the system's rebuild flag
@@ -1419,7 +1361,7 @@ int fmdg_pack_launch_start(const fmdg_pack_launch &P)
     return 1;
 }
 
-// phases: bit 0 slot tables + list (re)build, bit 1 EAM density, bit 2
+// phases: bit 0 list (re)build, bit 1 EAM density, bit 2
 // pair forces + finish step (all three for a step).  Returns the kernels
 // launched, or minus a status.
 int fmdg_pack_launch_forces(const fmdg_pack_launch &P, int phases)
@@ -1429,9 +1371,8 @@ int fmdg_pack_launch_forces(const fmdg_pack_launch &P, int phases)
     int n = 0;
     if (phases & 1)
     {
-        k_prep_skin<<<nab, 128, 0, st>>>(P.la, 1);
         k_nlist_skin<<<nab, 128, 0, st>>>(P.la);
-        n += 2;
+        n++;
     }
     if ((phases & 2) && (P.cats & (1 << FMDG_POT_EAM)))
     {
@@ -1459,10 +1400,15 @@ int fmdg_pack_launch_forces(const fmdg_pack_launch &P, int phases)
 // The single-system path on a skin list (fmdg_launch_nlist/density/
 // pair_forces dispatch here when the system has one): slot tables + list
 // (re)build; EAM density; pair forces (+ finish step).
-int fmdg_skin_launch_nlist(fmdg_sys_t *s)
+// prepped: a refresh has just written the per-atom tables.
+int fmdg_skin_launch_nlist(fmdg_sys_t *s, bool prepped)
 {
     const LocOne L{s->g};
-    k_prep_skin<<<fmdg_grid(s->g.cap, 128), 128, 0, s->stream>>>(L, 0);
+    if (!prepped)
+    {
+        k_prep_skin<<<fmdg_grid(s->g.cap, 128), 128, 0, s->stream>>>(L);
+        s->launches++;
+    }
     // lanes per slot by size, from build times measured on GB300 (LJ,
     // Morse, EAM jobs of 2k-190k atoms): 16 up to 2^14 slots, 8 up to 2^16,
     // then one thread per slot (enough warps; a group's ballots cost more
@@ -1481,7 +1427,7 @@ int fmdg_skin_launch_nlist(fmdg_sys_t *s)
     case 32: k_nlist_skin_grp<32><<<nbg, 128, 0, s->stream>>>(L); break;
     default: k_nlist_skin<<<nbg, 128, 0, s->stream>>>(L); break;
     }
-    s->launches += 2;
+    s->launches++;
     FMDG_CK(cudaGetLastError());
     return FMDG_OK;
 }
