@@ -69,6 +69,16 @@ int d2h_sync(fmdg_sys_t *s, void *dst, const void *src, size_t n)
 
 void dfree(fmdg_sys_t *s, void *p) { if (p) cudaFreeAsync(p, s->stream); }
 
+void invalidate_graph(fmdg_sys_t *s)
+{
+    for (cudaGraphExec_t &g : s->graph)
+    {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    }
+    s->graph_key_valid = 0;
+}
+
 void free_atoms(fmdg_sys_t *s)
 {
     Geo &g = s->g;
@@ -85,7 +95,7 @@ void free_atoms(fmdg_sys_t *s)
     g.fpb = nullptr; g.fpd = nullptr;
     g.cap = 0;
     s->atoms = false;
-    if (s->graph_key_valid) { cudaGraphExecDestroy(s->graph); s->graph_key_valid = 0; }
+    invalidate_graph(s);
 }
 
 // Lays the per-atom and per-cell buffers of a system out in one device
@@ -111,11 +121,6 @@ void drop_eam(fmdg_sys_t *s)
     g.pkf_rho = g.pkf_phi = g.pkf_F = g.pkf_pr = nullptr;
     g.pkd_rho = g.pkd_phi = nullptr;
     s->eam_borrowed = false;
-}
-
-void invalidate_graph(fmdg_sys_t *s)
-{
-    if (s->graph_key_valid) { cudaGraphExecDestroy(s->graph); s->graph_key_valid = 0; }
 }
 
 int read_dyn(fmdg_sys_t *s, Dyn *out)
@@ -264,6 +269,7 @@ extern "C" int fmdg_create(fmdg_sys_t **out, int device)
     FMDG_CK(cudaMemsetAsync(s->g.thermo, 0, sizeof(fmdg_thermo_t), s->stream));
     s->ttm_turi = -1;
     s->fblk = 128;
+    s->rec = REC_FULL;
     // Verlet skin of the neighbour list (A) of mixed-precision systems;
     // FMD_SKIN=0 keeps the exact per-step stencil list
     s->skin = 0.5;
@@ -950,6 +956,43 @@ static int se_step_launches(fmdg_sys_t *s, double dt, int group)
     return fmdg_launch_forces(s, group, 0, dt, 0, 1.0, 0.0, true);
 }
 
+// nsteps replays of the captured step `launches`: all but the last leave
+// only what the next step needs (`between`), the last one the thermo record,
+// which the host reads between batches only.  Each form is captured when it
+// is first needed.
+template <typename F>
+static int replay_steps(fmdg_sys_t *s, int nsteps, int between, F &&launches)
+{
+    for (int form = nsteps > 1 ? 0 : 1; form < 2; form++)
+    {
+        if (!s->graph[form])
+        {
+            cudaGraph_t graph;
+            FMDG_CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
+            const long long before = s->launches;
+            s->rec = form ? REC_FULL : between;
+            const int rc = launches();
+            s->rec = REC_FULL;
+            const cudaError_t e = cudaStreamEndCapture(s->stream, &graph);
+            s->graph_kernels[form] = (int)(s->launches - before);
+            s->launches = before;
+            if (rc) return rc;
+            if (e != cudaSuccess) return fmdg_fail("cudaStreamEndCapture", e);
+            const cudaError_t ei = cudaGraphInstantiate(&s->graph[form], graph, 0);
+            cudaGraphDestroy(graph);
+            if (ei != cudaSuccess)
+            {
+                s->graph[form] = nullptr;
+                return fmdg_fail("cudaGraphInstantiate", ei);
+            }
+        }
+        const int k = form ? 1 : nsteps - 1;
+        for (int q = 0; q < k; q++) FMDG_CK(cudaGraphLaunch(s->graph[form], s->stream));
+        s->launches += (long long)k * s->graph_kernels[form];
+    }
+    return FMDG_OK;
+}
+
 // Before the first step of a run the caller computes the forces of the
 // current positions (fmdg_compute_forces) and, with a thermostat, sets the
 // scale from the current temperature (fmdg_prepare_thermostat); each step
@@ -1001,26 +1044,13 @@ extern "C" int fmdg_vv_steps(fmdg_sys_t *s, int nsteps, double dt, int active_gr
     if (!same)
     {
         invalidate_graph(s);
-        cudaGraph_t graph;
-        FMDG_CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-        const long long before = s->launches;
-        int rc = vv_step_launches(s, dt, active_group, thermostat, tau, T0);
-        cudaError_t e = cudaStreamEndCapture(s->stream, &graph);
-        if (rc) return rc;
-        if (e != cudaSuccess) return fmdg_fail("cudaStreamEndCapture", e);
-        s->graph_steps = (int)(s->launches - before);     // kernels of the captured step
-        s->launches = before;
-        e = cudaGraphInstantiate(&s->graph, graph, 0);
-        cudaGraphDestroy(graph);
-        if (e != cudaSuccess) return fmdg_fail("cudaGraphInstantiate", e);
         s->graph_key_valid = 1;
         s->graph_dt = dt; s->graph_group = active_group; s->graph_thermo = thermostat;
         s->graph_tau = tau; s->graph_T0 = T0;
         s->graph_mode = 0;
     }
-    for (int k = 0; k < nsteps; k++) FMDG_CK(cudaGraphLaunch(s->graph, s->stream));
-    s->launches += (long long)nsteps * s->graph_steps;
-    return FMDG_OK;
+    return replay_steps(s, nsteps, thermostat ? REC_LAMBDA : REC_NONE,
+                        [&]() { return vv_step_launches(s, dt, active_group, thermostat, tau, T0); });
 }
 
 extern "C" int fmdg_se_steps(fmdg_sys_t *s, int nsteps, double dt, int active_group)
@@ -1063,26 +1093,12 @@ extern "C" int fmdg_se_steps(fmdg_sys_t *s, int nsteps, double dt, int active_gr
     if (!same)
     {
         invalidate_graph(s);
-        cudaGraph_t graph;
-        FMDG_CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-        const long long before = s->launches;
-        int rc = se_step_launches(s, dt, active_group);
-        cudaError_t e = cudaStreamEndCapture(s->stream, &graph);
-        if (rc) return rc;
-        if (e != cudaSuccess) return fmdg_fail("cudaStreamEndCapture", e);
-        s->graph_steps = (int)(s->launches - before);
-        s->launches = before;
-        e = cudaGraphInstantiate(&s->graph, graph, 0);
-        cudaGraphDestroy(graph);
-        if (e != cudaSuccess) return fmdg_fail("cudaGraphInstantiate", e);
         s->graph_key_valid = 1;
         s->graph_mode = 1;
         s->graph_dt = dt;
         s->graph_group = active_group;
     }
-    for (int k = 0; k < nsteps; k++) FMDG_CK(cudaGraphLaunch(s->graph, s->stream));
-    s->launches += (long long)nsteps * s->graph_steps;
-    return FMDG_OK;
+    return replay_steps(s, nsteps, REC_NONE, [&]() { return se_step_launches(s, dt, active_group); });
 }
 
 extern "C" int fmdg_set_time(fmdg_sys_t *s, double time, double dt)

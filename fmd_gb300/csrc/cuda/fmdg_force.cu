@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_nlist(__grid_
 // EAM pass 1 + embedding: rho_i = sum_j f_{elem(j)}(r_ij^2) (src/eam.h:270-406),
 // vaream_i = F'(rho_i), energy F(rho_i) (src/eam.c:160-179).
 template <class L, bool MIXED, bool HYBRID>
-__global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density(__grid_constant__ const L loc)
+__global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density(__grid_constant__ const L loc, int rec)
 {
     int bx, nb;
     const Geo &g = loc_geo(loc, bx, nb);
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density(__gri
             else g.fpdf[i] = make_float2(0.f, 0.f);
         }
     }
-    block_reduce_store<1>(acc, g.partials + (size_t)nb * 8 + bx, blockDim.x);
+    if (rec == REC_FULL) block_reduce_store<1>(acc, g.partials + (size_t)nb * 8 + bx, blockDim.x);
 }
 
 __global__ void k_reduce_final(Geo g, int nblocks, int keep_pe, int with_emb, int thermostat,
@@ -337,7 +337,7 @@ __global__ void k_reduce_final(Geo g, int nblocks, int keep_pe, int with_emb, in
 // Pair forces + per-atom half energies; with finish=1 also the
 // velocity-Verlet finishStep (src/integrators.c:94-126) and its reductions.
 template <class L, int CAT, bool MIXED>
-__global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_force(__grid_constant__ const L loc, int finish)
+__global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_force(__grid_constant__ const L loc, int finish, int rec)
 {
     int bx, nb;
     const Geo &g = loc_geo(loc, bx, nb);
@@ -519,6 +519,7 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_force(__grid_
             acc[5] = 1.0;
         }
     }
+    if (rec == REC_NONE) return;
     __shared__ double blk[7];
     __shared__ unsigned ticket;
     block_reduce_store<7>(acc, blk, blockDim.x);
@@ -533,12 +534,10 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_force(__grid_
     if (ticket == (unsigned)nb - 1)
     {
         __threadfence();
-        final_reduce(g, nb, 0, g.has_eam, g.st.thermostat, dt, g.st.tau, g.st.T0);
+        if (rec == REC_FULL) final_reduce(g, nb, 0, g.has_eam, g.st.thermostat, dt, g.st.tau, g.st.T0);
+        else final_lambda(g, nb, dt, g.st.tau, g.st.T0);
         if (threadIdx.x == 0)
-        {
             g.dyn->blocks_done = 0;
-            if (finish && g.dyn->steps_left > 0) g.dyn->steps_left--;
-        }
     }
 }
 
@@ -585,28 +584,28 @@ void launch_nlist_t(const L &loc, int n_prep, int prep_threads, int nb, int blk,
 }
 
 template <class L>
-void launch_density_t(const L &loc, bool mixed, bool hyb, int nb, int blk, cudaStream_t st)
+void launch_density_t(const L &loc, bool mixed, bool hyb, int rec, int nb, int blk, cudaStream_t st)
 {
     if (mixed)
     {
-        if (hyb) k_density<L, true, true><<<nb, blk, 0, st>>>(loc);
-        else k_density<L, true, false><<<nb, blk, 0, st>>>(loc);
+        if (hyb) k_density<L, true, true><<<nb, blk, 0, st>>>(loc, rec);
+        else k_density<L, true, false><<<nb, blk, 0, st>>>(loc, rec);
     }
     else
     {
-        if (hyb) k_density<L, false, true><<<nb, blk, 0, st>>>(loc);
-        else k_density<L, false, false><<<nb, blk, 0, st>>>(loc);
+        if (hyb) k_density<L, false, true><<<nb, blk, 0, st>>>(loc, rec);
+        else k_density<L, false, false><<<nb, blk, 0, st>>>(loc, rec);
     }
 }
 
 template <class L, bool MIXED>
-void launch_force_t(const L &loc, int cats, int finish, int nb, int blk, cudaStream_t st)
+void launch_force_t(const L &loc, int cats, int finish, int rec, int nb, int blk, cudaStream_t st)
 {
     const int ncat = __builtin_popcount(cats);
-    if (ncat > 1) k_force<L, CAT_HYBRID, MIXED><<<nb, blk, 0, st>>>(loc, finish);
-    else if (cats == (1 << FMDG_POT_LJ)) k_force<L, CAT_LJ, MIXED><<<nb, blk, 0, st>>>(loc, finish);
-    else if (cats == (1 << FMDG_POT_MORSE)) k_force<L, CAT_MORSE, MIXED><<<nb, blk, 0, st>>>(loc, finish);
-    else k_force<L, CAT_EAM, MIXED><<<nb, blk, 0, st>>>(loc, finish);
+    if (ncat > 1) k_force<L, CAT_HYBRID, MIXED><<<nb, blk, 0, st>>>(loc, finish, rec);
+    else if (cats == (1 << FMDG_POT_LJ)) k_force<L, CAT_LJ, MIXED><<<nb, blk, 0, st>>>(loc, finish, rec);
+    else if (cats == (1 << FMDG_POT_MORSE)) k_force<L, CAT_MORSE, MIXED><<<nb, blk, 0, st>>>(loc, finish, rec);
+    else k_force<L, CAT_EAM, MIXED><<<nb, blk, 0, st>>>(loc, finish, rec);
 }
 
 } // namespace
@@ -628,7 +627,7 @@ int fmdg_launch_density(fmdg_sys_t *s, int group)
     s->g.st.group = group;
     if (s->g.skin_on) return fmdg_skin_launch_density(s);
     launch_density_t(LocOne{s->g}, s->g.prec == FMDG_PREC_MIXED, __builtin_popcount(s->cats) > 1,
-                     fmdg_force_blocks(s), s->fblk, s->stream);
+                     s->rec, fmdg_force_blocks(s), s->fblk, s->stream);
     s->launches++;
     FMDG_CK(cudaGetLastError());
     return FMDG_OK;
@@ -647,8 +646,8 @@ int fmdg_launch_pair_forces(fmdg_sys_t *s, int group, int finish, double dt, int
     if (s->g.skin_on) return fmdg_skin_launch_pair_forces(s, finish);
     const LocOne L{s->g};
     const int nb = fmdg_force_blocks(s);
-    if (s->g.prec == FMDG_PREC_MIXED) launch_force_t<LocOne, true>(L, s->cats, finish, nb, s->fblk, s->stream);
-    else launch_force_t<LocOne, false>(L, s->cats, finish, nb, s->fblk, s->stream);
+    if (s->g.prec == FMDG_PREC_MIXED) launch_force_t<LocOne, true>(L, s->cats, finish, s->rec, nb, s->fblk, s->stream);
+    else launch_force_t<LocOne, false>(L, s->cats, finish, s->rec, nb, s->fblk, s->stream);
     s->launches++;
     FMDG_CK(cudaGetLastError());
     return FMDG_OK;

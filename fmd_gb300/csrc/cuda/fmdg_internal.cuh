@@ -179,11 +179,14 @@ struct fmdg_sys
     float prof_ms[6];
     int prof_n[6];
     long long launches;
-    // captured multi-step graph
-    cudaGraphExec_t graph;
+    int rec;                      // REC_* of the next launches
+    // captured step graphs: [0] a step whose record nobody reads, [1] one
+    // with the thermo record (the last of a batch)
+    cudaGraphExec_t graph[2];
     int graph_key_valid;
     double graph_dt, graph_tau, graph_T0;
-    int graph_group, graph_thermo, graph_steps;
+    int graph_group, graph_thermo;
+    int graph_kernels[2];         // kernels of a captured step
     void *l2buf;
     size_t l2bytes;
     // continuum grids
@@ -235,8 +238,14 @@ inline void set_step_dt(fmdg_sys_t *s, double dt)
 //            steps_left reached zero is skipped by every kernel.
 #define FMDG_PACK_MAX 32
 
+// what a force evaluation leaves besides the forces: nothing (a step whose
+// record the next one overwrites unread), the thermo record, or only the
+// Berendsen scale of the next step
+enum { REC_NONE = 0, REC_FULL = 1, REC_LAMBDA = 2 };
+
 struct LocOne
 {
+    static constexpr bool one_system = true;
     static constexpr int max_threads = 128;
     static constexpr int min_blocks = 0;      // 0: register count left to the compiler
     static constexpr int lean_min_blocks = 7; // lean force kernels: 7 blocks of 128 (72 registers), measured best
@@ -248,6 +257,7 @@ struct LocOne
 
 struct LocPack
 {
+    static constexpr bool one_system = false;
     static constexpr int max_threads = 256;
     static constexpr int min_blocks = 0;
     static constexpr int lean_min_blocks = 0; // packed lean force kernels: compiler's choice, measured best
@@ -291,8 +301,9 @@ __device__ __forceinline__ const Geo &loc_geo(const LocPack &L, int &bx, int &nb
 
 __device__ __forceinline__ bool loc_idle(const LocOne &, const Geo &) { return false; }
 __device__ __forceinline__ bool loc_idle(const LocPack &, const Geo &g) { return g.dyn->steps_left <= 0; }
-// does this step produce a thermo record?  Single systems: every step (the
-// fmd.h API reads it at any time).  Packed (served) systems report theirs
+// does this step produce a thermo record?  Single systems: when the host
+// asks for it (the last step of a batch: the record is read between batches
+// only).  Packed (served) systems report theirs
 // only after their last step, so only that step forms energies, kinetic
 // energy and momentum (uniform over a system's blocks: steps_left changes
 // only after the last of them has finished)

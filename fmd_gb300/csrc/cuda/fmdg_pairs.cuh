@@ -436,6 +436,33 @@ __device__ __forceinline__ void final_reduce(const Geo &g, int nblocks, int keep
     }
 }
 
+// The velocity scale alone (final_reduce's lambda), from the partial rows of
+// m v^2 and the count.  Run by one whole block of at most 256 threads.
+__device__ __forceinline__ void final_lambda(const Geo &g, int nblocks, double dt, double tau, double T0)
+{
+    __shared__ double red[2][8];
+    const int t = threadIdx.x;
+    double a = 0.0, b = 0.0;
+    for (int k = t; k < nblocks; k += blockDim.x)
+    {
+        a += __ldcg(&g.partials[(size_t)nblocks + k]);
+        b += __ldcg(&g.partials[(size_t)5 * nblocks + k]);
+    }
+    for (int off = 16; off > 0; off >>= 1)
+    {
+        a += __shfl_down_sync(0xffffffffu, a, off);
+        b += __shfl_down_sync(0xffffffffu, b, off);
+    }
+    if ((t & 31) == 0) { red[0][t >> 5] = a; red[1][t >> 5] = b; }
+    __syncthreads();
+    if (t == 0)
+    {
+        for (int w = 1; w < (int)(blockDim.x >> 5); w++) { a += red[0][w]; b += red[1][w]; }
+        const double temperature = a / (3.0 * b * K_BOLTZMANN_D);
+        g.dyn->lambda = sqrt(1 + dt / tau * (T0 / temperature - 1));
+    }
+}
+
 // ---- pair terms: force factor f (F_i += f * rv, rv = x_i - x_j) and half
 // the pair energy (each atom of the pair takes half)
 // LJ (src/lj.h:35-56): p = {4 eps, sigma^2, rc^2}

@@ -731,7 +731,7 @@ __device__ __forceinline__ void group_forces(const dfl (&v)[5], int gl, bool the
 // 2^lane_log lanes per slot (see k_force_skin).  LEAN (binary32, one kind, no group): the pair's table
 // row and cutoff in registers, no per-entry kind or group lookups.
 template <class L, bool MIXED, bool HYBRID, bool LEAN>
-__global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density_skin(__grid_constant__ const L loc)
+__global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density_skin(__grid_constant__ const L loc, int rec)
 {
     int bx, nb;
     const Geo &g = loc_geo(loc, bx, nb);
@@ -919,7 +919,7 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density_skin(
             if (!MIXED) g.fpdf[t] = make_float2(0.f, 0.f);
         }
     }
-    if (loc_thermo(loc, g)) block_reduce_store<1>(acc, g.partials + (size_t)nb * 8 + bx, blockDim.x >> gl);
+    if (rec == REC_FULL && loc_thermo(loc, g)) block_reduce_store<1>(acc, g.partials + (size_t)nb * 8 + bx, blockDim.x >> gl);
 }
 
 // Pair forces + velocity-Verlet finish step (src/integrators.c:94-126) and
@@ -928,7 +928,7 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density_skin(
 // group): pair parameters in registers, no per-entry kind or group
 // lookups, hardware exp2 / rsqrt / rcp approximations.
 template <class L, int CAT, bool MIXED, bool LEAN>
-__global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L::min_blocks) k_force_skin(__grid_constant__ const L loc, int finish)
+__global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L::min_blocks) k_force_skin(__grid_constant__ const L loc, int finish, int rec)
 {
     int bx, nb;
     const Geo &g = loc_geo(loc, bx, nb);
@@ -943,7 +943,8 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
     const Side S = g.side[dyn->cur];
     const int cap = g.cap;
     const int gl = L::one_lane ? 0 : g.lane_log, lane = threadIdx.x & ((1 << gl) - 1);
-    const bool thermo = loc_thermo(loc, g);
+    const bool thermo = rec == REC_FULL && loc_thermo(loc, g);
+    const bool sums = thermo || (L::one_system && rec == REC_LAMBDA);      // kinetic sums
     // pe, m v^2, m v (3), count, pair virial
     double acc[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     // this lane's shares of the force (3), energy and virial
@@ -970,7 +971,7 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
                 const dfl fpi = ((CAT == CAT_EAM || CAT == CAT_HYBRID) && on) ? df_of(g.fpdf[t]) : dfl{0.f, 0.f};
                 const dfl inv_h = df_of(df_split(g.inv_dr2));
                 const float kmax = (float)(nint - 1);
-                auto pair = [&](int js, float4 xjf, float4 o) {
+                auto pair = [&](auto with_e, int js, float4 xjf, float4 o) {
                     if (group >= 0 && g.gslot[js] != group) return;
                     const int pidx = ki * nk + __float_as_int(xjf.w);
                     const fmdg_pair_t &pp = sp.pairs[pidx];
@@ -982,14 +983,21 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
                     df_pair(g, sp, pidx, pp, cat, p, fpi, inv_h, kmax, nint, ne, [&]() { return df_of(g.fpdf[js]); },
                             fa, eh);
                     for (int d = 0; d < 3; d++) sum[d] = df_add(sum[d], df_mul(fa, p.rv[d]));
-                    sum[3] = df_add(sum[3], eh);
-                    sum[4] = df_add(sum[4], df_mul(fa, p.r2));     // rv . (fa rv), both sides of the pair
+                    if constexpr (decltype(with_e)::value)
+                    {
+                        sum[3] = df_add(sum[3], eh);
+                        sum[4] = df_add(sum[4], df_mul(fa, p.r2));     // rv . (fa rv), both sides of the pair
+                    }
                 };
+                auto pair_e = [&](int js, float4 xjf, float4 o) { pair(std::true_type{}, js, xjf, o); };
                 const int cnt = on ? g.nbr_count[t] : 0;
                 const int m_in = (CAT == CAT_EAM) ? (on ? g.nbc_count[(size_t)t * V + v] : 0)
                                                   : prune_share(g, so, cnt <= g.maxnb ? cnt : 0, t, v, V, ih);
-                for_each_pruned(g, so, m_in, t, v, V, pair);
-                if (cnt > g.maxnb && v == 0) for_each_slot_overflow(g, S, so, t, i, xi, pair);
+                if (thermo) for_each_pruned(g, so, m_in, t, v, V, pair_e);
+                else
+                    for_each_pruned(g, so, m_in, t, v, V,
+                                    [&](int js, float4 xjf, float4 o) { pair(std::false_type{}, js, xjf, o); });
+                if (cnt > g.maxnb && v == 0) for_each_slot_overflow(g, S, so, t, i, xi, pair_e);
             }
             else if (!on)
                 ;
@@ -1273,7 +1281,7 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
                     S.v[(size_t)d * cap + i] = v[d];
                 }
             }
-            if (thermo)
+            if (sums)
             {
                 acc[1] = m * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
                 acc[2] = m * v[0];
@@ -1285,10 +1293,12 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
     }
     __shared__ double blk[7];
     __shared__ unsigned ticket;
-    if (thermo) block_reduce_store<7>(acc, blk, blockDim.x >> gl);
+    if (sums) block_reduce_store<7>(acc, blk, blockDim.x >> gl);
+    else if (L::one_system)
+        return;     // (nothing for the last block to do)
     if (threadIdx.x == 0)
     {
-        if (thermo)
+        if (sums)
             for (int k = 0; k < 7; k++) g.partials[(size_t)k * nb + bx] = blk[k];
         __threadfence();
         ticket = atomicAdd(&dyn->blocks_done, 1u);
@@ -1298,6 +1308,7 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
     {
         __threadfence();
         if (thermo) final_reduce(g, nb, 0, g.has_eam, g.st.thermostat, dt, g.st.tau, g.st.T0);
+        else if (sums) final_lambda(g, nb, dt, g.st.tau, g.st.T0);
         if (threadIdx.x == 0)
         {
             dyn->blocks_done = 0;
@@ -1306,7 +1317,6 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
     }
 }
 
-// lean: one kind and no group (used in binary32 only)
 // dynamic shared bytes of slot_of_thread for NV values per slot
 size_t stage_bytes(const LocOne &L, int blk, int nv) { return L.g.lane_log ? (size_t)nv * 8 * (blk >> L.g.lane_log) : 0; }
 size_t stage_bytes(const LocPack &L, int blk, int nv)
@@ -1318,36 +1328,36 @@ size_t stage_bytes(const LocPack &L, int blk, int nv)
 }
 
 template <class L, bool MIXED>
-void launch_force_skin(const L &loc, int cats, int finish, int nb, int blk, cudaStream_t st, bool lean)
+void launch_force_skin(const L &loc, int cats, int finish, int rec, int nb, int blk, cudaStream_t st, bool lean)
 {
     const size_t sh = stage_bytes(loc, blk, 5);
     const int ncat = __builtin_popcount(cats);
-    if (ncat > 1) k_force_skin<L, CAT_HYBRID, MIXED, false><<<nb, blk, sh, st>>>(loc, finish);
+    if (ncat > 1) k_force_skin<L, CAT_HYBRID, MIXED, false><<<nb, blk, sh, st>>>(loc, finish, rec);
     else if (MIXED && lean)
     {
-        if (cats == (1 << FMDG_POT_LJ)) k_force_skin<L, CAT_LJ, true, true><<<nb, blk, sh, st>>>(loc, finish);
-        else if (cats == (1 << FMDG_POT_MORSE)) k_force_skin<L, CAT_MORSE, true, true><<<nb, blk, sh, st>>>(loc, finish);
-        else k_force_skin<L, CAT_EAM, true, true><<<nb, blk, sh, st>>>(loc, finish);
+        if (cats == (1 << FMDG_POT_LJ)) k_force_skin<L, CAT_LJ, true, true><<<nb, blk, sh, st>>>(loc, finish, rec);
+        else if (cats == (1 << FMDG_POT_MORSE)) k_force_skin<L, CAT_MORSE, true, true><<<nb, blk, sh, st>>>(loc, finish, rec);
+        else k_force_skin<L, CAT_EAM, true, true><<<nb, blk, sh, st>>>(loc, finish, rec);
     }
-    else if (cats == (1 << FMDG_POT_LJ)) k_force_skin<L, CAT_LJ, MIXED, false><<<nb, blk, sh, st>>>(loc, finish);
-    else if (cats == (1 << FMDG_POT_MORSE)) k_force_skin<L, CAT_MORSE, MIXED, false><<<nb, blk, sh, st>>>(loc, finish);
-    else k_force_skin<L, CAT_EAM, MIXED, false><<<nb, blk, sh, st>>>(loc, finish);
+    else if (cats == (1 << FMDG_POT_LJ)) k_force_skin<L, CAT_LJ, MIXED, false><<<nb, blk, sh, st>>>(loc, finish, rec);
+    else if (cats == (1 << FMDG_POT_MORSE)) k_force_skin<L, CAT_MORSE, MIXED, false><<<nb, blk, sh, st>>>(loc, finish, rec);
+    else k_force_skin<L, CAT_EAM, MIXED, false><<<nb, blk, sh, st>>>(loc, finish, rec);
 }
 
 template <class L>
-void launch_density_skin(const L &loc, bool mixed, bool hyb, int nb, int blk, cudaStream_t st, bool lean)
+void launch_density_skin(const L &loc, bool mixed, bool hyb, int rec, int nb, int blk, cudaStream_t st, bool lean)
 {
     const size_t sh = stage_bytes(loc, blk, 1);
     if (mixed)
     {
-        if (hyb) k_density_skin<L, true, true, false><<<nb, blk, sh, st>>>(loc);
-        else if (lean) k_density_skin<L, true, false, true><<<nb, blk, sh, st>>>(loc);
-        else k_density_skin<L, true, false, false><<<nb, blk, sh, st>>>(loc);
+        if (hyb) k_density_skin<L, true, true, false><<<nb, blk, sh, st>>>(loc, rec);
+        else if (lean) k_density_skin<L, true, false, true><<<nb, blk, sh, st>>>(loc, rec);
+        else k_density_skin<L, true, false, false><<<nb, blk, sh, st>>>(loc, rec);
     }
     else
     {
-        if (hyb) k_density_skin<L, false, true, false><<<nb, blk, sh, st>>>(loc);
-        else k_density_skin<L, false, false, false><<<nb, blk, sh, st>>>(loc);
+        if (hyb) k_density_skin<L, false, true, false><<<nb, blk, sh, st>>>(loc, rec);
+        else k_density_skin<L, false, false, false><<<nb, blk, sh, st>>>(loc, rec);
     }
 }
 
@@ -1376,8 +1386,8 @@ int fmdg_pack_launch_forces(const fmdg_pack_launch &P, int phases)
     }
     if ((phases & 2) && (P.cats & (1 << FMDG_POT_EAM)))
     {
-        if (P.shares) launch_density_skin(LocPackShares{P.lf}, P.mixed != 0, __builtin_popcount(P.cats) > 1, nfb, P.fblk, st, P.lean != 0);
-        else launch_density_skin(P.lf, P.mixed != 0, __builtin_popcount(P.cats) > 1, nfb, P.fblk, st, P.lean != 0);
+        if (P.shares) launch_density_skin(LocPackShares{P.lf}, P.mixed != 0, __builtin_popcount(P.cats) > 1, REC_FULL, nfb, P.fblk, st, P.lean != 0);
+        else launch_density_skin(P.lf, P.mixed != 0, __builtin_popcount(P.cats) > 1, REC_FULL, nfb, P.fblk, st, P.lean != 0);
         n++;
     }
     if (phases & 4)
@@ -1385,11 +1395,11 @@ int fmdg_pack_launch_forces(const fmdg_pack_launch &P, int phases)
         if (P.shares)
         {
             const LocPackShares L{P.lf};
-            if (P.mixed) launch_force_skin<LocPackShares, true>(L, P.cats, 1, nfb, P.fblk, st, P.lean != 0);
-            else launch_force_skin<LocPackShares, false>(L, P.cats, 1, nfb, P.fblk, st, false);
+            if (P.mixed) launch_force_skin<LocPackShares, true>(L, P.cats, 1, REC_FULL, nfb, P.fblk, st, P.lean != 0);
+            else launch_force_skin<LocPackShares, false>(L, P.cats, 1, REC_FULL, nfb, P.fblk, st, false);
         }
-        else if (P.mixed) launch_force_skin<LocPack, true>(P.lf, P.cats, 1, nfb, P.fblk, st, P.lean != 0);
-        else launch_force_skin<LocPack, false>(P.lf, P.cats, 1, nfb, P.fblk, st, false);
+        else if (P.mixed) launch_force_skin<LocPack, true>(P.lf, P.cats, 1, REC_FULL, nfb, P.fblk, st, P.lean != 0);
+        else launch_force_skin<LocPack, false>(P.lf, P.cats, 1, REC_FULL, nfb, P.fblk, st, false);
         n++;
     }
     cudaError_t e = cudaGetLastError();
@@ -1438,7 +1448,7 @@ static bool lean_system(const fmdg_sys_t *s) { return s->nkinds == 1 && s->g.st.
 int fmdg_skin_launch_density(fmdg_sys_t *s)
 {
     launch_density_skin(LocOne{s->g}, s->g.prec == FMDG_PREC_MIXED, __builtin_popcount(s->cats) > 1,
-                        fmdg_force_blocks(s), s->fblk, s->stream, lean_system(s));
+                        s->rec, fmdg_force_blocks(s), s->fblk, s->stream, lean_system(s));
     s->launches++;
     FMDG_CK(cudaGetLastError());
     return FMDG_OK;
@@ -1449,8 +1459,8 @@ int fmdg_skin_launch_pair_forces(fmdg_sys_t *s, int finish)
     const LocOne L{s->g};
     const int nb = fmdg_force_blocks(s);
     if (s->g.prec == FMDG_PREC_MIXED)
-        launch_force_skin<LocOne, true>(L, s->cats, finish, nb, s->fblk, s->stream, lean_system(s));
-    else launch_force_skin<LocOne, false>(L, s->cats, finish, nb, s->fblk, s->stream, false);
+        launch_force_skin<LocOne, true>(L, s->cats, finish, s->rec, nb, s->fblk, s->stream, lean_system(s));
+    else launch_force_skin<LocOne, false>(L, s->cats, finish, s->rec, nb, s->fblk, s->stream, false);
     s->launches++;
     FMDG_CK(cudaGetLastError());
     return FMDG_OK;
