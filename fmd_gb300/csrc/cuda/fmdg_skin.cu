@@ -87,6 +87,17 @@ __device__ __forceinline__ void load_offsets(const Geo &g, SkinOffT<LO> &so)
 __device__ __forceinline__ float scaled_xs2(const Geo &g) { return (float)(g.xs * g.xs); }
 __device__ __forceinline__ float scaled_index_factor(const Geo &g) { return (float)(g.inv_dr2 * (g.inv_xs * g.inv_xs)); }
 
+__device__ __forceinline__ float norm2(float3 v)
+{
+    return __fmaf_rn(v.z, v.z, __fmaf_rn(v.y, v.y, __fmul_rn(v.x, v.x)));
+}
+
+// spl_der with its roundings spelled out
+__device__ __forceinline__ float spl_der_rn(float4 t, float b, float inv_h)
+{
+    return __fmul_rn(__fmaf_rn(__fmaf_rn(__fmul_rn(3.f, t.w), b, __fmul_rn(2.f, t.z)), b, t.y), inv_h);
+}
+
 // binary32 pair vector x_i - x_j - offset without the offset's remainder
 // (list-radius prefilters)
 __device__ __forceinline__ float3 rv_of(float4 xi, float4 xj, float4 o)
@@ -1019,25 +1030,25 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
                 const float kmax = (float)(nint - 1);
                 const int ee = sp.pairs[0].iloc;
                 const float4 *tpr = g.pkf_pr + (size_t)ee * nint * 2;
-                // LJ / Morse pair: force factor and half energy
+                // LJ / Morse pair: force factor and half energy (explicitly
+                // rounded operations in the forces: the walks with and without
+                // the energy give the same bits)
                 auto pair_lm = [&](float r2, float &fa, float &e) {
                     if (CAT == CAT_LJ)
                     {
                         const float inv_r2 = rcp_approx(r2);
-                        const float s2 = pq.y * inv_r2;
-                        const float s6 = s2 * s2 * s2;
-                        const float s12 = s6 * s6;
-                        fa = lj_c * inv_r2 * (s12 - 0.5f * s6);
-                        e = 0.5f * (pq.x * (s12 - s6));
+                        const float s2 = __fmul_rn(pq.y, inv_r2);
+                        const float s6 = __fmul_rn(__fmul_rn(s2, s2), s2);
+                        fa = __fmul_rn(__fmul_rn(lj_c, inv_r2), __fmul_rn(s6, __fsub_rn(s6, 0.5f)));
+                        e = 0.5f * (pq.x * (s6 * s6 - s6));
                     }
                     else
                     {
                         const float inv_r = rsqrt_approx(r2);
-                        const float r = r2 * inv_r;
-                        const float e1 = ex2_approx((pq.z - r) * m_c1);
-                        const float e2 = e1 * e1;
-                        fa = m_c2 * inv_r * (e2 - e1);
-                        e = 0.5f * (pq.x * (e2 - 2.f * e1));
+                        const float r = __fmul_rn(r2, inv_r);
+                        const float e1 = ex2_approx(__fmul_rn(__fsub_rn(pq.z, r), m_c1));
+                        fa = __fmul_rn(__fmul_rn(m_c2, inv_r), __fmaf_rn(e1, e1, -e1));
+                        e = 0.5f * (pq.x * (e1 * e1 - 2.f * e1));
                     }
                 };
                 // E: the walk sums the energy, W: the pair virial (rv . F =
@@ -1053,7 +1064,7 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
                         const float band = 1e-4f * rc2f;
                         for_each_slot_pair<false>(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
                             const float3 rv = rv_of(xi, xj, o);
-                            const float r2 = rv.x * rv.x + rv.y * rv.y + rv.z * rv.z;
+                            const float r2 = norm2(rv);
                             bool in = r2 < rc2f;
                             if (fabsf(r2 - rc2f) <= band) in = geom64_mi(g, g.xd[t], g.xd[js]).r2 < rc2;
                             if (!in) return;
@@ -1061,15 +1072,15 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
                             const int ir2 = table_index(r2 * inv_hi, kmax, b);
                             float4 tph, trh;
                             ld_row32(tpr + 2 * ir2, tph, trh);
-                            const float phi_d = spl_der(tph, b, inv_h);
-                            const float rho_d = spl_der(trh, b, inv_h);
+                            const float phi_d = spl_der_rn(tph, b, inv_h);
+                            const float rho_d = spl_der_rn(trh, b, inv_h);
                             // F'(rho_j): w of the list position; an overflow
                             // fallback occurrence (code < 0) carries kind bits
                             const float fpj = __float_as_int(o.w) >= 0 ? xj.w : g.fpb[js];
-                            const float fa = -2.f * (fpi * rho_d + fpj * rho_d + phi_d);
-                            ac.part[0] += fa * rv.x;
-                            ac.part[1] += fa * rv.y;
-                            ac.part[2] += fa * rv.z;
+                            const float fa = __fmul_rn(-2.f, __fmaf_rn(__fadd_rn(fpi, fpj), rho_d, phi_d));
+                            ac.part[0] = __fmaf_rn(fa, rv.x, ac.part[0]);
+                            ac.part[1] = __fmaf_rn(fa, rv.y, ac.part[1]);
+                            ac.part[2] = __fmaf_rn(fa, rv.z, ac.part[2]);
                             if constexpr (E) ac.part[3] += 0.5f * spl_val(tph, b);
                             if constexpr (W) ac.part[NA - 1] += fa * r2;
                         }, [&](int k) { ac.entries(k); });
@@ -1089,7 +1100,7 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
                         float3 prv = make_float3(0.f, 0.f, 0.f);
                         for_each_slot_pair<true>(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
                             const float3 rv = rv_of(xi, xj, o);
-                            const float r2 = rv.x * rv.x + rv.y * rv.y + rv.z * rv.z;
+                            const float r2 = norm2(rv);
                             const bool near = fabsf(r2 - rc2f) <= band;
                             const bool in = (r2 < rc2f) && !near;
                             npend += near;
@@ -1099,9 +1110,9 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
                             pair_lm(r2, fa, e);
                             fa = in ? fa : 0.f;
                             e = in ? e : 0.f;
-                            ac.part[0] += fa * rv.x;
-                            ac.part[1] += fa * rv.y;
-                            ac.part[2] += fa * rv.z;
+                            ac.part[0] = __fmaf_rn(fa, rv.x, ac.part[0]);
+                            ac.part[1] = __fmaf_rn(fa, rv.y, ac.part[1]);
+                            ac.part[2] = __fmaf_rn(fa, rv.z, ac.part[2]);
                             if constexpr (E) ac.part[3] += e;
                             if constexpr (W) ac.part[NA - 1] += fa * r2;
                         }, [&](int k) { ac.entries(k); });
@@ -1110,12 +1121,12 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
                         {
                             if (geom64_mi(g, g.xd[t], g.xd[pend]).r2 < rc2)
                             {
-                                const float r2 = prv.x * prv.x + prv.y * prv.y + prv.z * prv.z;
+                                const float r2 = norm2(prv);
                                 float fa, e;
                                 pair_lm(r2, fa, e);
-                                ac.part[0] += fa * prv.x;
-                                ac.part[1] += fa * prv.y;
-                                ac.part[2] += fa * prv.z;
+                                ac.part[0] = __fmaf_rn(fa, prv.x, ac.part[0]);
+                                ac.part[1] = __fmaf_rn(fa, prv.y, ac.part[1]);
+                                ac.part[2] = __fmaf_rn(fa, prv.z, ac.part[2]);
                                 if constexpr (E) ac.part[3] += e;
                                 if constexpr (W) ac.part[NA - 1] += fa * r2;
                                 ac.flush();
@@ -1125,14 +1136,14 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
                         {
                             for_each_slot_pair<false>(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
                                 const float3 rv = rv_of(xi, xj, o);
-                                const float r2 = rv.x * rv.x + rv.y * rv.y + rv.z * rv.z;
+                                const float r2 = norm2(rv);
                                 if (!(fabsf(r2 - rc2f) <= band)) return;
                                 if (!(geom64_mi(g, g.xd[t], g.xd[js]).r2 < rc2)) return;
                                 float fa, e;
                                 pair_lm(r2, fa, e);
-                                ac.part[0] += fa * rv.x;
-                                ac.part[1] += fa * rv.y;
-                                ac.part[2] += fa * rv.z;
+                                ac.part[0] = __fmaf_rn(fa, rv.x, ac.part[0]);
+                                ac.part[1] = __fmaf_rn(fa, rv.y, ac.part[1]);
+                                ac.part[2] = __fmaf_rn(fa, rv.z, ac.part[2]);
                                 if constexpr (E) ac.part[3] += e;
                                 if constexpr (W) ac.part[NA - 1] += fa * r2;
                             }, [&](int k) { ac.entries(k); });
