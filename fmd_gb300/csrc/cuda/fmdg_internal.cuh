@@ -193,6 +193,8 @@ struct fmdg_sys
     DTuri turi[FMDG_MAXT];
     int nturi;
     int ttm_turi;                 // index of the TTM turi or -1
+    cudaStream_t side;            // second branch of a captured TTM step (created with the first turi)
+    cudaEvent_t fork, join;
     int graph_mode;               // 0 velocity Verlet, 1 symplectic Euler
     int fblk;                     // threads per block of the list/density/force kernels
     bool eam_borrowed;            // EAM tables belong to another system
@@ -341,10 +343,10 @@ int fmdg_set_error(const char *msg);
 
 // kernel launch wrappers (defined in their translation units)
 int fmdg_launch_refresh(fmdg_sys_t *s, int mode, double dt, int group, int thermostat);
-int fmdg_launch_turi(fmdg_sys_t *s, int k, double dt);
+int fmdg_launch_turi(fmdg_sys_t *s, int k, double dt, cudaStream_t st);
 // the two halves of fmdg_launch_turi: the field passes, then the TTM solver
-int fmdg_launch_turi_fields(fmdg_sys_t *s, int k, double dt);
-int fmdg_launch_ttm_solve(fmdg_sys_t *s, int k, double dt);
+int fmdg_launch_turi_fields(fmdg_sys_t *s, int k, double dt, cudaStream_t st);
+int fmdg_launch_ttm_solve(fmdg_sys_t *s, int k, double dt, cudaStream_t st);
 int fmdg_launch_forces(fmdg_sys_t *s, int group, int finish, double dt, int thermostat, double tau, double T0,
                        bool prepped);
 int fmdg_launch_density(fmdg_sys_t *s, int group);

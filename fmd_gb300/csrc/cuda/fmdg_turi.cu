@@ -287,12 +287,15 @@ __device__ double spline_adv(const double *xs, const double *ys, const double *d
     return a * ys[klo] + b * ys[khi] + ((a * a * a - a) * dd[klo] + (b * b * b - b) * dd[khi]) * (h * h) / 6.0;
 }
 
-// 1/x to a few ulps for positive x of binary32 range: a binary32 seed
-// refined by two Newton-Raphson steps r <- r + r (1 - x r), each of which
-// squares the relative error (2^-23 -> 2^-46 -> the binary64 rounding)
+// 1/x to a few ulps for positive normal x: the hardware approximation (PTX
+// rcp.approx.ftz.f64, about 2^-20; no conversion to binary32 and back, which
+// would issue at the binary64 rate) refined by two Newton-Raphson steps
+// r <- r + r (1 - x r), each of which squares the relative error (2^-20 ->
+// 2^-40 -> the binary64 rounding)
 __device__ __forceinline__ double recip_newton(double x)
 {
-    double r = (double)__frcp_rn((float)x);
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
     r = fma(r, fma(-x, r, 1.0), r);
     r = fma(r, fma(-x, r, 1.0), r);
     return r;
@@ -382,9 +385,20 @@ __global__ void k_ttm_solve(Geo g, DTuri t, double dt, int staged)
         __syncthreads();
     }
     double *Te = a.Te, *Te2 = a.Te2;
-    // presolve (src/ttm.c:194-231): reads neighbours' Te before this
-    // cell's own update, so it runs in cell order on one thread
-    if (threadIdx.x == 0)
+    // presolve (src/ttm.c:194-231): activation reads neighbours' Te before
+    // this cell's own update, so it runs in cell order on one thread; with
+    // no cell to activate every cell is on its own
+    bool wake = false;
+    for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) wake = wake || (Te[i] < 0.0 && a.num[i] >= p.min_atoms);
+    if (!__syncthreads_or(wake))
+    {
+        for (int i = lo + threadIdx.x; i < hi; i += blockDim.x)
+        {
+            a.xi[i] = 0.0;
+            if (a.num[i] < p.min_atoms) Te[i] = Te2[i] = -1.0;
+        }
+    }
+    else if (threadIdx.x == 0)
     {
         for (int i = lo; i < hi; i++)
         {
@@ -417,7 +431,49 @@ __global__ void k_ttm_solve(Geo g, DTuri t, double dt, int staged)
         a.srcz[i] = calc_source ? exp(p.laser_m_absdepth_inv * (z - p.frontsurf)) : 0.0;
     }
     __syncthreads();
-    for (int j = 0; j < p.ratio; j++)
+    // Type 1 with a thread per cell (every staged grid up to 1024 cells): the
+    // cell's state in registers, the neighbours that take part found once
+    // (activity does not change between substeps; a comparison of binary64
+    // numbers issues at the binary64 rate), one store and one barrier per
+    // substep.  A substep is a chain of dependent binary64 operations; a
+    // launch of 100 substeps on the 50-cell grid 104 -> 62 us.
+    const bool own = staged && p.type == 1 && hi - lo <= (int)blockDim.x;
+    if (own)
+    {
+        const int i = lo + threadIdx.x;
+        const bool mine = i < hi && Te[i] >= 0.0;
+        double te = 0.0, ti = 0.0, xi = 0.0, sz = 0.0;
+        int ilo = 0, ihi = 0;
+        if (mine)
+        {
+            const int im1 = (i == lo) ? 0 : i - 1;
+            te = Te[i];
+            ti = a.Ti[i];
+            sz = a.srcz[i];
+            ilo = (Te[im1] < 0) ? i : im1;
+            ihi = (Te[i + 1] < 0) ? i : i + 1;
+        }
+        for (int j = 0; j < p.ratio; j++)
+        {
+            if (mine)
+            {
+                // dte / (C_gamma te) * (K lap / dz2 - G (te - Ti) + source)
+                // with the constant quotients formed once per launch and one
+                // reciprocal instead of two IEEE divisions
+                const double q = dte_C * recip_newton(te);
+                const double source = calc_source ? a.spc[j] * sz : 0.0;
+                te = te + q * (K_dz2 * (Te[ihi] - 2 * te + Te[ilo]) - p.G * (te - ti) + source);
+                Te2[i] = te;
+                xi += te;
+            }
+            __syncthreads();
+            double *tmp = Te2;
+            Te2 = Te;
+            Te = tmp;
+        }
+        if (mine) a.xi[i] = xi;
+    }
+    for (int j = own ? p.ratio : 0; j < p.ratio; j++)
     {
         double spc = 0.0;
         if (calc_source)
@@ -440,10 +496,6 @@ __global__ void k_ttm_solve(Geo g, DTuri t, double dt, int staged)
             double nv;
             if (p.type == 1)
             {
-                // dte / (C_gamma te) * (K lap / dz2 - G (te - Ti) + source)
-                // with the constant quotients formed once per launch and one
-                // reciprocal: the substeps are a chain of dependent binary64
-                // operations, and an IEEE division is the longest link
                 const double q = dte_C * recip_newton(te);
                 nv = te + q * (K_dz2 * (Te[ihi] - 2 * te + Te[ilo]) - p.G * (te - a.Ti[i]) + source);
             }
@@ -539,10 +591,9 @@ extern "C" int fmdg_check_recip(fmdg_sys_t *s, const double *x, int n, double *o
     return e == cudaSuccess ? FMDG_OK : fmdg_fail("fmdg_check_recip", e);
 }
 
-int fmdg_launch_turi_fields(fmdg_sys_t *s, int k, double dt)
+int fmdg_launch_turi_fields(fmdg_sys_t *s, int k, double dt, cudaStream_t st)
 {
     DTuri &t = s->turi[k];
-    cudaStream_t st = s->stream;
     const int nbc = fmdg_grid(t.ncells, 256);
     // two blocks of 512 per SM, each looping over the atoms
     const int nba = std::max(1, std::min(2 * sm_count(s->device), fmdg_grid(s->g.cap, TURI_THREADS)));
@@ -565,20 +616,22 @@ int fmdg_launch_turi_fields(fmdg_sys_t *s, int k, double dt)
     return FMDG_OK;
 }
 
-int fmdg_launch_ttm_solve(fmdg_sys_t *s, int k, double dt)
+int fmdg_launch_ttm_solve(fmdg_sys_t *s, int k, double dt, cudaStream_t st)
 {
     DTuri &t = s->turi[k];
     if (!t.ttm) return FMDG_OK;
     const size_t bytes = ttm_stage_bytes(t.dims[2], t.p.ratio);
     const int staged = bytes <= 48 * 1024;
-    k_ttm_solve<<<1, 128, staged ? bytes : 0, s->stream>>>(s->g, t, dt, staged);
+    // a thread per cell where a block can (fewer idle warps at its barriers)
+    const int threads = std::min(1024, std::max(64, (t.itc_hi - t.itc_lo + 31) / 32 * 32));
+    k_ttm_solve<<<1, threads, staged ? bytes : 0, st>>>(s->g, t, dt, staged);
     s->launches++;
     FMDG_CK(cudaGetLastError());
     return FMDG_OK;
 }
 
-int fmdg_launch_turi(fmdg_sys_t *s, int k, double dt)
+int fmdg_launch_turi(fmdg_sys_t *s, int k, double dt, cudaStream_t st)
 {
-    int rc = fmdg_launch_turi_fields(s, k, dt);
-    return rc ? rc : fmdg_launch_ttm_solve(s, k, dt);
+    int rc = fmdg_launch_turi_fields(s, k, dt, st);
+    return rc ? rc : fmdg_launch_ttm_solve(s, k, dt, st);
 }
