@@ -151,6 +151,52 @@ __global__ void k_change_group(Geo g, int old_group, int new_group)
     if (old_group < 0 || S.group[i] == old_group) S.group[i] = new_group;
 }
 
+// Binary64 numbers as integers of the same order (comparisons of binary64
+// numbers issue at 1/64 of the integer rate)
+__host__ __device__ inline unsigned long long order_key(unsigned long long b)
+{
+    return (b >> 63) ? ~b : b | (1ull << 63);
+}
+__host__ __device__ inline unsigned long long order_bits(unsigned long long k)
+{
+    return (k >> 63) ? k & ~(1ull << 63) : ~k;
+}
+
+// smallest and largest coordinates of a group's atoms as order keys: out[d],
+// out[3 + d], merged into what is there; NaN is passed over
+__global__ void __launch_bounds__(256) k_limits(Geo g, int group, unsigned long long *out)
+{
+    const Dyn *dyn = g.dyn;
+    const int n = dyn->n;
+    const Side S = g.side[dyn->cur];
+    unsigned long long lo[3] = {~0ull, ~0ull, ~0ull}, hi[3] = {0ull, 0ull, 0ull};
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    {
+        if (group >= 0 && S.group[i] != group) continue;
+        for (int d = 0; d < 3; d++)
+        {
+            const unsigned long long b = (unsigned long long)__double_as_longlong(S.x[(size_t)d * g.cap + i]);
+            if ((b & 0x7fffffffffffffffull) > 0x7ff0000000000000ull) continue;
+            const unsigned long long k = order_key(b);
+            lo[d] = k < lo[d] ? k : lo[d];
+            hi[d] = k > hi[d] ? k : hi[d];
+        }
+    }
+    for (int d = 0; d < 3; d++)
+        for (int o = 16; o > 0; o >>= 1)
+        {
+            const unsigned long long a = __shfl_xor_sync(0xffffffffu, lo[d], o), b = __shfl_xor_sync(0xffffffffu, hi[d], o);
+            lo[d] = a < lo[d] ? a : lo[d];
+            hi[d] = b > hi[d] ? b : hi[d];
+        }
+    if ((threadIdx.x & 31) == 0)
+        for (int d = 0; d < 3; d++)
+        {
+            atomicMin(&out[d], lo[d]);
+            atomicMax(&out[3 + d], hi[d]);
+        }
+}
+
 __global__ void k_flush(unsigned *buf, size_t n)
 {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
@@ -1347,6 +1393,37 @@ extern "C" int fmdg_get_errors(fmdg_sys_t *s, unsigned *bits, int clear)
     {
         unsigned z = 0;
         FMDG_CK(cudaMemcpyAsync((char *)s->g.dyn + offsetof(Dyn, err), &z, sizeof z, cudaMemcpyHostToDevice, s->stream));
+    }
+    return FMDG_OK;
+}
+
+extern "C" int fmdg_find_limits(fmdg_sys_t *s, int group, double lower[3], double upper[3])
+{
+    if (!s->atoms) return FMDG_E_STATE;
+    // keys merged on the device from the caller's values; the reduction
+    // partials of a force evaluation hold nothing between evaluations
+    unsigned long long key[6];
+    for (int d = 0; d < 3; d++)
+    {
+        unsigned long long b;
+        memcpy(&b, &lower[d], 8);
+        key[d] = order_key(b);
+        memcpy(&b, &upper[d], 8);
+        key[3 + d] = order_key(b);
+    }
+    unsigned long long *dev = (unsigned long long *)s->g.partials;
+    FMDG_CK(cudaMemcpyAsync(dev, key, sizeof key, cudaMemcpyHostToDevice, s->stream));
+    const int blocks = fmdg_grid(s->g.cap, 256);
+    k_limits<<<blocks < 1024 ? blocks : 1024, 256, 0, s->stream>>>(s->g, group, dev);
+    s->launches++;
+    FMDG_CK(cudaGetLastError());
+    FMDG_D2H(key, dev, sizeof key);
+    for (int d = 0; d < 3; d++)
+    {
+        unsigned long long b = order_bits(key[d]);
+        memcpy(&lower[d], &b, 8);
+        b = order_bits(key[3 + d]);
+        memcpy(&upper[d], &b, 8);
     }
     return FMDG_OK;
 }

@@ -442,6 +442,11 @@ void fmd_matt_findLimits(fmd_t *md, int GroupID, fmd_rtriple_t LowerLimit, fmd_r
         LowerLimit[d] = 1.7976931348623157e308;
         UpperLimit[d] = 2.2250738585072014e-308;   /* DBL_MIN, as src/matter.c:215-218 */
     }
+    if (md->ParticlesDistributed)
+    {
+        fmdg_find_limits(md->dev, GroupID == FMD_GROUP_ALL ? -1 : GroupID, LowerLimit, UpperLimit);
+        return;
+    }
     if (_fmdh_current_atoms(md, &n, &x, &v, &kind, &group, &id) == 0)
         for (int i = 0; i < n; i++)
             if (GroupID == FMD_GROUP_ALL || GroupID == group[i])
