@@ -44,9 +44,8 @@ namespace cg = cooperative_groups;
 
 namespace {
 
-// Measured on one GB300, us per step of the whole refresh: 256 atoms 21 (eight
-// launches) -> 11 (one cluster kernel), 4000 atoms 24 -> 14, but 32 000 atoms
-// 26 (five grid kernels) against 61.
+// largest system of the cluster kernel: 4000 atoms refresh in 14 us against
+// 24 for the separate kernels, 32 000 atoms in 61 against 26
 constexpr int CLUSTER_ATOMS = 1 << 13;
 
 __device__ __forceinline__ int cell_flat(const Geo &g, int x, int y, int z)
@@ -416,6 +415,7 @@ __device__ __forceinline__ void load_half_kicks(const Geo &g, double *hk)
 
 __global__ void __launch_bounds__(256) k_bin_classify(__grid_constant__ const LocOne loc, int mode)
 {
+    step_wait();
     const Geo &g = loc.g;
     __shared__ double hk[FMDG_MAXK];
     load_half_kicks(g, hk);
@@ -427,6 +427,7 @@ __global__ void __launch_bounds__(256) k_bin_classify(__grid_constant__ const Lo
 // (one cluster)
 __global__ void __launch_bounds__(1024) k_bin_scan(__grid_constant__ const LocOne loc)
 {
+    step_wait();
     const Geo &g = loc.g;
     Dyn *dyn = g.dyn;
     if (!dyn->any_move) return;
@@ -437,6 +438,7 @@ __global__ void __launch_bounds__(1024) k_bin_scan(__grid_constant__ const LocOn
 
 __global__ void __launch_bounds__(128) k_bin_cells(__grid_constant__ const LocOne loc)
 {
+    step_wait();
     const Geo &g = loc.g;
     const Dyn *dyn = g.dyn;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -445,6 +447,7 @@ __global__ void __launch_bounds__(128) k_bin_cells(__grid_constant__ const LocOn
 
 __global__ void __launch_bounds__(128) k_bin_arrivals(__grid_constant__ const LocOne loc)
 {
+    step_wait();
     const Geo &g = loc.g;
     const Dyn *dyn = g.dyn;
     const int D = blockIdx.x * blockDim.x + threadIdx.x;
@@ -454,6 +457,7 @@ __global__ void __launch_bounds__(128) k_bin_arrivals(__grid_constant__ const Lo
 // the last block to finish swaps the sides
 __global__ void __launch_bounds__(256) k_bin_place(__grid_constant__ const LocOne loc, int mode)
 {
+    step_wait();
     const Geo &g = loc.g;
     Dyn *dyn = g.dyn;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -486,6 +490,7 @@ __device__ __forceinline__ const Geo &cluster_geo(const LocPack &L, int s) { ret
 template <class L>
 __global__ void __launch_bounds__(512) k_refresh_cluster(__grid_constant__ const L loc, int mode)
 {
+    step_wait();
     constexpr bool PACK = L::renumbered;
     cg::cluster_group cl = cg::this_cluster();
     const int nblk = cl.num_blocks(), rank = cl.block_rank();
@@ -499,9 +504,7 @@ __global__ void __launch_bounds__(512) k_refresh_cluster(__grid_constant__ const
     const int n = dyn->n, cur = dyn->cur, ncell = g.ncell;
     const Side S = g.side[cur], T = g.side[cur ^ 1];
     const int tid = rank * blockDim.x + threadIdx.x, nt = nblk * blockDim.x;
-    // (dep_count, arr_lower, arr_total, bucket_fill are contiguous)
-    for (int c = tid; c < 4 * ncell; c += nt) g.dep_count[c] = 0;
-    cl.sync();
+    // (the cells' counters are zero between refreshes: cleared below)
     for (int i = tid; i < n; i += nt) classify_atom(g, dyn, S, i, mode, hk);
     cl.sync();
     const bool moved = *(volatile int *)&dyn->any_move != 0;
@@ -519,33 +522,20 @@ __global__ void __launch_bounds__(512) k_refresh_cluster(__grid_constant__ const
     if (PACK)
         for (int i = n_next + tid; i < g.cap; i += nt) g.pos[i] = -1;
     cl.sync();
+    // (dep_count, arr_lower, arr_total, bucket_fill are contiguous)
+    if (moved)
+        for (int c = tid; c < 4 * ncell; c += nt) g.dep_count[c] = 0;
     if (tid == 0) flip_sides(g, dyn, mode);
 }
 
-// grid: blocks of `threads` in clusters of `cluster`
-template <class L>
-cudaError_t launch_cluster(void (*kernel)(L, int), const L &loc, int mode, int blocks, int threads, int cluster, cudaStream_t st)
+// Eight blocks (the portable cluster size) refresh a system of n atoms, of
+// as few threads as give every atom one: the phases are binary64 work, which
+// an SM issues for one warp at a time, so few warps on many SMs.
+constexpr int REFRESH_BLOCKS = 8;
+int refresh_threads(int n)
 {
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = cluster;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(threads);
-    cfg.stream = st;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, loc, mode);
-}
-
-// blocks of 512 in the cluster that refreshes a system of n atoms: one
-// thread per atom up to the portable cluster size
-int refresh_blocks(int n)
-{
-    int b = 1;
-    while (b < 8 && b * 512 < n) b <<= 1;
-    return b;
+    const int t = (fmdg_grid(n, REFRESH_BLOCKS) + 31) & ~31;
+    return t < 64 ? 64 : (t > 512 ? 512 : t);
 }
 
 } // namespace
@@ -563,32 +553,20 @@ int fmdg_launch_refresh(fmdg_sys_t *s, int mode, double dt, int group, int therm
     const LocOne L{g};
     if (g.cap <= CLUSTER_ATOMS)
     {
-        const int b = refresh_blocks(g.cap);
-        FMDG_CK(launch_cluster(k_refresh_cluster<LocOne>, L, mode, b, 512, b, st));
+        FMDG_CK(fmdg_launch(k_refresh_cluster<LocOne>, REFRESH_BLOCKS, refresh_threads(g.cap), 0, st, s->overlap,
+                            REFRESH_BLOCKS, L, mode));
         s->launches++;
         return FMDG_OK;
     }
     // dep_count, arr_lower, arr_total, bucket_fill are contiguous
     FMDG_CK(cudaMemsetAsync(g.dep_count, 0, sizeof(int) * 4 * (size_t)g.ncell, st));
-    k_bin_classify<<<fmdg_grid(g.cap, 256), 256, 0, st>>>(L, mode);
-    {
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = 8;
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(8);
-        cfg.blockDim = dim3(1024);
-        cfg.stream = st;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        FMDG_CK(cudaLaunchKernelEx(&cfg, k_bin_scan, L));
-    }
-    k_bin_cells<<<fmdg_grid(g.ncell, 128), 128, 0, st>>>(L);
-    k_bin_arrivals<<<fmdg_grid(g.ncell, 128), 128, 0, st>>>(L);
-    k_bin_place<<<fmdg_grid(g.cap, 256), 256, 0, st>>>(L, mode);
+    const bool ov = s->overlap;
+    FMDG_CK(fmdg_launch(k_bin_classify, fmdg_grid(g.cap, 256), 256, 0, st, false, 1, L, mode));
+    FMDG_CK(fmdg_launch(k_bin_scan, 8, 1024, 0, st, ov, 8, L));
+    FMDG_CK(fmdg_launch(k_bin_cells, fmdg_grid(g.ncell, 128), 128, 0, st, ov, 1, L));
+    FMDG_CK(fmdg_launch(k_bin_arrivals, fmdg_grid(g.ncell, 128), 128, 0, st, ov, 1, L));
+    FMDG_CK(fmdg_launch(k_bin_place, fmdg_grid(g.cap, 256), 256, 0, st, ov, 1, L, mode));
     s->launches += 5;
-    FMDG_CK(cudaGetLastError());
     return FMDG_OK;
 }
 
@@ -603,8 +581,8 @@ int fmdg_pack_launch_refresh(const fmdg_pack_launch &P)
     if (n < 0) return n;
     int most = 1;
     for (int k = 0; k < P.nsys; k++) most = P.la.geos[k].cap > most ? P.la.geos[k].cap : most;
-    const int b = refresh_blocks(most);
-    const cudaError_t e = launch_cluster(k_refresh_cluster<LocPack>, P.la, FMDG_REFRESH_ONLY, b * P.nsys, 512, b, st);
+    const cudaError_t e = fmdg_launch(k_refresh_cluster<LocPack>, REFRESH_BLOCKS * P.nsys, refresh_threads(most), 0, st,
+                                      P.overlap, REFRESH_BLOCKS, P.la, FMDG_REFRESH_ONLY);
     if (e != cudaSuccess) return -fmdg_fail("pack refresh", e);
     return n + 1;
 }

@@ -117,7 +117,7 @@ struct Carver
 void drop_eam(fmdg_sys_t *s)
 {
     Geo &g = s->g;
-    g.pk_rho = g.pk_phi = g.pk_F = nullptr;
+    g.pk_F = nullptr;
     g.pkf_rho = g.pkf_phi = g.pkf_F = g.pkf_pr = nullptr;
     g.pkd_rho = g.pkd_phi = nullptr;
     s->eam_borrowed = false;
@@ -334,7 +334,7 @@ extern "C" void fmdg_destroy(fmdg_sys_t *s)
     if (s->eam_borrowed) drop_eam(s);
     dfree(s, (void *)s->g.pairs); dfree(s, (void *)s->g.mass); dfree(s, (void *)s->g.eam_elem);
     dfree(s, (void *)s->g.pairf); dfree(s, (void *)s->g.paird);
-    dfree(s, (void *)s->g.pk_rho); dfree(s, (void *)s->g.pk_phi); dfree(s, (void *)s->g.pk_F);
+    dfree(s, (void *)s->g.pk_F);
     dfree(s, (void *)s->g.pkf_rho); dfree(s, (void *)s->g.pkf_phi); dfree(s, (void *)s->g.pkf_F);
     dfree(s, (void *)s->g.pkf_pr); dfree(s, (void *)s->g.pkd_rho); dfree(s, (void *)s->g.pkd_phi);
     for (int k = 0; k < s->nturi; k++)
@@ -372,6 +372,8 @@ extern "C" int fmdg_set_box(fmdg_sys_t *s, const double l[3], const int pbc[3], 
         s->g.inv_cellh[d] = 1.0 / cellh[d];
         s->g.l_f[d] = (float)l[d];
         s->g.inv_cellh_f[d] = (float)s->g.inv_cellh[d];
+        s->g.cellh_f[d] = (float)cellh[d];
+        s->g.cellh_lo[d] = (float)(cellh[d] - (double)s->g.cellh_f[d]);
     }
     const long long ncell = (long long)nc[0] * nc[1] * nc[2];
     if (ncell > (1 << 24)) return fmdg_set_error("fmdg_set_box: more than 2^24 cells");
@@ -454,7 +456,14 @@ int fmdg_skin_scale(fmdg_sys_t *s)
     const double xs = (g.prec == FMDG_PREC_MIXED) ? (double)(float)g.cellh[0] / g.cellh[0] : 1.0;
     g.xs = xs;
     g.inv_xs = 1.0 / xs;
-    for (int d = 0; d < 3; d++) g.cellh_s[d] = (float)(g.cellh[d] * xs);
+    for (int d = 0; d < 3; d++)
+    {
+        g.cellh_s[d] = (float)(g.cellh[d] * xs);
+        g.cellh_slo[d] = (float)(g.cellh[d] * xs - (double)g.cellh_s[d]);
+    }
+    g.xs2_f = (float)(xs * xs);
+    g.inv_hi_f = (float)(g.inv_dr2 * (g.inv_xs * g.inv_xs));
+    g.inv_h_df = df_split(g.inv_dr2);
     if (s->rsk > 0.0)
     {
         g.rskin2 = (float)(s->rsk * xs * s->rsk * xs);
@@ -510,7 +519,7 @@ extern "C" int fmdg_set_eam(fmdg_sys_t *s, int nelem, int Nrho, double drho, int
     // algebraically the reference's a/b form (a = 1-b).  Computed in binary64;
     // the binary32 copy keeps k1 (the per-interval increment) to full relative
     // precision, which the two-sample difference y_k+1 - y_k would not.
-    dfree(s, (void *)g.pk_rho); dfree(s, (void *)g.pk_phi); dfree(s, (void *)g.pk_F);
+    dfree(s, (void *)g.pk_F);
     dfree(s, (void *)g.pkf_rho); dfree(s, (void *)g.pkf_phi); dfree(s, (void *)g.pkf_F);
     dfree(s, (void *)g.pkf_pr); dfree(s, (void *)g.pkd_rho); dfree(s, (void *)g.pkd_phi);
     auto pack = [&](const double *y, const double *ydd, double h, int npts, int nfun, const double4_32a **d64,
@@ -535,8 +544,12 @@ extern "C" int fmdg_set_eam(fmdg_sys_t *s, int nelem, int Nrho, double drho, int
                 }
             }
         int rc2;
-        if ((rc2 = dalloc(s, (double4_32a **)d64, h64.size())) || (rc2 = dalloc(s, (float4 **)d32, h32.size()))) return rc2;
-        FMDG_CK(cudaMemcpyAsync((void *)*d64, h64.data(), h64.size() * sizeof(double4_32a), cudaMemcpyHostToDevice, s->stream));
+        if (d64)
+        {
+            if ((rc2 = dalloc(s, (double4_32a **)d64, h64.size()))) return rc2;
+            FMDG_CK(cudaMemcpyAsync((void *)*d64, h64.data(), h64.size() * sizeof(double4_32a), cudaMemcpyHostToDevice, s->stream));
+        }
+        if ((rc2 = dalloc(s, (float4 **)d32, h32.size()))) return rc2;
         FMDG_CK(cudaMemcpyAsync((void *)*d32, h32.data(), h32.size() * sizeof(float4), cudaMemcpyHostToDevice, s->stream));
         if (ddf)
         {
@@ -545,8 +558,8 @@ extern "C" int fmdg_set_eam(fmdg_sys_t *s, int nelem, int Nrho, double drho, int
         }
         return FMDG_OK;
     };
-    if ((rc = pack(rho, rhoDD, dr2, Nr2, nelem, &g.pk_rho, &g.pkf_rho, &g.pkd_rho))) return rc;
-    if ((rc = pack(phi, phiDD, dr2, Nr2, nelem * nelem, &g.pk_phi, &g.pkf_phi, &g.pkd_phi))) return rc;
+    if ((rc = pack(rho, rhoDD, dr2, Nr2, nelem, nullptr, &g.pkf_rho, &g.pkd_rho))) return rc;
+    if ((rc = pack(phi, phiDD, dr2, Nr2, nelem * nelem, nullptr, &g.pkf_phi, &g.pkd_phi))) return rc;
     if ((rc = pack(F, F_DD, drho, Nrho, nelem, &g.pk_F, &g.pkf_F, nullptr))) return rc;
     {
         // the one-element pair rows side by side for the lean force kernels
@@ -655,7 +668,10 @@ int fmdg_share_log(const fmdg_sys_t *s, int n)
     int target = s->g.prec == FMDG_PREC_FP64 ? 400000 : 1 << 16;
     if (s->served) target = s->g.prec == FMDG_PREC_FP64 ? 1 << 14 : 1 << 13;
     int l = 0;
-    while (l < 4 && ((long long)n << (l + 1)) <= target) l++;
+    // (32 shares: argon 256 atoms 32.6 -> 30.9 us, EAM 2048 50 -> 46.6, but
+    // argon 4000 36.0 -> 38.6)
+    const int most = (!s->served && n <= 2048) ? 5 : 4;
+    while (l < most && ((long long)n << (l + 1)) <= target) l++;
     return l;
 }
 
@@ -690,17 +706,17 @@ extern "C" int fmdg_set_skin(fmdg_sys_t *s, double skin)
 // the owner must outlive every borrower.
 extern "C" int fmdg_share_eam(fmdg_sys_t *s, const fmdg_sys_t *owner)
 {
-    if (!owner || !owner->g.pk_rho) return fmdg_set_error("fmdg_share_eam: the owner has no EAM tables");
+    if (!owner || !owner->g.pk_F) return fmdg_set_error("fmdg_share_eam: the owner has no EAM tables");
     if (owner->device != s->device) return fmdg_set_error("fmdg_share_eam: different devices");
     Geo &g = s->g;
     if (!s->eam_borrowed)
     {
-        dfree(s, (void *)g.pk_rho); dfree(s, (void *)g.pk_phi); dfree(s, (void *)g.pk_F);
+        dfree(s, (void *)g.pk_F);
         dfree(s, (void *)g.pkf_rho); dfree(s, (void *)g.pkf_phi); dfree(s, (void *)g.pkf_F);
         dfree(s, (void *)g.pkf_pr); dfree(s, (void *)g.pkd_rho); dfree(s, (void *)g.pkd_phi);
     }
     const Geo &o = owner->g;
-    g.pk_rho = o.pk_rho; g.pk_phi = o.pk_phi; g.pk_F = o.pk_F;
+    g.pk_F = o.pk_F;
     g.pkf_rho = o.pkf_rho; g.pkf_phi = o.pkf_phi; g.pkf_F = o.pkf_F; g.pkf_pr = o.pkf_pr;
     g.pkd_rho = o.pkd_rho; g.pkd_phi = o.pkd_phi;
     g.nelem = o.nelem; g.Nrho = o.Nrho; g.Nr2 = o.Nr2; g.drho = o.drho; g.dr2 = o.dr2;
@@ -756,10 +772,6 @@ extern "C" int fmdg_upload(fmdg_sys_t *s, int n, const int *cell_count, const do
     }
     const double rlist = sqrt(rc2max) + 1e-2;
     g.rlist2 = (float)(rlist * rlist);
-    for (int d3 = 0; d3 < 3; d3++)
-    {
-        g.cellh_f[d3] = (float)g.cellh[d3];
-    }
     // a skin list needs the list radius below half of every periodic box
     // length (one image inside it) and within two cells; otherwise the
     // exact stencil list is rebuilt every step.  The default skin shrinks to
@@ -878,6 +890,7 @@ extern "C" int fmdg_upload(fmdg_sys_t *s, int n, const int *cell_count, const do
     FMDG_CK(cudaMemcpyAsync((void *)g.corig, corig.data(), (size_t)ncell * sizeof(double4_32a),
                             cudaMemcpyHostToDevice, st));
     FMDG_CK(cudaMemsetAsync(g.F, 0, 3 * (size_t)cap * 8, st));
+    FMDG_CK(cudaMemsetAsync(g.dep_count, 0, 4 * (size_t)ncell * sizeof(int), st));     // zero between refreshes
     FMDG_CK(cudaMemsetAsync(g.vaream, 0, (size_t)cap * 8, st));
     const double keep_time = d.time, keep_dt = d.dt;
     memset(&d, 0, sizeof d);
@@ -1034,7 +1047,9 @@ static int replay_steps(fmdg_sys_t *s, int nsteps, int between, F &&launches)
             FMDG_CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
             const long long before = s->launches;
             s->rec = form ? REC_FULL : between;
+            s->overlap = s->nturi == 0;     // (a branched step is launched plainly)
             const int rc = launches();
+            s->overlap = false;
             s->rec = REC_FULL;
             const cudaError_t e = cudaStreamEndCapture(s->stream, &graph);
             s->graph_kernels[form] = (int)(s->launches - before);

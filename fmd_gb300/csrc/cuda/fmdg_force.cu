@@ -146,6 +146,7 @@ __device__ __forceinline__ bool within_cut_df(const Geo &g, const Side &S, int i
 template <class L>
 __global__ void k_prep_local(__grid_constant__ const L loc)
 {
+    step_wait();
     int bx, nb;
     const Geo &g = loc_geo(loc, bx, nb);
     if (loc_idle(loc, g)) return;
@@ -161,6 +162,7 @@ __global__ void k_prep_local(__grid_constant__ const L loc)
 template <class L>
 __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_nlist(__grid_constant__ const L loc)
 {
+    step_wait();
     int bx, nb;
     const Geo &g = loc_geo(loc, bx, nb);
     if (loc_idle(loc, g)) return;
@@ -224,10 +226,11 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density(__gri
 {
     int bx, nb;
     const Geo &g = loc_geo(loc, bx, nb);
-    if (loc_idle(loc, g)) return;
     const int group = g.st.group;
     __shared__ SmemPotT<!MIXED> sp;
-    load_pot(g, sp);
+    load_pot<true>(g, sp, g.pairf);
+    step_wait();
+    if (loc_idle(loc, g)) return;
     Dyn *dyn = g.dyn;
     const int n = dyn->n;
     const Side S = g.side[dyn->cur];
@@ -249,7 +252,7 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density(__gri
                 // double-float pair arithmetic (fmdg_df.cuh)
                 float4 ih, il;
                 ld_row32(g.xdf + 2 * (size_t)i, ih, il);
-                const dfl inv_h = df_of(df_split(g.inv_dr2));
+                const dfl inv_h = df_of(g.inv_h_df);
                 const float kmax = (float)(nint - 1);
                 dfl acc_rho = {0.f, 0.f};
                 for_each_pair(g, S, i, ci, [&](int j, int code) {
@@ -268,7 +271,7 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density(__gri
             else
             {
                 const float4 xi = g.xf4[i];
-                const float inv_h = (float)g.inv_dr2;
+                const float inv_h = g.inv_h_df.x;
                 const float kmax = (float)(nint - 1);
                 Acc32<1> ac;
                 for_each_pair(g, S, i, ci, [&](int j, int code) {
@@ -341,11 +344,12 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_force(__grid_
 {
     int bx, nb;
     const Geo &g = loc_geo(loc, bx, nb);
-    if (loc_idle(loc, g)) return;
     const int group = g.st.group;
     const double dt = g.st.dt;
     __shared__ SmemPotT<!MIXED> sp;
-    load_pot(g, sp);
+    load_pot<true>(g, sp, g.pairf);
+    step_wait();
+    if (loc_idle(loc, g)) return;
     Dyn *dyn = g.dyn;
     const int n = dyn->n;
     const Side S = g.side[dyn->cur];
@@ -374,7 +378,7 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_force(__grid_
                 float4 ih, il;
                 ld_row32(g.xdf + 2 * (size_t)i, ih, il);
                 const dfl fpi = (CAT == CAT_EAM || CAT == CAT_HYBRID) ? df_of(g.fpdf[i]) : dfl{0.f, 0.f};
-                const dfl inv_h = df_of(df_split(g.inv_dr2));
+                const dfl inv_h = df_of(g.inv_h_df);
                 const float kmax = (float)(nint - 1);
                 dfl fs[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}}, pes = {0.f, 0.f}, virs = {0.f, 0.f};
                 for_each_pair(g, S, i, ci, [&](int j, int code) {
@@ -402,7 +406,7 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_force(__grid_
             {
                 const float4 xi = g.xf4[i];
                 const float fpi = (CAT == CAT_EAM || CAT == CAT_HYBRID) ? g.fpf[i] : 0.f;
-                const float inv_h = (float)g.inv_dr2;
+                const float inv_h = g.inv_h_df.x;
                 const float kmax = (float)(nint - 1);
                 Acc32<5> ac;
                 for_each_pair(g, S, i, ci, [&](int j, int code) {
@@ -577,35 +581,35 @@ int fmdg_force_blocks(const fmdg_sys_t *s)
 namespace {
 
 template <class L>
-void launch_nlist_t(const L &loc, int n_prep, int prep_threads, int nb, int blk, cudaStream_t st)
+void launch_nlist_t(const L &loc, int n_prep, int prep_threads, int nb, int blk, cudaStream_t st, bool overlap)
 {
     if (n_prep > 0) k_prep_local<<<n_prep, prep_threads, 0, st>>>(loc);
-    k_nlist<<<nb, blk, 0, st>>>(loc);
+    fmdg_launch(k_nlist<L>, nb, blk, 0, st, overlap && n_prep == 0, 1, loc);
 }
 
 template <class L>
-void launch_density_t(const L &loc, bool mixed, bool hyb, int rec, int nb, int blk, cudaStream_t st)
+void launch_density_t(const L &loc, bool mixed, bool hyb, int rec, int nb, int blk, cudaStream_t st, bool overlap)
 {
     if (mixed)
     {
-        if (hyb) k_density<L, true, true><<<nb, blk, 0, st>>>(loc, rec);
-        else k_density<L, true, false><<<nb, blk, 0, st>>>(loc, rec);
+        if (hyb) fmdg_launch(k_density<L, true, true>, nb, blk, 0, st, overlap, 1, loc, rec);
+        else fmdg_launch(k_density<L, true, false>, nb, blk, 0, st, overlap, 1, loc, rec);
     }
     else
     {
-        if (hyb) k_density<L, false, true><<<nb, blk, 0, st>>>(loc, rec);
-        else k_density<L, false, false><<<nb, blk, 0, st>>>(loc, rec);
+        if (hyb) fmdg_launch(k_density<L, false, true>, nb, blk, 0, st, overlap, 1, loc, rec);
+        else fmdg_launch(k_density<L, false, false>, nb, blk, 0, st, overlap, 1, loc, rec);
     }
 }
 
 template <class L, bool MIXED>
-void launch_force_t(const L &loc, int cats, int finish, int rec, int nb, int blk, cudaStream_t st)
+void launch_force_t(const L &loc, int cats, int finish, int rec, int nb, int blk, cudaStream_t st, bool overlap)
 {
     const int ncat = __builtin_popcount(cats);
-    if (ncat > 1) k_force<L, CAT_HYBRID, MIXED><<<nb, blk, 0, st>>>(loc, finish, rec);
-    else if (cats == (1 << FMDG_POT_LJ)) k_force<L, CAT_LJ, MIXED><<<nb, blk, 0, st>>>(loc, finish, rec);
-    else if (cats == (1 << FMDG_POT_MORSE)) k_force<L, CAT_MORSE, MIXED><<<nb, blk, 0, st>>>(loc, finish, rec);
-    else k_force<L, CAT_EAM, MIXED><<<nb, blk, 0, st>>>(loc, finish, rec);
+    if (ncat > 1) fmdg_launch(k_force<L, CAT_HYBRID, MIXED>, nb, blk, 0, st, overlap, 1, loc, finish, rec);
+    else if (cats == (1 << FMDG_POT_LJ)) fmdg_launch(k_force<L, CAT_LJ, MIXED>, nb, blk, 0, st, overlap, 1, loc, finish, rec);
+    else if (cats == (1 << FMDG_POT_MORSE)) fmdg_launch(k_force<L, CAT_MORSE, MIXED>, nb, blk, 0, st, overlap, 1, loc, finish, rec);
+    else fmdg_launch(k_force<L, CAT_EAM, MIXED>, nb, blk, 0, st, overlap, 1, loc, finish, rec);
 }
 
 } // namespace
@@ -614,7 +618,7 @@ void launch_force_t(const L &loc, int cats, int finish, int rec, int nb, int blk
 int fmdg_launch_nlist(fmdg_sys_t *s, bool prepped)
 {
     if (s->g.skin_on) return fmdg_skin_launch_nlist(s, prepped);
-    launch_nlist_t(LocOne{s->g}, prepped ? 0 : fmdg_grid(s->g.cap, 256), 256, fmdg_force_blocks(s), s->fblk, s->stream);
+    launch_nlist_t(LocOne{s->g}, prepped ? 0 : fmdg_grid(s->g.cap, 256), 256, fmdg_force_blocks(s), s->fblk, s->stream, s->overlap);
     s->launches += prepped ? 1 : 2;
     FMDG_CK(cudaGetLastError());
     return FMDG_OK;
@@ -627,7 +631,7 @@ int fmdg_launch_density(fmdg_sys_t *s, int group)
     s->g.st.group = group;
     if (s->g.skin_on) return fmdg_skin_launch_density(s);
     launch_density_t(LocOne{s->g}, s->g.prec == FMDG_PREC_MIXED, __builtin_popcount(s->cats) > 1,
-                     s->rec, fmdg_force_blocks(s), s->fblk, s->stream);
+                     s->rec, fmdg_force_blocks(s), s->fblk, s->stream, s->overlap);
     s->launches++;
     FMDG_CK(cudaGetLastError());
     return FMDG_OK;
@@ -646,8 +650,8 @@ int fmdg_launch_pair_forces(fmdg_sys_t *s, int group, int finish, double dt, int
     if (s->g.skin_on) return fmdg_skin_launch_pair_forces(s, finish);
     const LocOne L{s->g};
     const int nb = fmdg_force_blocks(s);
-    if (s->g.prec == FMDG_PREC_MIXED) launch_force_t<LocOne, true>(L, s->cats, finish, s->rec, nb, s->fblk, s->stream);
-    else launch_force_t<LocOne, false>(L, s->cats, finish, s->rec, nb, s->fblk, s->stream);
+    if (s->g.prec == FMDG_PREC_MIXED) launch_force_t<LocOne, true>(L, s->cats, finish, s->rec, nb, s->fblk, s->stream, s->overlap);
+    else launch_force_t<LocOne, false>(L, s->cats, finish, s->rec, nb, s->fblk, s->stream, s->overlap);
     s->launches++;
     FMDG_CK(cudaGetLastError());
     return FMDG_OK;

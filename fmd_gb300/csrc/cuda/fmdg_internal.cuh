@@ -79,9 +79,9 @@ struct Geo   // passed by value to kernels
     int maxnb;
     unsigned char share_log, lane_log;   // skin lists: log2 of the shares of a slot's walk and of its lanes (fmdg_skin.cu)
     float rlist2;      // binary32 prefilter radius^2 (largest cutoff + margin)
-    float cellh_f[3];  // binary32 cell widths (remainders cellh - cellh_f formed per block)
+    float cellh_f[3], cellh_lo[3];   // binary32 cell widths and the remainders
     // packed spline tables: per interval k {y_k, y_k+1, y''_k, y''_k+1}
-    const double4_32a *pk_rho, *pk_phi, *pk_F;     // binary64
+    const double4_32a *pk_F;                       // binary64 (embedding)
     const float4 *pkf_rho, *pkf_phi, *pkf_F;   // binary32 copies (mixed mode)
     const float4 *pkf_pr;       // per element e and interval k: {phi_ee, rho_e} side by side (one 32 B row)
     // binary64 mode, EAM: double-float forms (fmdg_df.cuh) of the tables
@@ -154,10 +154,14 @@ struct Geo   // passed by value to kernels
     // work in scaled units with parameters scaled on the host
     // (skin_params), form the real force factor, and scale each atom's
     // force by 1/xs and its virial by 1/xs^2 in binary64; energies need no
-    // scaling.  (Binary32 xs^2 and the EAM index factor inv_dr2 / xs^2 of a
-    // scaled r^2 are formed per thread from xs.)
+    // scaling.
     double xs, inv_xs;
-    float cellh_s[3];      // scaled cell widths, binary32 (remainders cellh xs - cellh_s formed per block)
+    float cellh_s[3], cellh_slo[3];   // scaled cell widths, binary32, and the remainders cellh xs - cellh_s
+    // binary32 constants of the pair kernels, formed on the host (binary64
+    // work in a kernel's prologue issues once per warp at 1/64 of the rate)
+    float xs2_f;           // xs^2
+    float inv_hi_f;        // EAM table index factor of a scaled r^2: inv_dr2 / xs^2
+    float2 inv_h_df;       // inv_dr2 as double-float
 };
 
 struct fmdg_sys
@@ -180,6 +184,7 @@ struct fmdg_sys
     int prof_n[6];
     long long launches;
     int rec;                      // REC_* of the next launches
+    bool overlap;                 // the next launches are a captured step's (fmdg_launch)
     // captured step graphs: [0] a step whose record nobody reads, [1] one
     // with the thermo record (the last of a batch)
     cudaGraphExec_t graph[2];
@@ -250,6 +255,7 @@ struct LocOne
     static constexpr bool one_system = true;
     static constexpr int max_threads = 128;
     static constexpr int min_blocks = 0;      // 0: register count left to the compiler
+    static constexpr int df_min_blocks = 7;   // double-float kernels: 72 registers (EAM 256 000 26.5 ms a pass at 96-120, 25.1 at 72)
     static constexpr int lean_min_blocks = 7; // lean force kernels: 7 blocks of 128 (72 registers), measured best
     static constexpr bool one_lane = false;     // lanes by Geo::lane_log
     static constexpr bool split_shares = false; // every share has its lane
@@ -262,6 +268,7 @@ struct LocPack
     static constexpr bool one_system = false;
     static constexpr int max_threads = 256;
     static constexpr int min_blocks = 0;
+    static constexpr int df_min_blocks = 4;   // 64 registers: 60 binary64 jobs of up to 100 000 atoms 5.0e8 -> 5.45e8 atom-steps/s
     static constexpr int lean_min_blocks = 0; // packed lean force kernels: compiler's choice, measured best
     static constexpr bool one_lane = true;      // one share, one lane per slot
     static constexpr bool split_shares = false;
@@ -274,6 +281,7 @@ struct LocPack
 // (fmdg_skin.cu): the kernels of the others keep their code free of it
 struct LocPackShares : LocPack
 {
+    static constexpr int df_min_blocks = 0;     // (bounded: 300 small binary64 jobs 3.4e8 -> 3.0e8)
     static constexpr bool one_lane = false;
     static constexpr bool split_shares = true;  // a lane may walk several shares
 };
@@ -323,6 +331,7 @@ struct fmdg_pack_launch
     int lean;                   // every member has one kind (lean binary32 kernels)
     int shares;                 // the members' list walks are split into shares (small systems)
     int fblk;                   // threads per block of the list/density/force kernels
+    bool overlap;               // the launches are a captured step's (fmdg_launch)
     LocPack la;                 // 128-thread atom blocks
     LocPack lf;                 // force blocks of fblk threads
 };
@@ -365,6 +374,51 @@ int fmdg_skin_launch_nlist(fmdg_sys_t *s, bool prepped);
 int fmdg_skin_launch_density(fmdg_sys_t *s);
 int fmdg_skin_launch_pair_forces(fmdg_sys_t *s, int finish);
 
+// Launch of a step kernel.  overlap: the kernel may be set up while the one
+// before it in the stream finishes (programmatic dependent launch): it waits
+// in step_wait() before it touches anything the kernels before it wrote, so
+// only launch latency and the block prologues overlap.  Used inside captured
+// steps, where a kernel follows a kernel.  Kernels release the next one at
+// their end, or where only their short epilogue is left (step_trigger);
+// released at their start, the waiting blocks took SM slots from other
+// packs' kernels (60 small jobs 157 -> 217 us per step).  Measured: argon
+// 4000 atoms 37.4 -> 36.2 us per step, EAM 2048 52 -> 50.  cluster: blocks
+// per cluster (1: none).
+template <typename... P, typename... A>
+inline cudaError_t fmdg_launch(void (*kernel)(P...), int grid, int block, size_t shared, cudaStream_t st, bool overlap,
+                               int cluster, const A &...args)
+{
+    cudaLaunchAttribute at[2];
+    int n = 0;
+    if (cluster > 1)
+    {
+        at[n].id = cudaLaunchAttributeClusterDimension;
+        at[n].val.clusterDim.x = cluster;
+        at[n].val.clusterDim.y = at[n].val.clusterDim.z = 1;
+        n++;
+    }
+    if (overlap)
+    {
+        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[n].val.programmaticStreamSerializationAllowed = 1;
+        n++;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = shared;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = n;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+// the next kernel may be set up from here on / wait for the kernels before
+// this one (nothing they wrote may be touched earlier, and every block of a
+// step kernel must wait); no-ops without an overlapping launch
+__device__ __forceinline__ void step_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void step_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // refresh modes
 #define FMDG_REFRESH_ONLY  0     // positions already updated
 #define FMDG_REFRESH_VV    1     // velocity-Verlet start step first
@@ -402,16 +456,23 @@ __device__ __forceinline__ float d2f_rn(double x)
     return __uint_as_float(f | (hi & 0x80000000u));
 }
 
+// binary32 -> binary64 with integer operations (exact); zero, subnormal and
+// non-finite inputs take the conversion instruction
+__device__ __forceinline__ double f2d(float x)
+{
+    const unsigned b = __float_as_uint(x), e = (b >> 23) & 0xffu;
+    if (e - 1u > 253u) return (double)x;
+    return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
+}
+
 // floor_div as an int, through a binary32 estimate when its fraction is
 // clear of an integer by more than its error (then both agree; one binary64
 // instruction instead of a dozen -- binary64 issues at 1/64 of the binary32
 // rate on GB300), else in binary64.  Results below -2 or above 2^30 come
-// back as -2 (callers test against [-1, nc]).  (Conversion-free forms of
-// the binary32 path -- d2f_rn, a magic-number floor -- measured no faster:
-// the binning kernel is memory bound.)
+// back as -2 (callers test against [-1, nc]).
 __device__ __forceinline__ int cell_floor(double x, double h, double inv_h, float inv_hf)
 {
-    const float qf = __fmul_rn((float)x, inv_hf);
+    const float qf = __fmul_rn(d2f_rn(x), inv_hf);
     const float ff = floorf(qf);
     const float fr = __fsub_rn(qf, ff);
     const float m = 4e-7f * (fabsf(qf) + 1.f);

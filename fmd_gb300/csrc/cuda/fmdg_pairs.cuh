@@ -47,16 +47,16 @@ __device__ __forceinline__ void ld_row32(const float4 *p, float4 &a, float4 &b)
 // instruction (conversions issue at the binary64 rate on GB300)
 __device__ __forceinline__ float small_int_f(int v) { return __int_as_float(0x4B400000 + v) - 12582912.f; }
 
-// Block prologue: pair parameters, per-kind constants and the 27 stencil
-// offsets into shared memory.  DF: also the double-float parameters and
-// offset remainders (binary64 mode).  Everything was formed on the host
-// (no binary64 or conversion work here).
-template <bool DF, bool ONE>
-__device__ __forceinline__ void load_pot(const Geo &g, SmemPotT<DF, ONE> &sp, const float4 *pf = nullptr)
+// Block prologue: pair parameters, per-kind constants and (OFF: the
+// per-step kernels) the 27 stencil offsets into shared memory.  DF: also the
+// double-float parameters and offset remainders (binary64 mode).  Everything
+// was formed on the host: binary64 or conversion work here would issue once
+// per warp, which was a fifth of a small system's force kernel (4000 argon
+// atoms: 4450 of 23 000 cycles).  pf: the binary32 parameter table (g.pairf,
+// or the skin kernels' scaled frame skin_params(g)).
+template <bool OFF, bool DF, bool ONE>
+__device__ __forceinline__ void load_pot(const Geo &g, SmemPotT<DF, ONE> &sp, const float4 *pf)
 {
-    // pf: the binary32 parameter table (default g.pairf; the skin kernels
-    // pass skin_params(g), their scaled frame)
-    if (!pf) pf = g.pairf;
     const int nk2 = ONE ? 1 : g.nkinds * g.nkinds;
     for (int k = threadIdx.x; k < nk2; k += blockDim.x)
     {
@@ -72,14 +72,11 @@ __device__ __forceinline__ void load_pot(const Geo &g, SmemPotT<DF, ONE> &sp, co
         sp.hk[k] = g.st.hk[k];
         sp.elem[k] = g.eam_elem[k];
     }
-    // remainders cellh - binary32 cellh (3 binary64 operations per block)
-    const float lx = (float)(g.cellh[0] - (double)g.cellh_f[0]), ly = (float)(g.cellh[1] - (double)g.cellh_f[1]),
-                lz = (float)(g.cellh[2] - (double)g.cellh_f[2]);
-    for (int c = threadIdx.x; c < (ONE ? 0 : 27); c += blockDim.x)
+    for (int c = threadIdx.x; c < (OFF ? 27 : 0); c += blockDim.x)
     {
         const float ox = small_int_f(c / 9 - 1), oy = small_int_f((c / 3) % 3 - 1), oz = small_int_f(c % 3 - 1);
         sp.off[c] = make_float4(ox * g.cellh_f[0], oy * g.cellh_f[1], oz * g.cellh_f[2], 0.f);
-        sp.offl[c] = make_float4(ox * lx, oy * ly, oz * lz, 0.f);
+        sp.offl[c] = make_float4(ox * g.cellh_lo[0], oy * g.cellh_lo[1], oz * g.cellh_lo[2], 0.f);
     }
     __syncthreads();
 }

@@ -17,25 +17,27 @@ __device__ __forceinline__ void slot_rel_build(const Geo &g, Dyn *dyn, int t, co
     const double o3[3] = {ob.x, ob.y, ob.z};
     float l3[3];
     double u3[3];
-    const double xs = g.xs;     // (1 in binary64 mode: xll below holds remainders of unscaled values)
+    // (the scale is 1 in binary64 mode, the remainders below are of unscaled values)
+    const bool fp64 = g.prec == FMDG_PREC_FP64;
+    const double xs = g.xs;
+    auto scaled = [&](double u) { return fp64 ? u : u * xs; };
     for (int d = 0; d < 3; d++)
     {
         double u = x[d] - o3[d];
-        float uf = d2f_rn(u * xs);
+        float uf = d2f_rn(scaled(u));
         // unwrap across a periodic face (binary64 test near half a box)
         if (g.pbc[d] && fabsf(uf) > 0.49f * g.l_f[d])
         {
             if (u > 0.5 * g.l[d]) u -= g.l[d];
             else if (u < -0.5 * g.l[d]) u += g.l[d];
-            uf = d2f_rn(u * xs);
+            uf = d2f_rn(scaled(u));
         }
         l3[d] = uf;
         u3[d] = u;
     }
     g.xl[t] = make_float4(l3[0], l3[1], l3[2], kb);
-    if (g.prec == FMDG_PREC_FP64)
-        g.xll[t] = make_float4((float)(u3[0] - (double)l3[0]), (float)(u3[1] - (double)l3[1]),
-                               (float)(u3[2] - (double)l3[2]), 0.f);
+    if (fp64)
+        g.xll[t] = make_float4(d2f_rn(u3[0] - f2d(l3[0])), d2f_rn(u3[1] - f2d(l3[1])), d2f_rn(u3[2] - f2d(l3[2])), 0.f);
     const float4 o = g.xb[t];
     const float dx = l3[0] - o.x, dy = l3[1] - o.y, dz = l3[2] - o.z;
     if (!(dx * dx + dy * dy + dz * dz <= g.half_skin2)) dyn->rebuild = 1;
@@ -54,8 +56,9 @@ __device__ __forceinline__ void prep_skin_atom(const Geo &g, Dyn *dyn, int i, in
     // relative to the current cell (a rebuild starts from these)
     const double4_32a oc = g.corig[c];
     const double ux = x[0] - oc.x, uy = x[1] - oc.y, uz = x[2] - oc.z;
-    const double xs = g.xs;     // (1 in binary64 mode: the remainders below are of unscaled values)
-    const float lx = d2f_rn(ux * xs), ly = d2f_rn(uy * xs), lz = d2f_rn(uz * xs);
+    const bool fp64 = g.prec == FMDG_PREC_FP64;      // (scale 1)
+    const double xs = g.xs;
+    const float lx = d2f_rn(fp64 ? ux : ux * xs), ly = d2f_rn(fp64 ? uy : uy * xs), lz = d2f_rn(fp64 ? uz : uz * xs);
     g.xf4[i] = make_float4(lx, ly, lz, kb);
     if (relative) slot_rel_build(g, dyn, t, x, kb);
 }

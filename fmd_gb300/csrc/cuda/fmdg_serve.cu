@@ -446,8 +446,10 @@ int rebuild(fmdg_server_t *S, Pack &p)
     // re-captures 10-11 kernels, not chunk_steps times as many
     int rc = FMDG_OK, nk = 0;
     {
+        P.overlap = true;
         int a = fmdg_pack_launch_refresh(P);
         int b = a < 0 ? a : fmdg_pack_launch_forces(P, 7);
+        P.overlap = false;
         if (a < 0 || b < 0) rc = -(a < 0 ? a : b);
         else nk = a + b;
     }

@@ -68,24 +68,17 @@ struct SkinOffT
 template <bool LO>
 __device__ __forceinline__ void load_offsets(const Geo &g, SkinOffT<LO> &so)
 {
-    const int R = g.srad, W = 2 * R + 1;
-    // remainders cellh xs - cellh_s (3 binary64 operations per block)
-    const float lx = (float)(g.cellh[0] * g.xs - (double)g.cellh_s[0]),
-                ly = (float)(g.cellh[1] * g.xs - (double)g.cellh_s[1]),
-                lz = (float)(g.cellh[2] * g.xs - (double)g.cellh_s[2]);
-    for (int c = threadIdx.x; c < W * W * W; c += blockDim.x)
+    // (constant divisors: the stencil is 3 or 5 cells wide)
+    const int R = g.srad, n = R == 1 ? 27 : 125;
+    for (int c = threadIdx.x; c < n; c += blockDim.x)
     {
-        const float ox = small_int_f(c / (W * W) - R), oy = small_int_f((c / W) % W - R), oz = small_int_f(c % W - R);
+        const int cx = R == 1 ? c / 9 : c / 25, cy = R == 1 ? c / 3 % 3 : c / 5 % 5, cz = R == 1 ? c % 3 : c % 5;
+        const float ox = small_int_f(cx - R), oy = small_int_f(cy - R), oz = small_int_f(cz - R);
         so.off[c] = make_float4(ox * g.cellh_s[0], oy * g.cellh_s[1], oz * g.cellh_s[2], __int_as_float(c));
-        if (LO) so.offl[c] = make_float4(ox * lx, oy * ly, oz * lz, 0.f);
+        if (LO) so.offl[c] = make_float4(ox * g.cellh_slo[0], oy * g.cellh_slo[1], oz * g.cellh_slo[2], 0.f);
     }
     __syncthreads();
 }
-
-// the scaled frame (Geo::xs): binary32 xs^2 (force constants) and the EAM
-// r^2-grid index factor of a scaled r^2
-__device__ __forceinline__ float scaled_xs2(const Geo &g) { return (float)(g.xs * g.xs); }
-__device__ __forceinline__ float scaled_index_factor(const Geo &g) { return (float)(g.inv_dr2 * (g.inv_xs * g.inv_xs)); }
 
 __device__ __forceinline__ float norm2(float3 v)
 {
@@ -413,6 +406,7 @@ __device__ __forceinline__ dfl group_sum(dfl v, int G)
 template <class L>
 __global__ void k_skin_start(__grid_constant__ const L loc)
 {
+    step_wait();
     int bx, nb;
     const Geo &g = loc_geo(loc, bx, nb);
     if (loc_idle(loc, g)) return;
@@ -513,6 +507,7 @@ __device__ __forceinline__ void finish_build(Dyn *dyn, int nb)
 template <class L>
 __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_nlist_skin(__grid_constant__ const L loc)
 {
+    step_wait();
     int bx, nb;
     const Geo &g = loc_geo(loc, bx, nb);
     if (loc_idle(loc, g)) return;
@@ -638,6 +633,7 @@ __device__ __forceinline__ void build_slot_grouped(const Geo &g, const Side &S, 
 template <int G>
 __global__ void __launch_bounds__(128) k_nlist_skin_grp(__grid_constant__ const LocOne loc)
 {
+    step_wait();
     static_assert(G >= 2 && G <= 32 && (G & (G - 1)) == 0, "G: a power of two up to the warp");
     const Geo &g = loc.g;
     Dyn *dyn = g.dyn;
@@ -742,16 +738,17 @@ __device__ __forceinline__ void group_forces(const dfl (&v)[5], int gl, bool the
 // 2^lane_log lanes per slot (see k_force_skin).  LEAN (binary32, one kind, no group): the pair's table
 // row and cutoff in registers, no per-entry kind or group lookups.
 template <class L, bool MIXED, bool HYBRID, bool LEAN>
-__global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density_skin(__grid_constant__ const L loc, int rec)
+__global__ void __launch_bounds__(L::max_threads, MIXED ? L::min_blocks : L::df_min_blocks) k_density_skin(__grid_constant__ const L loc, int rec)
 {
     int bx, nb;
     const Geo &g = loc_geo(loc, bx, nb);
-    if (loc_idle(loc, g)) return;
     const int group = g.st.group;
     __shared__ SmemPotT<!MIXED, LEAN> sp;
     __shared__ SkinOffT<!MIXED || !LEAN> so;   // lean binary32 kernels: no remainders (exact on a cubic grid)
-    load_pot(g, sp, skin_params(g));
+    load_pot<false>(g, sp, skin_params(g));
     load_offsets(g, so);
+    step_wait();        // (the tables above were set up before any step)
+    if (loc_idle(loc, g)) return;
     Dyn *dyn = g.dyn;
     const Side S = g.side[dyn->cur];
     const int gl = L::one_lane ? 0 : g.lane_log, lane = threadIdx.x & ((1 << gl) - 1);
@@ -777,7 +774,7 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density_skin(
             {
                 // double-float pair arithmetic (fmdg_df.cuh)
                 const float4 ih = on ? xi : make_float4(0.f, 0.f, 0.f, 0.f), il = on ? g.xll[t] : ih;
-                const dfl inv_h = df_of(df_split(g.inv_dr2));
+                const dfl inv_h = df_of(g.inv_h_df);
                 const float kmax = (float)(nint - 1);
                 auto pair = [&](int js, float4 xjf, float4 o) {
                     if (group >= 0 && g.gslot[js] != group) return;
@@ -801,7 +798,7 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density_skin(
                 // branch-free walk (table rows read for every entry, entries
                 // beyond the cutoff add zero); near-cutoff entries decided in
                 // binary64 after the walk, as in the lean force kernel
-                const float inv_h = scaled_index_factor(g);   // (scaled r^2: index only)
+                const float inv_h = g.inv_hi_f;   // (scaled r^2: index only)
                 const float kmax = (float)(nint - 1);
                 const float4 *trho = g.pkf_rho + (size_t)sp.pairs[0].jloc * nint;
                 const float rc2f = sp.pf[0][2], band = 2e-5f * rc2f;
@@ -850,7 +847,7 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density_skin(
             }
             else
             {
-                const float inv_h = scaled_index_factor(g);   // (scaled r^2: index only)
+                const float inv_h = g.inv_hi_f;   // (scaled r^2: index only)
                 const float kmax = (float)(nint - 1);
                 Acc32<1> ac;
                 for_each_slot_pair(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
@@ -877,6 +874,7 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density_skin(
         if constexpr (L::split_shares)
             if (M > 1) part_tree(part, M, 1, dens);
     }
+    step_trigger();
     // embedding, one thread per slot
     const double rho = group_value(dens[0], gl);
     const int t = slot_of_thread(g, bx, gl);
@@ -939,17 +937,18 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density_skin(
 // group): pair parameters in registers, no per-entry kind or group
 // lookups, hardware exp2 / rsqrt / rcp approximations.
 template <class L, int CAT, bool MIXED, bool LEAN>
-__global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L::min_blocks) k_force_skin(__grid_constant__ const L loc, int finish, int rec)
+__global__ void __launch_bounds__(L::max_threads, !MIXED ? L::df_min_blocks : (LEAN ? L::lean_min_blocks : L::min_blocks)) k_force_skin(__grid_constant__ const L loc, int finish, int rec)
 {
     int bx, nb;
     const Geo &g = loc_geo(loc, bx, nb);
-    if (loc_idle(loc, g)) return;
     const int group = g.st.group;
     const double dt = g.st.dt;
     __shared__ SmemPotT<!MIXED, LEAN> sp;
     __shared__ SkinOffT<!MIXED || !LEAN> so;   // lean binary32 kernels: no remainders (exact on a cubic grid)
-    load_pot(g, sp, skin_params(g));
+    load_pot<false>(g, sp, skin_params(g));
     load_offsets(g, so);
+    step_wait();        // (the tables above were set up before any step)
+    if (loc_idle(loc, g)) return;
     Dyn *dyn = g.dyn;
     const Side S = g.side[dyn->cur];
     const int cap = g.cap;
@@ -980,7 +979,7 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
                 // double-float pair arithmetic (fmdg_df.cuh, df_pair)
                 const float4 ih = on ? xi : make_float4(0.f, 0.f, 0.f, 0.f), il = on ? g.xll[t] : ih;
                 const dfl fpi = ((CAT == CAT_EAM || CAT == CAT_HYBRID) && on) ? df_of(g.fpdf[t]) : dfl{0.f, 0.f};
-                const dfl inv_h = df_of(df_split(g.inv_dr2));
+                const dfl inv_h = df_of(g.inv_h_df);
                 const float kmax = (float)(nint - 1);
                 auto pair = [&](auto with_e, int js, float4 xjf, float4 o) {
                     if (group >= 0 && g.gslot[js] != group) return;
@@ -1021,12 +1020,12 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
                 // force factors from scaled geometry.  Morse: 2^((r0' - r')
                 // alpha' log2 e) with alpha' = alpha / xs, r0' = r0 xs, factor
                 // 2 alpha D0 xs = 2 alpha' D0 xs^2; LJ: 12 eps4 xs^2 / r'^2
-                const float xs2 = scaled_xs2(g);
+                const float xs2 = g.xs2_f;
                 const float m_c1 = pq.y * 1.44269504f, m_c2 = 2.f * pq.y * pq.x * xs2;
                 const float lj_c = 12.f * pq.x * xs2;
                 const float fpi = (CAT == CAT_EAM) ? g.fpb[t] : 0.f;
-                const float inv_h = (float)g.inv_dr2;         // derivatives with respect to the real r^2
-                const float inv_hi = scaled_index_factor(g);  // table index of the scaled r^2
+                const float inv_h = g.inv_h_df.x;         // derivatives with respect to the real r^2
+                const float inv_hi = g.inv_hi_f;  // table index of the scaled r^2
                 const float kmax = (float)(nint - 1);
                 const int ee = sp.pairs[0].iloc;
                 const float4 *tpr = g.pkf_pr + (size_t)ee * nint * 2;
@@ -1166,10 +1165,10 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
             else
             {
                 const float fpi = (CAT == CAT_EAM || CAT == CAT_HYBRID) ? g.fpb[t] : 0.f;
-                const float inv_h = (float)g.inv_dr2;         // derivatives with respect to the real r^2
-                const float inv_hi = scaled_index_factor(g);  // table index of the scaled r^2
+                const float inv_h = g.inv_h_df.x;         // derivatives with respect to the real r^2
+                const float inv_hi = g.inv_hi_f;  // table index of the scaled r^2
                 const float kmax = (float)(nint - 1);
-                const float xs2 = scaled_xs2(g);
+                const float xs2 = g.xs2_f;
                 Acc32<5> ac;
                 for_each_slot_pair(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
                     if (group >= 0 && g.gslot[js] != group) return;
@@ -1241,6 +1240,7 @@ __global__ void __launch_bounds__(L::max_threads, LEAN ? L::lean_min_blocks : L:
         if constexpr (L::split_shares)
             if (M > 1) part_tree(part, M, thermo ? 5 : 3, sum);
     }
+    step_trigger();
     // the group's sums, then one thread per slot
     double fin[5];
     group_forces(sum, gl, thermo, fin);
@@ -1339,36 +1339,36 @@ size_t stage_bytes(const LocPack &L, int blk, int nv)
 }
 
 template <class L, bool MIXED>
-void launch_force_skin(const L &loc, int cats, int finish, int rec, int nb, int blk, cudaStream_t st, bool lean)
+void launch_force_skin(const L &loc, int cats, int finish, int rec, int nb, int blk, cudaStream_t st, bool lean, bool overlap)
 {
     const size_t sh = stage_bytes(loc, blk, 5);
     const int ncat = __builtin_popcount(cats);
-    if (ncat > 1) k_force_skin<L, CAT_HYBRID, MIXED, false><<<nb, blk, sh, st>>>(loc, finish, rec);
+    if (ncat > 1) fmdg_launch(k_force_skin<L, CAT_HYBRID, MIXED, false>, nb, blk, sh, st, overlap, 1, loc, finish, rec);
     else if (MIXED && lean)
     {
-        if (cats == (1 << FMDG_POT_LJ)) k_force_skin<L, CAT_LJ, true, true><<<nb, blk, sh, st>>>(loc, finish, rec);
-        else if (cats == (1 << FMDG_POT_MORSE)) k_force_skin<L, CAT_MORSE, true, true><<<nb, blk, sh, st>>>(loc, finish, rec);
-        else k_force_skin<L, CAT_EAM, true, true><<<nb, blk, sh, st>>>(loc, finish, rec);
+        if (cats == (1 << FMDG_POT_LJ)) fmdg_launch(k_force_skin<L, CAT_LJ, true, true>, nb, blk, sh, st, overlap, 1, loc, finish, rec);
+        else if (cats == (1 << FMDG_POT_MORSE)) fmdg_launch(k_force_skin<L, CAT_MORSE, true, true>, nb, blk, sh, st, overlap, 1, loc, finish, rec);
+        else fmdg_launch(k_force_skin<L, CAT_EAM, true, true>, nb, blk, sh, st, overlap, 1, loc, finish, rec);
     }
-    else if (cats == (1 << FMDG_POT_LJ)) k_force_skin<L, CAT_LJ, MIXED, false><<<nb, blk, sh, st>>>(loc, finish, rec);
-    else if (cats == (1 << FMDG_POT_MORSE)) k_force_skin<L, CAT_MORSE, MIXED, false><<<nb, blk, sh, st>>>(loc, finish, rec);
-    else k_force_skin<L, CAT_EAM, MIXED, false><<<nb, blk, sh, st>>>(loc, finish, rec);
+    else if (cats == (1 << FMDG_POT_LJ)) fmdg_launch(k_force_skin<L, CAT_LJ, MIXED, false>, nb, blk, sh, st, overlap, 1, loc, finish, rec);
+    else if (cats == (1 << FMDG_POT_MORSE)) fmdg_launch(k_force_skin<L, CAT_MORSE, MIXED, false>, nb, blk, sh, st, overlap, 1, loc, finish, rec);
+    else fmdg_launch(k_force_skin<L, CAT_EAM, MIXED, false>, nb, blk, sh, st, overlap, 1, loc, finish, rec);
 }
 
 template <class L>
-void launch_density_skin(const L &loc, bool mixed, bool hyb, int rec, int nb, int blk, cudaStream_t st, bool lean)
+void launch_density_skin(const L &loc, bool mixed, bool hyb, int rec, int nb, int blk, cudaStream_t st, bool lean, bool overlap)
 {
     const size_t sh = stage_bytes(loc, blk, 1);
     if (mixed)
     {
-        if (hyb) k_density_skin<L, true, true, false><<<nb, blk, sh, st>>>(loc, rec);
-        else if (lean) k_density_skin<L, true, false, true><<<nb, blk, sh, st>>>(loc, rec);
-        else k_density_skin<L, true, false, false><<<nb, blk, sh, st>>>(loc, rec);
+        if (hyb) fmdg_launch(k_density_skin<L, true, true, false>, nb, blk, sh, st, overlap, 1, loc, rec);
+        else if (lean) fmdg_launch(k_density_skin<L, true, false, true>, nb, blk, sh, st, overlap, 1, loc, rec);
+        else fmdg_launch(k_density_skin<L, true, false, false>, nb, blk, sh, st, overlap, 1, loc, rec);
     }
     else
     {
-        if (hyb) k_density_skin<L, false, true, false><<<nb, blk, sh, st>>>(loc, rec);
-        else k_density_skin<L, false, false, false><<<nb, blk, sh, st>>>(loc, rec);
+        if (hyb) fmdg_launch(k_density_skin<L, false, true, false>, nb, blk, sh, st, overlap, 1, loc, rec);
+        else fmdg_launch(k_density_skin<L, false, false, false>, nb, blk, sh, st, overlap, 1, loc, rec);
     }
 }
 
@@ -1376,8 +1376,7 @@ void launch_density_skin(const L &loc, bool mixed, bool hyb, int rec, int nb, in
 
 int fmdg_pack_launch_start(const fmdg_pack_launch &P)
 {
-    k_skin_start<<<P.la.bstart[P.nsys], 128, 0, P.stream>>>(P.la);
-    cudaError_t e = cudaGetLastError();
+    const cudaError_t e = fmdg_launch(k_skin_start<LocPack>, P.la.bstart[P.nsys], 128, 0, P.stream, P.overlap, 1, P.la);
     if (e != cudaSuccess) return -fmdg_fail("pack start", e);
     return 1;
 }
@@ -1392,13 +1391,13 @@ int fmdg_pack_launch_forces(const fmdg_pack_launch &P, int phases)
     int n = 0;
     if (phases & 1)
     {
-        k_nlist_skin<<<nab, 128, 0, st>>>(P.la);
+        fmdg_launch(k_nlist_skin<LocPack>, nab, 128, 0, st, P.overlap, 1, P.la);
         n++;
     }
     if ((phases & 2) && (P.cats & (1 << FMDG_POT_EAM)))
     {
-        if (P.shares) launch_density_skin(LocPackShares{P.lf}, P.mixed != 0, __builtin_popcount(P.cats) > 1, REC_FULL, nfb, P.fblk, st, P.lean != 0);
-        else launch_density_skin(P.lf, P.mixed != 0, __builtin_popcount(P.cats) > 1, REC_FULL, nfb, P.fblk, st, P.lean != 0);
+        if (P.shares) launch_density_skin(LocPackShares{P.lf}, P.mixed != 0, __builtin_popcount(P.cats) > 1, REC_FULL, nfb, P.fblk, st, P.lean != 0, P.overlap);
+        else launch_density_skin(P.lf, P.mixed != 0, __builtin_popcount(P.cats) > 1, REC_FULL, nfb, P.fblk, st, P.lean != 0, P.overlap);
         n++;
     }
     if (phases & 4)
@@ -1406,11 +1405,11 @@ int fmdg_pack_launch_forces(const fmdg_pack_launch &P, int phases)
         if (P.shares)
         {
             const LocPackShares L{P.lf};
-            if (P.mixed) launch_force_skin<LocPackShares, true>(L, P.cats, 1, REC_FULL, nfb, P.fblk, st, P.lean != 0);
-            else launch_force_skin<LocPackShares, false>(L, P.cats, 1, REC_FULL, nfb, P.fblk, st, false);
+            if (P.mixed) launch_force_skin<LocPackShares, true>(L, P.cats, 1, REC_FULL, nfb, P.fblk, st, P.lean != 0, P.overlap);
+            else launch_force_skin<LocPackShares, false>(L, P.cats, 1, REC_FULL, nfb, P.fblk, st, false, P.overlap);
         }
-        else if (P.mixed) launch_force_skin<LocPack, true>(P.lf, P.cats, 1, REC_FULL, nfb, P.fblk, st, P.lean != 0);
-        else launch_force_skin<LocPack, false>(P.lf, P.cats, 1, REC_FULL, nfb, P.fblk, st, false);
+        else if (P.mixed) launch_force_skin<LocPack, true>(P.lf, P.cats, 1, REC_FULL, nfb, P.fblk, st, P.lean != 0, P.overlap);
+        else launch_force_skin<LocPack, false>(P.lf, P.cats, 1, REC_FULL, nfb, P.fblk, st, false, P.overlap);
         n++;
     }
     cudaError_t e = cudaGetLastError();
@@ -1441,12 +1440,12 @@ int fmdg_skin_launch_nlist(fmdg_sys_t *s, bool prepped)
     const int nbg = fmdg_grid(cap > 0 ? cap * G : 1, 128);
     switch (G)
     {
-    case 2: k_nlist_skin_grp<2><<<nbg, 128, 0, s->stream>>>(L); break;
-    case 4: k_nlist_skin_grp<4><<<nbg, 128, 0, s->stream>>>(L); break;
-    case 8: k_nlist_skin_grp<8><<<nbg, 128, 0, s->stream>>>(L); break;
-    case 16: k_nlist_skin_grp<16><<<nbg, 128, 0, s->stream>>>(L); break;
-    case 32: k_nlist_skin_grp<32><<<nbg, 128, 0, s->stream>>>(L); break;
-    default: k_nlist_skin<<<nbg, 128, 0, s->stream>>>(L); break;
+    case 2: fmdg_launch(k_nlist_skin_grp<2>, nbg, 128, 0, s->stream, s->overlap, 1, L); break;
+    case 4: fmdg_launch(k_nlist_skin_grp<4>, nbg, 128, 0, s->stream, s->overlap, 1, L); break;
+    case 8: fmdg_launch(k_nlist_skin_grp<8>, nbg, 128, 0, s->stream, s->overlap, 1, L); break;
+    case 16: fmdg_launch(k_nlist_skin_grp<16>, nbg, 128, 0, s->stream, s->overlap, 1, L); break;
+    case 32: fmdg_launch(k_nlist_skin_grp<32>, nbg, 128, 0, s->stream, s->overlap, 1, L); break;
+    default: fmdg_launch(k_nlist_skin<LocOne>, nbg, 128, 0, s->stream, s->overlap, 1, L); break;
     }
     s->launches++;
     FMDG_CK(cudaGetLastError());
@@ -1459,7 +1458,7 @@ static bool lean_system(const fmdg_sys_t *s) { return s->nkinds == 1 && s->g.st.
 int fmdg_skin_launch_density(fmdg_sys_t *s)
 {
     launch_density_skin(LocOne{s->g}, s->g.prec == FMDG_PREC_MIXED, __builtin_popcount(s->cats) > 1,
-                        s->rec, fmdg_force_blocks(s), s->fblk, s->stream, lean_system(s));
+                        s->rec, fmdg_force_blocks(s), s->fblk, s->stream, lean_system(s), s->overlap);
     s->launches++;
     FMDG_CK(cudaGetLastError());
     return FMDG_OK;
@@ -1470,8 +1469,8 @@ int fmdg_skin_launch_pair_forces(fmdg_sys_t *s, int finish)
     const LocOne L{s->g};
     const int nb = fmdg_force_blocks(s);
     if (s->g.prec == FMDG_PREC_MIXED)
-        launch_force_skin<LocOne, true>(L, s->cats, finish, s->rec, nb, s->fblk, s->stream, lean_system(s));
-    else launch_force_skin<LocOne, false>(L, s->cats, finish, s->rec, nb, s->fblk, s->stream, false);
+        launch_force_skin<LocOne, true>(L, s->cats, finish, s->rec, nb, s->fblk, s->stream, lean_system(s), s->overlap);
+    else launch_force_skin<LocOne, false>(L, s->cats, finish, s->rec, nb, s->fblk, s->stream, false, s->overlap);
     s->launches++;
     FMDG_CK(cudaGetLastError());
     return FMDG_OK;
