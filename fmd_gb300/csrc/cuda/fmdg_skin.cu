@@ -796,53 +796,72 @@ __global__ void __launch_bounds__(L::max_threads, MIXED ? L::min_blocks : L::df_
             else if constexpr (LEAN)
             {
                 // branch-free walk (table rows read for every entry, entries
-                // beyond the cutoff add zero); near-cutoff entries decided in
-                // binary64 after the walk, as in the lean force kernel
+                // beyond the cutoff add zero), in rounds of four as in the
+                // lean force kernel: cutoff decided in binary32, a round with
+                // an entry near it gone through again (256k: 84 -> 77 us)
                 const float inv_h = g.inv_hi_f;   // (scaled r^2: index only)
                 const float kmax = (float)(nint - 1);
                 const float4 *trho = g.pkf_rho + (size_t)sp.pairs[0].jloc * nint;
-                const float rc2f = sp.pf[0][2], band = 2e-5f * rc2f;
+                const float rc2f = sp.pf[0][2], band = 5e-6f * rc2f;
                 const double rc2 = sp.pairs[0].p[2];
                 Acc32<1> ac;
-                int npend = 0, pend = 0;
-                float pr2 = 0.f;
-                for_each_slot_pair<true>(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
-                    const float3 rv = rv_of(xi, xj, o);
-                    const float r2 = rv.x * rv.x + rv.y * rv.y + rv.z * rv.z;
-                    const bool near = fabsf(r2 - rc2f) <= band;
-                    const bool in = (r2 < rc2f) && !near;
-                    npend += near;
-                    pend = near ? js : pend;
-                    pr2 = near ? r2 : pr2;
+                auto value = [&](float r2) {
                     float b;
                     const int ir2 = table_index(r2 * inv_h, kmax, b);
-                    const float v = spl_val(trho[ir2], b);
-                    ac.part[0] += in ? v : 0.f;
-                }, [&](int k) { ac.entries(k); });
-                ac.flush();
-                if (npend == 1)
-                {
-                    if (geom64_mi(g, g.xd[t], g.xd[pend]).r2 < rc2)
+                    return spl_val(trho[ir2], b);
+                };
+                auto round = [&](int4 e4, int left, auto last) {
+                    constexpr bool LAST = decltype(last)::value;
+                    const int e[4] = {e4.x, (LAST && left < 2) ? e4.x : e4.y, (LAST && left < 3) ? e4.x : e4.z,
+                                      LAST ? e4.x : e4.w};
+                    float4 x[4];
+                    for (int w = 0; w < 4; w++) x[w] = g.xl[e[w] & SLOT_MASK];
+                    float r2[4];
+                    for (int w = 0; w < 4; w++)
                     {
-                        float b;
-                        const int ir2 = table_index(pr2 * inv_h, kmax, b);
-                        ac.part[0] += spl_val(trho[ir2], b);
-                        ac.flush();
+                        r2[w] = norm2(rv_of(xi, x[w], so.off[(unsigned)e[w] >> SLOT_BITS]));
+                        if (LAST && w >= left) r2[w] = 4.f * rc2f;
                     }
-                }
-                else if (npend > 1)
+                    for (int w = 0; w < 4; w++)
+                    {
+                        const float y = value(r2[w]);
+                        ac.part[0] += r2[w] < rc2f ? y : 0.f;
+                    }
+                    const float near = fminf(fminf(fabsf(r2[0] - rc2f), fabsf(r2[1] - rc2f)),
+                                             fminf(fabsf(r2[2] - rc2f), fabsf(r2[3] - rc2f)));
+                    if (near <= band)
+                        for (int w = 0; w < 4; w++)
+                            if (fabsf(r2[w] - rc2f) <= band)
+                            {
+                                const bool in = geom64_mi(g, g.xd[t], g.xd[e[w] & SLOT_MASK]).r2 < rc2;
+                                if (in != (r2[w] < rc2f)) ac.part[0] += in ? value(r2[w]) : -value(r2[w]);
+                            }
+                    ac.entries(LAST ? left : 4);
+                };
+                const int cnt = g.nbr_count[t];
+                if (cnt <= g.maxnb)
                 {
-                    for_each_slot_pair<false>(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
-                        const float3 rv = rv_of(xi, xj, o);
-                        const float r2 = rv.x * rv.x + rv.y * rv.y + rv.z * rv.z;
-                        if (!(fabsf(r2 - rc2f) <= band)) return;
-                        if (!(geom64_mi(g, g.xd[t], g.xd[js]).r2 < rc2)) return;
-                        float b;
-                        const int ir2 = table_index(r2 * inv_h, kmax, b);
-                        ac.part[0] += spl_val(trho[ir2], b);
-                    }, [&](int k) { ac.entries(k); });
-                    ac.flush();
+                    const int step = 4 * V;
+                    const size_t cap = g.cap;
+                    const int4 *col = reinterpret_cast<const int4 *>(g.nbr) + t;
+                    int k = 4 * v;
+                    for (; k + 4 <= cnt; k += step)
+                    {
+                        if (k + step + 4 <= cnt)
+                            asm volatile("prefetch.global.L1 [%0];" ::"l"(col + (size_t)((k + step) >> 2) * cap));
+                        round(__ldg(col + (size_t)(k >> 2) * cap), 4, std::false_type{});
+                    }
+                    if (k < cnt) round(__ldg(col + (size_t)(k >> 2) * cap), cnt - k, std::true_type{});
                 }
+                else if (v == 0)
+                    for_each_slot_overflow(g, S, so, t, i, xi, [&](int js, float4 xj, float4 o) {
+                        const float r2 = norm2(rv_of(xi, xj, o));
+                        bool in = r2 < rc2f;
+                        if (fabsf(r2 - rc2f) <= band) in = geom64_mi(g, g.xd[t], g.xd[js]).r2 < rc2;
+                        if (in) ac.part[0] += value(r2);
+                        ac.entries(1);
+                    });
+                ac.flush();
                 acc_rho = {ac.hi[0], ac.lo[0]};
             }
             else
@@ -1052,113 +1071,126 @@ __global__ void __launch_bounds__(L::max_threads, !MIXED ? L::df_min_blocks : (L
                 };
                 // E: the walk sums the energy, W: the pair virial (rv . F =
                 // fa r^2); both on steps that form the thermo record only
-                // (the EAM walk keeps its energy term on every step)
                 auto walk = [&](auto with_e, auto with_v) {
                     constexpr bool E = decltype(with_e)::value;
                     constexpr bool W = decltype(with_v)::value;
                     constexpr int NA = W ? 5 : (E ? 4 : 3);
                     Acc32<NA> ac;
-                    if constexpr (CAT == CAT_EAM)
-                    {
-                        const float band = 1e-4f * rc2f;
-                        for_each_slot_pair<false>(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
-                            const float3 rv = rv_of(xi, xj, o);
-                            const float r2 = norm2(rv);
-                            bool in = r2 < rc2f;
-                            if (fabsf(r2 - rc2f) <= band) in = geom64_mi(g, g.xd[t], g.xd[js]).r2 < rc2;
-                            if (!in) return;
+                    // adds a pair's force (times sign), energy and virial
+                    auto add = [&](float sign, float3 rv, float r2, float fpj) {
+                        float fa, e;
+                        if constexpr (CAT == CAT_EAM)
+                        {
                             float b;
                             const int ir2 = table_index(r2 * inv_hi, kmax, b);
                             float4 tph, trh;
                             ld_row32(tpr + 2 * ir2, tph, trh);
                             const float phi_d = spl_der_rn(tph, b, inv_h);
                             const float rho_d = spl_der_rn(trh, b, inv_h);
-                            // F'(rho_j): w of the list position; an overflow
-                            // fallback occurrence (code < 0) carries kind bits
-                            const float fpj = __float_as_int(o.w) >= 0 ? xj.w : g.fpb[js];
-                            const float fa = __fmul_rn(-2.f, __fmaf_rn(__fadd_rn(fpi, fpj), rho_d, phi_d));
-                            ac.part[0] = __fmaf_rn(fa, rv.x, ac.part[0]);
-                            ac.part[1] = __fmaf_rn(fa, rv.y, ac.part[1]);
-                            ac.part[2] = __fmaf_rn(fa, rv.z, ac.part[2]);
-                            if constexpr (E) ac.part[3] += 0.5f * spl_val(tph, b);
-                            if constexpr (W) ac.part[NA - 1] += fa * r2;
-                        }, [&](int k) { ac.entries(k); });
-                        ac.flush();
-                    }
-                    else
-                    {
-                        // Branch-free walk: the arithmetic runs for every entry and
-                        // entries beyond the cutoff add zero.  An entry within
-                        // 2e-5 relative of the cutoff (several times the binary32
-                        // error of r^2) is decided in binary64 after the walk: one
-                        // such entry per atom is kept in registers, more (rare)
-                        // send the atom through a second walk over its near
-                        // entries only.
-                        const float band = 2e-5f * rc2f;
-                        int npend = 0, pend = 0;
-                        float3 prv = make_float3(0.f, 0.f, 0.f);
-                        for_each_slot_pair<true>(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
-                            const float3 rv = rv_of(xi, xj, o);
-                            const float r2 = norm2(rv);
-                            const bool near = fabsf(r2 - rc2f) <= band;
-                            const bool in = (r2 < rc2f) && !near;
-                            npend += near;
-                            pend = near ? js : pend;
-                            prv = near ? rv : prv;
-                            float fa, e;
+                            fa = __fmul_rn(-2.f, __fmaf_rn(__fadd_rn(fpi, fpj), rho_d, phi_d));
+                            if constexpr (E) e = 0.5f * spl_val(tph, b);
+                        }
+                        else
                             pair_lm(r2, fa, e);
-                            fa = in ? fa : 0.f;
-                            e = in ? e : 0.f;
-                            ac.part[0] = __fmaf_rn(fa, rv.x, ac.part[0]);
-                            ac.part[1] = __fmaf_rn(fa, rv.y, ac.part[1]);
-                            ac.part[2] = __fmaf_rn(fa, rv.z, ac.part[2]);
-                            if constexpr (E) ac.part[3] += e;
-                            if constexpr (W) ac.part[NA - 1] += fa * r2;
-                        }, [&](int k) { ac.entries(k); });
-                        ac.flush();
-                        if (npend == 1)
+                        fa = __fmul_rn(fa, sign);
+                        ac.part[0] = __fmaf_rn(fa, rv.x, ac.part[0]);
+                        ac.part[1] = __fmaf_rn(fa, rv.y, ac.part[1]);
+                        ac.part[2] = __fmaf_rn(fa, rv.z, ac.part[2]);
+                        if constexpr (E) ac.part[3] += sign * e;
+                        if constexpr (W) ac.part[NA - 1] += fa * r2;
+                    };
+                    // A round of four entries (LAST: the first `left` of
+                    // them).  The cutoff is decided in binary32; when an
+                    // entry of the round lies within `band` of it, the round
+                    // is gone through again and an entry that binary64 decides
+                    // otherwise is added or taken back: one test a round
+                    // instead of several instructions an entry.  (Error of the
+                    // binary32 r^2: coordinates and offsets below 2 rc, three
+                    // roundings each of 1.2e-7 rc and the subtractions' own:
+                    // 5e-7 rc a component, 2e-6 rc^2 at most.)  L1 throughput
+                    // and issue bound the walk (gathers and shared offsets);
+                    // against a flag per entry and a second walk, without the
+                    // record: EAM 256k 142 -> 112 us, Morse 512k 256 -> 250,
+                    // LJ 32k 18.0 -> 16.5.
+                    const float band = 5e-6f * rc2f;
+                    auto round = [&](int4 e4, int left, auto last) {
+                        constexpr bool LAST = decltype(last)::value;
+                        const int e[4] = {e4.x, (LAST && left < 2) ? e4.x : e4.y, (LAST && left < 3) ? e4.x : e4.z,
+                                          LAST ? e4.x : e4.w};
+                        float4 x[4];
+                        for (int w = 0; w < 4; w++) x[w] = g.xl[e[w] & SLOT_MASK];
+                        float3 rv[4];
+                        float r2[4];
+                        for (int w = 0; w < 4; w++)
                         {
-                            if (geom64_mi(g, g.xd[t], g.xd[pend]).r2 < rc2)
+                            rv[w] = rv_of(xi, x[w], so.off[(unsigned)e[w] >> SLOT_BITS]);
+                            r2[w] = norm2(rv[w]);
+                            if (LAST && w >= left) r2[w] = 4.f * rc2f;
+                        }
+                        for (int w = 0; w < 4; w++)
+                        {
+                            if constexpr (CAT == CAT_EAM)
                             {
-                                const float r2 = norm2(prv);
+                                if (r2[w] < rc2f) add(1.f, rv[w], r2[w], x[w].w);
+                            }
+                            else
+                            {
                                 float fa, e;
-                                pair_lm(r2, fa, e);
-                                ac.part[0] = __fmaf_rn(fa, prv.x, ac.part[0]);
-                                ac.part[1] = __fmaf_rn(fa, prv.y, ac.part[1]);
-                                ac.part[2] = __fmaf_rn(fa, prv.z, ac.part[2]);
-                                if constexpr (E) ac.part[3] += e;
-                                if constexpr (W) ac.part[NA - 1] += fa * r2;
-                                ac.flush();
+                                pair_lm(r2[w], fa, e);
+                                const bool in = r2[w] < rc2f;
+                                fa = in ? fa : 0.f;
+                                ac.part[0] = __fmaf_rn(fa, rv[w].x, ac.part[0]);
+                                ac.part[1] = __fmaf_rn(fa, rv[w].y, ac.part[1]);
+                                ac.part[2] = __fmaf_rn(fa, rv[w].z, ac.part[2]);
+                                if constexpr (E) ac.part[3] += in ? e : 0.f;
+                                if constexpr (W) ac.part[NA - 1] += fa * r2[w];
                             }
                         }
-                        else if (npend > 1)
+                        const float near = fminf(fminf(fabsf(r2[0] - rc2f), fabsf(r2[1] - rc2f)),
+                                                 fminf(fabsf(r2[2] - rc2f), fabsf(r2[3] - rc2f)));
+                        if (near <= band)
                         {
-                            for_each_slot_pair<false>(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
-                                const float3 rv = rv_of(xi, xj, o);
-                                const float r2 = norm2(rv);
-                                if (!(fabsf(r2 - rc2f) <= band)) return;
-                                if (!(geom64_mi(g, g.xd[t], g.xd[js]).r2 < rc2)) return;
-                                float fa, e;
-                                pair_lm(r2, fa, e);
-                                ac.part[0] = __fmaf_rn(fa, rv.x, ac.part[0]);
-                                ac.part[1] = __fmaf_rn(fa, rv.y, ac.part[1]);
-                                ac.part[2] = __fmaf_rn(fa, rv.z, ac.part[2]);
-                                if constexpr (E) ac.part[3] += e;
-                                if constexpr (W) ac.part[NA - 1] += fa * r2;
-                            }, [&](int k) { ac.entries(k); });
-                            ac.flush();
+                            for (int w = 0; w < 4; w++)
+                                if (fabsf(r2[w] - rc2f) <= band)
+                                {
+                                    const bool in = geom64_mi(g, g.xd[t], g.xd[e[w] & SLOT_MASK]).r2 < rc2;
+                                    if (in != (r2[w] < rc2f)) add(in ? 1.f : -1.f, rv[w], r2[w], x[w].w);
+                                }
                         }
+                        ac.entries(LAST ? left : 4);
+                    };
+                    const int cnt = g.nbr_count[t];
+                    if (cnt <= g.maxnb)
+                    {
+                        constexpr bool PF = CAT != CAT_EAM;      // prefetch of the next list row
+                        const int step = 4 * V;
+                        const int4 *col = reinterpret_cast<const int4 *>(g.nbr) + t;
+                        int k = 4 * v;
+                        for (; k + 4 <= cnt; k += step)
+                        {
+                            if (PF && k + step + 4 <= cnt)
+                                asm volatile("prefetch.global.L1 [%0];" ::"l"(col + (size_t)((k + step) >> 2) * cap));
+                            round(__ldg(col + (size_t)(k >> 2) * cap), 4, std::false_type{});
+                        }
+                        if (k < cnt) round(__ldg(col + (size_t)(k >> 2) * cap), cnt - k, std::true_type{});
                     }
+                    else if (v == 0)
+                        for_each_slot_overflow(g, S, so, t, i, xi, [&](int js, float4 xj, float4 o) {
+                            const float3 rv = rv_of(xi, xj, o);
+                            const float r2 = norm2(rv);
+                            bool in = r2 < rc2f;
+                            if (fabsf(r2 - rc2f) <= band) in = geom64_mi(g, g.xd[t], g.xd[js]).r2 < rc2;
+                            // (xj.w: kind bits here)
+                            if (in) add(1.f, rv, r2, CAT == CAT_EAM ? g.fpb[js] : 0.f);
+                            ac.entries(1);
+                        });
+                    ac.flush();
                     for (int d = 0; d < 3; d++) sum[d] = {ac.hi[d], ac.lo[d]};
                     if constexpr (E) sum[3] = {ac.hi[3], ac.lo[3]};
                     if constexpr (W) sum[4] = {ac.hi[NA - 1], ac.lo[NA - 1]};
                 };
-                // (the EAM walk keeps its energy term: dropping it measured
-                // slower for that kernel)
                 if (thermo)
                     walk(std::true_type{}, std::true_type{});
-                else if constexpr (CAT == CAT_EAM)
-                    walk(std::true_type{}, std::false_type{});
                 else
                     walk(std::false_type{}, std::false_type{});
             }
