@@ -63,6 +63,7 @@ struct SkinOffT
 {
     float4 off[125];    // image offset of each stencil code, binary32; .w: the code's bits
     float4 offl[LO ? 125 : 1];   // the remainders (binary64 offset - off)
+    unsigned steps[125];         // (ox, oy, oz), for rv_steps
 };
 
 template <bool LO>
@@ -76,6 +77,7 @@ __device__ __forceinline__ void load_offsets(const Geo &g, SkinOffT<LO> &so)
         const float ox = small_int_f(cx - R), oy = small_int_f(cy - R), oz = small_int_f(cz - R);
         so.off[c] = make_float4(ox * g.cellh_s[0], oy * g.cellh_s[1], oz * g.cellh_s[2], __int_as_float(c));
         if (LO) so.offl[c] = make_float4(ox * g.cellh_slo[0], oy * g.cellh_slo[1], oz * g.cellh_slo[2], 0.f);
+        so.steps[c] = __float_as_uint(ox) | __float_as_uint(oy) >> 10 | __float_as_uint(oz) >> 20;
     }
     __syncthreads();
 }
@@ -92,10 +94,25 @@ __device__ __forceinline__ float spl_der_rn(float4 t, float b, float inv_h)
 }
 
 // binary32 pair vector x_i - x_j - offset without the offset's remainder
-// (list-radius prefilters)
+// (prefilters, overflow fallback)
 __device__ __forceinline__ float3 rv_of(float4 xi, float4 xj, float4 o)
 {
     return make_float3(xi.x - xj.x - o.x, xi.y - xj.y - o.y, xi.z - xj.z - o.z);
+}
+
+// The same vector, bit for bit, from the cell steps packed in one word: a
+// step (-2 .. 2) is the top ten bits of its binary32 form, step * cellh is
+// exact, so one fused operation rounds as the subtraction of the offset
+// does.  The walks are bound by L1 wavefronts: a 16-byte row of shared
+// offsets took 4.4 of them per warp and entry beside the position gather's
+// 12, one word takes one or two (EAM 256k density 77 -> 67 us, force
+// 112 -> 102; Morse 512k 250 -> 233; binary64 EAM 256k density 194 -> 187).
+__device__ __forceinline__ float3 rv_steps(float4 xi, float4 xj, unsigned w, float3 h)
+{
+    const float sx = __uint_as_float(w & 0xffc00000u), sy = __uint_as_float((w << 10) & 0xffc00000u),
+                sz = __uint_as_float(w << 20);
+    return make_float3(__fmaf_rn(-sx, h.x, xi.x - xj.x), __fmaf_rn(-sy, h.y, xi.y - xj.y),
+                       __fmaf_rn(-sz, h.z, xi.z - xj.z));
 }
 
 // binary32 pair vector of a list entry with the offset's remainder: the
@@ -344,6 +361,7 @@ __device__ __forceinline__ int prune_share(const Geo &g, const SkinOffT<true> &s
     const float lim = g.rcut2;
     const int4 *col = reinterpret_cast<const int4 *>(g.nbr) + t;
     unsigned *out = g.nbc + (size_t)t * V + v;
+    const float3 h3 = make_float3(g.cellh_s[0], g.cellh_s[1], g.cellh_s[2]);
     int m = 0;
     for (int k = 4 * v; k < cnt; k += 4 * V)
     {
@@ -356,7 +374,7 @@ __device__ __forceinline__ int prune_share(const Geo &g, const SkinOffT<true> &s
         for (int w = 0; w < 4; w++) x[w] = g.xl[e[w] & SLOT_MASK];
         for (int w = 0; w < 4; w++)
         {
-            const float3 d = rv_of(ih, x[w], so.off[e[w] >> SLOT_BITS]);
+            const float3 d = rv_steps(ih, x[w], so.steps[e[w] >> SLOT_BITS], h3);
             if (w < left && d.x * d.x + d.y * d.y + d.z * d.z < lim)
             {
                 *out = e[w];
@@ -802,6 +820,7 @@ __global__ void __launch_bounds__(L::max_threads, MIXED ? L::min_blocks : L::df_
                 const float inv_h = g.inv_hi_f;   // (scaled r^2: index only)
                 const float kmax = (float)(nint - 1);
                 const float4 *trho = g.pkf_rho + (size_t)sp.pairs[0].jloc * nint;
+                const float3 h3 = make_float3(g.cellh_s[0], g.cellh_s[1], g.cellh_s[2]);
                 const float rc2f = sp.pf[0][2], band = 5e-6f * rc2f;
                 const double rc2 = sp.pairs[0].p[2];
                 Acc32<1> ac;
@@ -819,7 +838,7 @@ __global__ void __launch_bounds__(L::max_threads, MIXED ? L::min_blocks : L::df_
                     float r2[4];
                     for (int w = 0; w < 4; w++)
                     {
-                        r2[w] = norm2(rv_of(xi, x[w], so.off[(unsigned)e[w] >> SLOT_BITS]));
+                        r2[w] = norm2(rv_steps(xi, x[w], so.steps[(unsigned)e[w] >> SLOT_BITS], h3));
                         if (LAST && w >= left) r2[w] = 4.f * rc2f;
                     }
                     for (int w = 0; w < 4; w++)
@@ -1108,11 +1127,12 @@ __global__ void __launch_bounds__(L::max_threads, !MIXED ? L::df_min_blocks : (L
                     // binary32 r^2: coordinates and offsets below 2 rc, three
                     // roundings each of 1.2e-7 rc and the subtractions' own:
                     // 5e-7 rc a component, 2e-6 rc^2 at most.)  L1 throughput
-                    // and issue bound the walk (gathers and shared offsets);
+                    // and issue bound the walk;
                     // against a flag per entry and a second walk, without the
                     // record: EAM 256k 142 -> 112 us, Morse 512k 256 -> 250,
                     // LJ 32k 18.0 -> 16.5.
                     const float band = 5e-6f * rc2f;
+                    const float3 h3 = make_float3(g.cellh_s[0], g.cellh_s[1], g.cellh_s[2]);
                     auto round = [&](int4 e4, int left, auto last) {
                         constexpr bool LAST = decltype(last)::value;
                         const int e[4] = {e4.x, (LAST && left < 2) ? e4.x : e4.y, (LAST && left < 3) ? e4.x : e4.z,
@@ -1123,7 +1143,7 @@ __global__ void __launch_bounds__(L::max_threads, !MIXED ? L::df_min_blocks : (L
                         float r2[4];
                         for (int w = 0; w < 4; w++)
                         {
-                            rv[w] = rv_of(xi, x[w], so.off[(unsigned)e[w] >> SLOT_BITS]);
+                            rv[w] = rv_steps(xi, x[w], so.steps[(unsigned)e[w] >> SLOT_BITS], h3);
                             r2[w] = norm2(rv[w]);
                             if (LAST && w >= left) r2[w] = 4.f * rc2f;
                         }
