@@ -119,7 +119,7 @@ void drop_eam(fmdg_sys_t *s)
     Geo &g = s->g;
     g.pk_F = nullptr;
     g.pkf_rho = g.pkf_phi = g.pkf_F = g.pkf_pr = nullptr;
-    g.pkd_rho = g.pkd_phi = nullptr;
+    g.pkd_rho = g.pkd_phi = g.pkd_pr = nullptr;
     s->eam_borrowed = false;
 }
 
@@ -336,7 +336,7 @@ extern "C" void fmdg_destroy(fmdg_sys_t *s)
     dfree(s, (void *)s->g.pairf); dfree(s, (void *)s->g.paird);
     dfree(s, (void *)s->g.pk_F);
     dfree(s, (void *)s->g.pkf_rho); dfree(s, (void *)s->g.pkf_phi); dfree(s, (void *)s->g.pkf_F);
-    dfree(s, (void *)s->g.pkf_pr); dfree(s, (void *)s->g.pkd_rho); dfree(s, (void *)s->g.pkd_phi);
+    dfree(s, (void *)s->g.pkf_pr); dfree(s, (void *)s->g.pkd_rho); dfree(s, (void *)s->g.pkd_phi); dfree(s, (void *)s->g.pkd_pr);
     for (int k = 0; k < s->nturi; k++)
     {
         DTuri &t = s->turi[k];
@@ -521,7 +521,7 @@ extern "C" int fmdg_set_eam(fmdg_sys_t *s, int nelem, int Nrho, double drho, int
     // precision, which the two-sample difference y_k+1 - y_k would not.
     dfree(s, (void *)g.pk_F);
     dfree(s, (void *)g.pkf_rho); dfree(s, (void *)g.pkf_phi); dfree(s, (void *)g.pkf_F);
-    dfree(s, (void *)g.pkf_pr); dfree(s, (void *)g.pkd_rho); dfree(s, (void *)g.pkd_phi);
+    dfree(s, (void *)g.pkf_pr); dfree(s, (void *)g.pkd_rho); dfree(s, (void *)g.pkd_phi); dfree(s, (void *)g.pkd_pr);
     auto pack = [&](const double *y, const double *ydd, double h, int npts, int nfun, const double4_32a **d64,
                     const float4 **d32, const float4 **ddf) -> int {
         const size_t nint = (size_t)npts - 1;
@@ -575,9 +575,25 @@ extern "C" int fmdg_set_eam(fmdg_sys_t *s, int nelem, int Nrho, double drho, int
             }
         if ((rc = dalloc(s, (float4 **)&g.pkf_pr, pr.size()))) return rc;
         FMDG_CK(cudaMemcpyAsync((void *)g.pkf_pr, pr.data(), pr.size() * sizeof(float4), cudaMemcpyHostToDevice, s->stream));
+        // and in double-float: what the slopes need first (eam_pair_row)
+        std::vector<float4> phid(2 * nint * nelem * nelem), rhod(2 * nint * nelem), prd(4 * nint * nelem);
+        FMDG_D2H(phid.data(), g.pkd_phi, phid.size() * sizeof(float4));
+        FMDG_D2H(rhod.data(), g.pkd_rho, rhod.size() * sizeof(float4));
+        for (int e = 0; e < nelem; e++)
+            for (size_t k = 0; k < nint; k++)
+            {
+                const float4 *p = &phid[2 * (((size_t)e * nelem + e) * nint + k)], *r = &rhod[2 * (e * nint + k)];
+                float4 *q = &prd[4 * (e * nint + k)];
+                q[0] = make_float4(p[0].y, p[0].z, p[0].w, r[0].y);
+                q[1] = make_float4(r[0].z, r[0].w, p[1].y, p[1].z);
+                q[2] = make_float4(p[1].w, r[1].y, r[1].z, r[1].w);
+                q[3] = make_float4(p[0].x, p[1].x, 0.f, 0.f);
+            }
+        if ((rc = dalloc(s, (float4 **)&g.pkd_pr, prd.size()))) return rc;
+        FMDG_CK(cudaMemcpyAsync((void *)g.pkd_pr, prd.data(), prd.size() * sizeof(float4), cudaMemcpyHostToDevice, s->stream));
     }
     // the 32-byte row tables are read with 256-bit loads (ld_row32)
-    if (((uintptr_t)g.pkf_pr | (uintptr_t)g.pkd_rho | (uintptr_t)g.pkd_phi) % 32)
+    if (((uintptr_t)g.pkf_pr | (uintptr_t)g.pkd_rho | (uintptr_t)g.pkd_phi | (uintptr_t)g.pkd_pr) % 32)
         return fmdg_set_error("fmdg_set_eam: row tables not 32-byte aligned");
     invalidate_graph(s);
     // other systems may read these tables on their own streams
@@ -713,12 +729,12 @@ extern "C" int fmdg_share_eam(fmdg_sys_t *s, const fmdg_sys_t *owner)
     {
         dfree(s, (void *)g.pk_F);
         dfree(s, (void *)g.pkf_rho); dfree(s, (void *)g.pkf_phi); dfree(s, (void *)g.pkf_F);
-        dfree(s, (void *)g.pkf_pr); dfree(s, (void *)g.pkd_rho); dfree(s, (void *)g.pkd_phi);
+        dfree(s, (void *)g.pkf_pr); dfree(s, (void *)g.pkd_rho); dfree(s, (void *)g.pkd_phi); dfree(s, (void *)g.pkd_pr);
     }
     const Geo &o = owner->g;
     g.pk_F = o.pk_F;
     g.pkf_rho = o.pkf_rho; g.pkf_phi = o.pkf_phi; g.pkf_F = o.pkf_F; g.pkf_pr = o.pkf_pr;
-    g.pkd_rho = o.pkd_rho; g.pkd_phi = o.pkd_phi;
+    g.pkd_rho = o.pkd_rho; g.pkd_phi = o.pkd_phi; g.pkd_pr = o.pkd_pr;
     g.nelem = o.nelem; g.Nrho = o.Nrho; g.Nr2 = o.Nr2; g.drho = o.drho; g.dr2 = o.dr2;
     g.inv_dr2 = o.inv_dr2; g.inv_drho = o.inv_drho;
     s->eam_borrowed = true;
@@ -828,7 +844,7 @@ extern "C" int fmdg_upload(fmdg_sys_t *s, int n, const int *cell_count, const do
         {
             c.take(g.pos, cap); c.take(g.cb, cap); c.take(g.xl, cap); c.take(g.xb, cap);
             c.take(g.xd, cap); c.take(g.gslot, cap); c.take(g.fpb, cap); c.take(g.fpd, cap);
-            c.take(g.xll, cap);
+            c.take(g.xr, 2 * (size_t)cap);
             c.take(g.nbc, pruned); c.take(g.nbc_count, pruned ? (size_t)cap * shares : 0);
         }
     };

@@ -184,10 +184,14 @@ __device__ __forceinline__ dfl df_spl_val(float4 h, float4 l, dfl b)
     return df_fma(t, b, {h.x, l.x});
 }
 
+// k1 + 2 k2 b + 3 k3 b^2
+__device__ __forceinline__ dfl df_slope(dfl k1, dfl k2, dfl k3, dfl b)
+{
+    return df_fma(df_fma(df_mul_f(k3, 3.f), b, df_scale2(k2, 2.f)), b, k1);
+}
+
 // dy/dx = (k1 + 2 k2 b + 3 k3 b^2) * inv_h
 __device__ __forceinline__ dfl df_spl_der(float4 h, float4 l, dfl b, dfl inv_h)
 {
-    dfl t = df_fma(df_mul_f({h.w, l.w}, 3.f), b, df_scale2({h.z, l.z}, 2.f));
-    t = df_fma(t, b, {h.y, l.y});
-    return df_mul(t, inv_h);
+    return df_mul(df_slope({h.y, l.y}, {h.z, l.z}, {h.w, l.w}, b), inv_h);
 }

@@ -88,9 +88,13 @@ struct Geo   // passed by value to kernels
     // (per interval {hi coefficients, lo coefficients}), of the cell-local
     // coordinates and of F'(rho)
     const float4 *pkd_rho, *pkd_phi;
+    const float4 *pkd_pr;       // per element e and interval: phi_ee and rho_e, 64 B (eam_pair_row)
     float4 *xdf;       // per index {xf4, lo parts}: one 32-byte row (one 256-bit load per neighbour)
     float2 *fpdf;
-    float4 *xll;       // skin lists, binary64 mode: lo parts of xl (double-float build-frame positions)
+    // skin lists, binary64 mode: double-float build-frame position of a slot
+    // in one 32-byte row {hi x, y, z, w | lo x, y, z, w}; w: the kind's bits
+    // and 0, or F'(rho) of the slot (one kind: written by the density pass)
+    float4 *xr;
     double inv_dr2, inv_drho;
     // binning scratch
     int *bdest;        // destination interior cell, -1 deleted, -2 stays
@@ -328,7 +332,7 @@ struct fmdg_pack_launch
     int nsys;
     int cats;                   // bit mask (1 << FMDG_POT_*) of the members' pair categories
     int mixed;
-    int lean;                   // every member has one kind (lean binary32 kernels)
+    int lean;                   // every member has one kind (lean kernels)
     int shares;                 // the members' list walks are split into shares (small systems)
     int fblk;                   // threads per block of the list/density/force kernels
     bool overlap;               // the launches are a captured step's (fmdg_launch)

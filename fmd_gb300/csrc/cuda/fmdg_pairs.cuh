@@ -43,6 +43,14 @@ __device__ __forceinline__ void ld_row32(const float4 *p, float4 &a, float4 &b)
         : "l"(p));
 }
 
+// the same of a row that kernels of this step wrote
+__device__ __forceinline__ void ld_slot32(const float4 *p, float4 &a, float4 &b)
+{
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(p));
+}
+
 // small integer v (|v| < 2^22) as binary32 without a conversion
 // instruction (conversions issue at the binary64 rate on GB300)
 __device__ __forceinline__ float small_int_f(int v) { return __int_as_float(0x4B400000 + v) - 12582912.f; }
@@ -209,6 +217,23 @@ __device__ __forceinline__ GeomDF geom_df_of64(const Geom64 &q)
     return p;
 }
 
+// Slopes (dy/db) of phi and rho and the value of phi at fraction b of one
+// interval's 64-byte row.  The coefficients the slopes need fill the row's
+// first 48 bytes: a walk without energies reads 32 + 16 bytes of one line
+// instead of two rows of 32 in two tables, which are gathered from L1 and L2
+// at random.
+__device__ __forceinline__ void eam_pair_row(const float4 *row, dfl b, dfl &phi_s, dfl &rho_s, dfl &phi_v)
+{
+    float4 p, q;
+    ld_row32(row, p, q);
+    const float4 u = __ldg(row + 2);
+    const float2 k0 = __ldg(reinterpret_cast<const float2 *>(row + 3));
+    const dfl p1 = {p.x, q.z}, p2 = {p.y, q.w}, p3 = {p.z, u.x};
+    phi_s = df_slope(p1, p2, p3, b);
+    rho_s = df_slope({p.w, u.y}, {q.x, u.z}, {q.y, u.w}, b);
+    phi_v = df_fma(df_fma(df_fma(p3, b, p2), b, p1), b, {k0.x, k0.y});
+}
+
 // Binary64-mode pair arithmetic in double-float, in the reference's formulas
 // -- LJ src/lj.h:35-56, Morse src/morse.h:35-56, EAM src/eam.h:186-226 --
 // for a pair of category cat: f_i += fa * rv, energy share eh.  fpj() gives
@@ -244,18 +269,25 @@ __device__ __forceinline__ void df_pair(const Geo &g, const SmemPotT<DF, ONE> &s
         dfl b;
         const int ir2 = df_table_index(df_mul(p.r2, inv_h), kmax, b);
         const int ei = pp.iloc, ej = pp.jloc;
+        if (ONE || ei == ej)
+        {
+            // one element: F'_i rho' + F'_j rho' = (F'_i + F'_j) rho', the
+            // table spacing divided out once, both slopes from one row
+            dfl phi_s, rho_s, phi_v;
+            eam_pair_row(g.pkd_pr + 4 * ((size_t)ei * nint + ir2), b, phi_s, rho_s, phi_v);
+            const dfl s = df_add(df_mul(df_add(fpi, fpj()), rho_s), phi_s);
+            fa = df_neg(df_scale2(df_mul(s, inv_h), 2.f));
+            eh = df_scale2(phi_v, 0.5f);
+            return;
+        }
         float4 ph0, ph1, ri0, ri1;
         ld_row32(g.pkd_phi + 2 * (((size_t)ei * ne + ej) * nint + ir2), ph0, ph1);
         ld_row32(g.pkd_rho + 2 * ((size_t)ei * nint + ir2), ri0, ri1);
         const dfl phi_d = df_spl_der(ph0, ph1, b, inv_h);
         const dfl rho_ip = df_spl_der(ri0, ri1, b, inv_h);
-        dfl rho_jp = rho_ip;
-        if (ei != ej)
-        {
-            float4 rj0, rj1;
-            ld_row32(g.pkd_rho + 2 * ((size_t)ej * nint + ir2), rj0, rj1);
-            rho_jp = df_spl_der(rj0, rj1, b, inv_h);
-        }
+        float4 rj0, rj1;
+        ld_row32(g.pkd_rho + 2 * ((size_t)ej * nint + ir2), rj0, rj1);
+        const dfl rho_jp = df_spl_der(rj0, rj1, b, inv_h);
         const dfl fj = fpj();
         fa = df_neg(df_scale2(df_add(df_add(df_mul(fpi, rho_jp), df_mul(fj, rho_ip)), phi_d), 2.f));
         eh = df_scale2(df_spl_val(ph0, ph1, b), 0.5f);

@@ -37,7 +37,11 @@ __device__ __forceinline__ void slot_rel_build(const Geo &g, Dyn *dyn, int t, co
     }
     g.xl[t] = make_float4(l3[0], l3[1], l3[2], kb);
     if (fp64)
-        g.xll[t] = make_float4(d2f_rn(u3[0] - f2d(l3[0])), d2f_rn(u3[1] - f2d(l3[1])), d2f_rn(u3[2] - f2d(l3[2])), 0.f);
+    {
+        g.xr[2 * (size_t)t] = make_float4(l3[0], l3[1], l3[2], kb);
+        g.xr[2 * (size_t)t + 1] =
+            make_float4(d2f_rn(u3[0] - f2d(l3[0])), d2f_rn(u3[1] - f2d(l3[1])), d2f_rn(u3[2] - f2d(l3[2])), 0.f);
+    }
     const float4 o = g.xb[t];
     const float dx = l3[0] - o.x, dy = l3[1] - o.y, dz = l3[2] - o.z;
     if (!(dx * dx + dy * dy + dz * dz <= g.half_skin2)) dyn->rebuild = 1;

@@ -101,7 +101,7 @@ struct Chunk
 struct Pack
 {
     int cls = 0, mixed = 0;
-    int lean = 0;       // one-kind jobs (lean binary32 kernels); a job's variant never depends on the mix
+    int lean = 0;       // one-kind jobs (lean kernels); a job's variant never depends on the mix
     int shares = 0;     // small jobs, whose list walks are split into shares (Geo::share_log > 0)
     cudaStream_t stream = nullptr;
     std::vector<Job *> members;

@@ -56,9 +56,9 @@ constexpr int SLOT_MASK = (1 << SLOT_BITS) - 1;
 // Image offsets of the stencil codes in shared memory, in the scaled frame
 // (Geo::xs): off = (ox, oy, oz) * cellh_s is exact in binary32 (|o| <= 2);
 // the remainder offl = (ox, oy, oz) * (cellh xs - cellh_s) completes it to
-// the binary64 offset (double-float in binary64 mode; in binary32 one more
-// subtraction in the general kernels, zero on a cubic grid).
-template <bool LO>   // LO: with the remainders (binary64 mode, general binary32 kernels); lean layouts go without
+// the binary64 offset (in binary32 one more subtraction in the general
+// kernels, zero on a cubic grid; binary64 mode forms both from the steps).
+template <bool LO>   // LO: with the remainders (general binary32 kernels)
 struct SkinOffT
 {
     float4 off[125];    // image offset of each stencil code, binary32; .w: the code's bits
@@ -164,20 +164,19 @@ __device__ __forceinline__ float axis_gap(int o, float u, float h)
     return o > 0 ? fmaxf(0.f, (float)o * h - u) : (o < 0 ? fmaxf(0.f, u + (float)(-o - 1) * h) : 0.f);
 }
 
-// Binary64 mode: double-float geometry of a list entry (build frame: slot
-// positions xl + xll and the entry's stencil offset) or of an overflow
-// fallback occurrence (code < 0 in o.w: current-cell frame, formed from the
-// binary64 positions); the cutoff decision within 1e-6 relative of the
-// cutoff is the binary64 minimum-image one.
-template <bool DF>
-__device__ __forceinline__ GeomDF skin_geom_df(const Geo &g, const SkinOffT<DF> &so, int t, float4 ih, float4 il, int js,
-                                               float4 xj, float4 o)
+// Binary64 mode: double-float geometry of a list entry (build frame: the
+// slots' rows and the entry's cell steps, times the double-float cell width:
+// exact, and rounded once)
+__device__ __forceinline__ GeomDF skin_geom_df(float4 ih, float4 il, float4 jh, float4 jl, unsigned w, float3 h, float3 hl)
 {
-    const int code = __float_as_int(o.w);
-    if (code >= 0) return geom_df(ih, il, xj, g.xll[js], o, so.offl[code]);
-    return geom_df_of64(geom64_mi(g, g.xd[t], g.xd[js]));
+    const float sx = __uint_as_float(w & 0xffc00000u), sy = __uint_as_float((w << 10) & 0xffc00000u),
+                sz = __uint_as_float(w << 20);
+    return geom_df(ih, il, jh, jl, make_float4(sx * h.x, sy * h.y, sz * h.z, 0.f),
+                   make_float4(sx * hl.x, sy * hl.y, sz * hl.z, 0.f));
 }
 
+// the cutoff decision within 1e-6 relative of the cutoff is the binary64
+// minimum-image one
 __device__ __forceinline__ bool within_cut_df_mi(const Geo &g, int t, int js, dfl r2, float rc2f, double rc2)
 {
     const float d = __fsub_rn(r2.hi, rc2f);
@@ -353,7 +352,7 @@ __device__ __forceinline__ void for_each_slot_pair(const Geo &g, const Side &S, 
 // written to the share's own compact list (entry m at nbc[m cap V + t V + v]:
 // a row over consecutive shares), which the double-float loop then walks.
 // The EAM force pass reuses the density pass's compact lists.
-__device__ __forceinline__ int prune_share(const Geo &g, const SkinOffT<true> &so, int cnt, int t, int v, int V,
+__device__ __forceinline__ int prune_share(const Geo &g, const SkinOffT<false> &so, int cnt, int t, int v, int V,
                                            float4 ih)
 {
     const int cap = g.cap;
@@ -386,10 +385,15 @@ __device__ __forceinline__ int prune_share(const Geo &g, const SkinOffT<true> &s
     return m;
 }
 
-// f(neighbour slot, position, image offset) for the m entries of a share's
-// compact list
+// f(neighbour slot, its double-float row, the entry's cell steps) for the m
+// entries of a share's compact list.  L1 wavefronts bound the walk (80 % of
+// their peak, the FMA pipe at 38 to 50 %), so a neighbour is one 32-byte row
+// and its offset one shared word (rv_steps), F'(rho_j) rides in the row
+// (LEAN) and the EAM slopes come from one 64-byte row (eam_pair_row): 256k
+// EAM density 187 -> 166 us, force 230 -> 175; 300 jobs of 600 to 3000
+// atoms 1464 -> 1160 us a step.
 template <typename F>
-__device__ __forceinline__ void for_each_pruned(const Geo &g, const SkinOffT<true> &so, int m, int t, int v, int V, F &&f)
+__device__ __forceinline__ void for_each_pruned(const Geo &g, const SkinOffT<false> &so, int m, int t, int v, int V, F &&f)
 {
     const size_t row = (size_t)g.cap * V;
     const unsigned *p = g.nbc + (size_t)t * V + v;
@@ -399,7 +403,9 @@ __device__ __forceinline__ void for_each_pruned(const Geo &g, const SkinOffT<tru
         const unsigned e = next;
         p += row;
         if (k + 1 < m) next = *p;
-        f((int)(e & SLOT_MASK), g.xl[e & SLOT_MASK], so.off[e >> SLOT_BITS]);
+        float4 jh, jl;
+        ld_slot32(g.xr + 2 * (size_t)(e & SLOT_MASK), jh, jl);
+        f((int)(e & SLOT_MASK), jh, jl, so.steps[e >> SLOT_BITS]);
     }
 }
 
@@ -498,8 +504,9 @@ __device__ __forceinline__ void record_build(const Geo &g, const Side &S, int t,
     {
         // (xs is 1 in binary64 mode)
         const double4_32a x = g.xd[t], o = g.corig[S.cell_of[i]];
-        g.xll[t] = make_float4((float)(x.x - o.x - (double)xi.x), (float)(x.y - o.y - (double)xi.y),
-                               (float)(x.z - o.z - (double)xi.z), 0.f);
+        g.xr[2 * (size_t)t] = xi;
+        g.xr[2 * (size_t)t + 1] = make_float4((float)(x.x - o.x - (double)xi.x), (float)(x.y - o.y - (double)xi.y),
+                                              (float)(x.z - o.z - (double)xi.z), 0.f);
     }
 }
 
@@ -753,8 +760,9 @@ __device__ __forceinline__ void group_forces(const dfl (&v)[5], int gl, bool the
 }
 
 // EAM pass 1 + embedding (src/eam.h:270-406, src/eam.c:160-179), a group of
-// 2^lane_log lanes per slot (see k_force_skin).  LEAN (binary32, one kind, no group): the pair's table
-// row and cutoff in registers, no per-entry kind or group lookups.
+// 2^lane_log lanes per slot (see k_force_skin).  LEAN (one kind, no group): the pair's table
+// row and cutoff in registers, no per-entry kind or group lookups; F'(rho)
+// goes into the slots' rows.
 template <class L, bool MIXED, bool HYBRID, bool LEAN>
 __global__ void __launch_bounds__(L::max_threads, MIXED ? L::min_blocks : L::df_min_blocks) k_density_skin(__grid_constant__ const L loc, int rec)
 {
@@ -762,7 +770,7 @@ __global__ void __launch_bounds__(L::max_threads, MIXED ? L::min_blocks : L::df_
     const Geo &g = loc_geo(loc, bx, nb);
     const int group = g.st.group;
     __shared__ SmemPotT<!MIXED, LEAN> sp;
-    __shared__ SkinOffT<!MIXED || !LEAN> so;   // lean binary32 kernels: no remainders (exact on a cubic grid)
+    __shared__ SkinOffT<MIXED && !LEAN> so;   // (lean binary32: no remainders, exact on a cubic grid)
     load_pot<false>(g, sp, skin_params(g));
     load_offsets(g, so);
     step_wait();        // (the tables above were set up before any step)
@@ -791,23 +799,32 @@ __global__ void __launch_bounds__(L::max_threads, MIXED ? L::min_blocks : L::df_
             if constexpr (!MIXED)
             {
                 // double-float pair arithmetic (fmdg_df.cuh)
-                const float4 ih = on ? xi : make_float4(0.f, 0.f, 0.f, 0.f), il = on ? g.xll[t] : ih;
+                const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 ih = on ? g.xr[2 * (size_t)t] : zero, il = on ? g.xr[2 * (size_t)t + 1] : zero;
+                const float3 h3 = make_float3(g.cellh_s[0], g.cellh_s[1], g.cellh_s[2]);
+                const float3 hl3 = make_float3(g.cellh_slo[0], g.cellh_slo[1], g.cellh_slo[2]);
                 const dfl inv_h = df_of(g.inv_h_df);
                 const float kmax = (float)(nint - 1);
-                auto pair = [&](int js, float4 xjf, float4 o) {
-                    if (group >= 0 && g.gslot[js] != group) return;
-                    const int pidx = ki * nk + __float_as_int(xjf.w);
+                // (LEAN: the rows' w is not the kind)
+                auto pair = [&](int js, float w, auto &&geom) {
+                    if (!LEAN && group >= 0 && g.gslot[js] != group) return;
+                    const int pidx = LEAN ? 0 : ki * nk + __float_as_int(w);
                     const fmdg_pair_t &pp = sp.pairs[pidx];
                     if (HYBRID && pp.cat != FMDG_POT_EAM) return;
-                    const GeomDF p = skin_geom_df(g, so, t, ih, il, js, xjf, o);
+                    const GeomDF p = geom();
                     if (within_cut_df_mi(g, t, js, p.r2, sp.pf[pidx][2], pp.p[2]))
                         acc_rho = df_add(acc_rho, df_rho(g, pp, p, inv_h, kmax, nint));
                 };
                 const int cnt = on ? g.nbr_count[t] : 0;
                 const int m_in = prune_share(g, so, cnt <= g.maxnb ? cnt : 0, t, v, V, ih);
                 if (on) g.nbc_count[(size_t)t * V + v] = m_in;
-                for_each_pruned(g, so, m_in, t, v, V, pair);
-                if (cnt > g.maxnb && v == 0) for_each_slot_overflow(g, S, so, t, i, xi, pair);
+                for_each_pruned(g, so, m_in, t, v, V, [&](int js, float4 jh, float4 jl, unsigned w) {
+                    pair(js, jh.w, [&]() { return skin_geom_df(ih, il, jh, jl, w, h3, hl3); });
+                });
+                if (cnt > g.maxnb && v == 0)
+                    for_each_slot_overflow(g, S, so, t, i, xi, [&](int js, float4 xj, float4) {
+                        pair(js, xj.w, [&]() { return geom_df_of64(geom64_mi(g, g.xd[t], g.xd[js])); });
+                    });
             }
             else if (!on)
                 ;
@@ -913,6 +930,18 @@ __global__ void __launch_bounds__(L::max_threads, MIXED ? L::min_blocks : L::df_
             if (M > 1) part_tree(part, M, 1, dens);
     }
     step_trigger();
+    // binary64 mode: F'(rho) as a double-float, in the w of the slot's row
+    // where the rows need no kind (as below in binary32)
+    auto store_fp = [&](int t, float2 fp) {
+        if (LEAN)
+        {
+            float *w = reinterpret_cast<float *>(g.xr + 2 * (size_t)t);
+            w[3] = fp.x;
+            w[7] = fp.y;
+        }
+        else
+            g.fpdf[t] = fp;
+    };
     // embedding, one thread per slot
     const double rho = group_value(dens[0], gl);
     const int t = slot_of_thread(g, bx, gl);
@@ -955,15 +984,15 @@ __global__ void __launch_bounds__(L::max_threads, MIXED ? L::min_blocks : L::df_
             }
             g.vaream[i] = fp;
             g.fpd[t] = fp;
-            if (!MIXED) g.fpdf[t] = df_split(fp);
+            if (!MIXED) store_fp(t, df_split(fp));
         }
         else
         {
             g.vaream[i] = 0.0;
             g.fpd[t] = 0.0;
             g.fpb[t] = 0.f;
-            if (LEAN) reinterpret_cast<float *>(g.xl + t)[3] = 0.f;
-            if (!MIXED) g.fpdf[t] = make_float2(0.f, 0.f);
+            if (MIXED && LEAN) reinterpret_cast<float *>(g.xl + t)[3] = 0.f;
+            if (!MIXED) store_fp(t, make_float2(0.f, 0.f));
         }
     }
     if (rec == REC_FULL && loc_thermo(loc, g)) block_reduce_store<1>(acc, g.partials + (size_t)nb * 8 + bx, blockDim.x >> gl);
@@ -971,9 +1000,10 @@ __global__ void __launch_bounds__(L::max_threads, MIXED ? L::min_blocks : L::df_
 
 // Pair forces + velocity-Verlet finish step (src/integrators.c:94-126) and
 // the thermo record, 2^lane_log lanes per slot (shares and lanes, above);
-// the forces are stored in the current order for the next start step.  LEAN (binary32, one kind, no
-// group): pair parameters in registers, no per-entry kind or group
-// lookups, hardware exp2 / rsqrt / rcp approximations.
+// the forces are stored in the current order for the next start step.  LEAN
+// (one kind, no group; the density pass of the same step ran LEAN too): pair
+// parameters in registers, no per-entry kind or group lookups; in binary32
+// hardware exp2 / rsqrt / rcp approximations.
 template <class L, int CAT, bool MIXED, bool LEAN>
 __global__ void __launch_bounds__(L::max_threads, !MIXED ? L::df_min_blocks : (LEAN ? L::lean_min_blocks : L::min_blocks)) k_force_skin(__grid_constant__ const L loc, int finish, int rec)
 {
@@ -982,7 +1012,7 @@ __global__ void __launch_bounds__(L::max_threads, !MIXED ? L::df_min_blocks : (L
     const int group = g.st.group;
     const double dt = g.st.dt;
     __shared__ SmemPotT<!MIXED, LEAN> sp;
-    __shared__ SkinOffT<!MIXED || !LEAN> so;   // lean binary32 kernels: no remainders (exact on a cubic grid)
+    __shared__ SkinOffT<MIXED && !LEAN> so;   // (lean binary32: no remainders, exact on a cubic grid)
     load_pot<false>(g, sp, skin_params(g));
     load_offsets(g, so);
     step_wait();        // (the tables above were set up before any step)
@@ -1015,21 +1045,25 @@ __global__ void __launch_bounds__(L::max_threads, !MIXED ? L::df_min_blocks : (L
             if constexpr (!MIXED)
             {
                 // double-float pair arithmetic (fmdg_df.cuh, df_pair)
-                const float4 ih = on ? xi : make_float4(0.f, 0.f, 0.f, 0.f), il = on ? g.xll[t] : ih;
-                const dfl fpi = ((CAT == CAT_EAM || CAT == CAT_HYBRID) && on) ? df_of(g.fpdf[t]) : dfl{0.f, 0.f};
+                const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 ih = on ? g.xr[2 * (size_t)t] : zero, il = on ? g.xr[2 * (size_t)t + 1] : zero;
+                const float3 h3 = make_float3(g.cellh_s[0], g.cellh_s[1], g.cellh_s[2]);
+                const float3 hl3 = make_float3(g.cellh_slo[0], g.cellh_slo[1], g.cellh_slo[2]);
+                dfl fpi = {0.f, 0.f};
+                if (LEAN) fpi = {ih.w, il.w};
+                else if ((CAT == CAT_EAM || CAT == CAT_HYBRID) && on) fpi = df_of(g.fpdf[t]);
                 const dfl inv_h = df_of(g.inv_h_df);
                 const float kmax = (float)(nint - 1);
-                auto pair = [&](auto with_e, int js, float4 xjf, float4 o) {
-                    if (group >= 0 && g.gslot[js] != group) return;
-                    const int pidx = ki * nk + __float_as_int(xjf.w);
+                auto pair = [&](auto with_e, int js, float w, auto &&geom, auto &&fpj) {
+                    if (!LEAN && group >= 0 && g.gslot[js] != group) return;
+                    const int pidx = LEAN ? 0 : ki * nk + __float_as_int(w);
                     const fmdg_pair_t &pp = sp.pairs[pidx];
                     const int cat = (CAT == CAT_HYBRID) ? pp.cat : CAT;
                     const int rci = (cat == FMDG_POT_MORSE) ? 3 : 2;
-                    const GeomDF p = skin_geom_df(g, so, t, ih, il, js, xjf, o);
+                    const GeomDF p = geom();
                     if (!within_cut_df_mi(g, t, js, p.r2, sp.pf[pidx][rci], pp.p[rci])) return;
                     dfl fa, eh;
-                    df_pair(g, sp, pidx, pp, cat, p, fpi, inv_h, kmax, nint, ne, [&]() { return df_of(g.fpdf[js]); },
-                            fa, eh);
+                    df_pair(g, sp, pidx, pp, cat, p, fpi, inv_h, kmax, nint, ne, fpj, fa, eh);
                     for (int d = 0; d < 3; d++) sum[d] = df_add(sum[d], df_mul(fa, p.rv[d]));
                     if constexpr (decltype(with_e)::value)
                     {
@@ -1037,15 +1071,26 @@ __global__ void __launch_bounds__(L::max_threads, !MIXED ? L::df_min_blocks : (L
                         sum[4] = df_add(sum[4], df_mul(fa, p.r2));     // rv . (fa rv), both sides of the pair
                     }
                 };
-                auto pair_e = [&](int js, float4 xjf, float4 o) { pair(std::true_type{}, js, xjf, o); };
+                // F'(rho_j): in the row, or (kinds in the rows, overflow) in a table
+                auto listed = [&](auto with_e) {
+                    return [&, with_e](int js, float4 jh, float4 jl, unsigned w) {
+                        pair(with_e, js, jh.w, [&]() { return skin_geom_df(ih, il, jh, jl, w, h3, hl3); },
+                             [&]() { return LEAN ? dfl{jh.w, jl.w} : df_of(g.fpdf[js]); });
+                    };
+                };
                 const int cnt = on ? g.nbr_count[t] : 0;
                 const int m_in = (CAT == CAT_EAM) ? (on ? g.nbc_count[(size_t)t * V + v] : 0)
                                                   : prune_share(g, so, cnt <= g.maxnb ? cnt : 0, t, v, V, ih);
-                if (thermo) for_each_pruned(g, so, m_in, t, v, V, pair_e);
-                else
-                    for_each_pruned(g, so, m_in, t, v, V,
-                                    [&](int js, float4 xjf, float4 o) { pair(std::false_type{}, js, xjf, o); });
-                if (cnt > g.maxnb && v == 0) for_each_slot_overflow(g, S, so, t, i, xi, pair_e);
+                if (thermo) for_each_pruned(g, so, m_in, t, v, V, listed(std::true_type{}));
+                else for_each_pruned(g, so, m_in, t, v, V, listed(std::false_type{}));
+                if (cnt > g.maxnb && v == 0)
+                    for_each_slot_overflow(g, S, so, t, i, xi, [&](int js, float4 xj, float4) {
+                        pair(std::true_type{}, js, xj.w, [&]() { return geom_df_of64(geom64_mi(g, g.xd[t], g.xd[js])); },
+                             [&]() {
+                                 const float4 *r = g.xr + 2 * (size_t)js;
+                                 return LEAN ? dfl{r[0].w, r[1].w} : df_of(g.fpdf[js]);
+                             });
+                    });
             }
             else if (!on)
                 ;
@@ -1396,11 +1441,11 @@ void launch_force_skin(const L &loc, int cats, int finish, int rec, int nb, int 
     const size_t sh = stage_bytes(loc, blk, 5);
     const int ncat = __builtin_popcount(cats);
     if (ncat > 1) fmdg_launch(k_force_skin<L, CAT_HYBRID, MIXED, false>, nb, blk, sh, st, overlap, 1, loc, finish, rec);
-    else if (MIXED && lean)
+    else if (lean)
     {
-        if (cats == (1 << FMDG_POT_LJ)) fmdg_launch(k_force_skin<L, CAT_LJ, true, true>, nb, blk, sh, st, overlap, 1, loc, finish, rec);
-        else if (cats == (1 << FMDG_POT_MORSE)) fmdg_launch(k_force_skin<L, CAT_MORSE, true, true>, nb, blk, sh, st, overlap, 1, loc, finish, rec);
-        else fmdg_launch(k_force_skin<L, CAT_EAM, true, true>, nb, blk, sh, st, overlap, 1, loc, finish, rec);
+        if (cats == (1 << FMDG_POT_LJ)) fmdg_launch(k_force_skin<L, CAT_LJ, MIXED, true>, nb, blk, sh, st, overlap, 1, loc, finish, rec);
+        else if (cats == (1 << FMDG_POT_MORSE)) fmdg_launch(k_force_skin<L, CAT_MORSE, MIXED, true>, nb, blk, sh, st, overlap, 1, loc, finish, rec);
+        else fmdg_launch(k_force_skin<L, CAT_EAM, MIXED, true>, nb, blk, sh, st, overlap, 1, loc, finish, rec);
     }
     else if (cats == (1 << FMDG_POT_LJ)) fmdg_launch(k_force_skin<L, CAT_LJ, MIXED, false>, nb, blk, sh, st, overlap, 1, loc, finish, rec);
     else if (cats == (1 << FMDG_POT_MORSE)) fmdg_launch(k_force_skin<L, CAT_MORSE, MIXED, false>, nb, blk, sh, st, overlap, 1, loc, finish, rec);
@@ -1420,6 +1465,7 @@ void launch_density_skin(const L &loc, bool mixed, bool hyb, int rec, int nb, in
     else
     {
         if (hyb) fmdg_launch(k_density_skin<L, false, true, false>, nb, blk, sh, st, overlap, 1, loc, rec);
+        else if (lean) fmdg_launch(k_density_skin<L, false, false, true>, nb, blk, sh, st, overlap, 1, loc, rec);
         else fmdg_launch(k_density_skin<L, false, false, false>, nb, blk, sh, st, overlap, 1, loc, rec);
     }
 }
@@ -1458,10 +1504,10 @@ int fmdg_pack_launch_forces(const fmdg_pack_launch &P, int phases)
         {
             const LocPackShares L{P.lf};
             if (P.mixed) launch_force_skin<LocPackShares, true>(L, P.cats, 1, REC_FULL, nfb, P.fblk, st, P.lean != 0, P.overlap);
-            else launch_force_skin<LocPackShares, false>(L, P.cats, 1, REC_FULL, nfb, P.fblk, st, false, P.overlap);
+            else launch_force_skin<LocPackShares, false>(L, P.cats, 1, REC_FULL, nfb, P.fblk, st, P.lean != 0, P.overlap);
         }
         else if (P.mixed) launch_force_skin<LocPack, true>(P.lf, P.cats, 1, REC_FULL, nfb, P.fblk, st, P.lean != 0, P.overlap);
-        else launch_force_skin<LocPack, false>(P.lf, P.cats, 1, REC_FULL, nfb, P.fblk, st, false, P.overlap);
+        else launch_force_skin<LocPack, false>(P.lf, P.cats, 1, REC_FULL, nfb, P.fblk, st, P.lean != 0, P.overlap);
         n++;
     }
     cudaError_t e = cudaGetLastError();
@@ -1522,7 +1568,7 @@ int fmdg_skin_launch_pair_forces(fmdg_sys_t *s, int finish)
     const int nb = fmdg_force_blocks(s);
     if (s->g.prec == FMDG_PREC_MIXED)
         launch_force_skin<LocOne, true>(L, s->cats, finish, s->rec, nb, s->fblk, s->stream, lean_system(s), s->overlap);
-    else launch_force_skin<LocOne, false>(L, s->cats, finish, s->rec, nb, s->fblk, s->stream, false, s->overlap);
+    else launch_force_skin<LocOne, false>(L, s->cats, finish, s->rec, nb, s->fblk, s->stream, lean_system(s), s->overlap);
     s->launches++;
     FMDG_CK(cudaGetLastError());
     return FMDG_OK;
