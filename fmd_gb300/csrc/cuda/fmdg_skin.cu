@@ -552,37 +552,48 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_nlist_skin(__
             const float4 xi = g.xf4[i];
             const float rl2 = g.rskin2;
             int4 *row = reinterpret_cast<int4 *>(g.nbr) + t;
-            // hits shift through a four-entry register buffer (in order:
-            // x oldest); every fourth hit writes one 16-byte row; the
-            // buffer update is branch-free (a warp's lanes hit at different
-            // candidates).  The self test is only in the atom's own cell;
-            // the radius is widened by 1e-5 relative so the folded rounding
-            // of the cell offsets can only add entries.
-            int4 buf = make_int4(0, 0, 0, 0);
+            // Up to 32 candidates of a cell give a mask of hits first, then
+            // the hits are taken from the mask: a lane hits at 8 % of its
+            // candidates but some lane of the warp at nearly all, so a
+            // candidate costs what every lane runs for it, and the test
+            // alone is 11 instructions where test and entry were 25 (512k
+            // atoms, 8 A cutoff: 1020 us a build before, 850 now; 256k EAM 337
+            // and 246; 600 jobs of 600 to 3000 atoms 785 and 740 us a step).
+            // Entries shift through a four-entry register buffer (in order:
+            // x oldest); every fourth writes one 16-byte row.  The radius is
+            // widened by 1e-5 relative so the folded rounding of the cell
+            // offsets can only add entries.
             const float rb2 = rl2 * 1.00001f;
-            auto take = [&](int j, int code, float ax, float ay, float az) {
-                const float4 xj = __ldg(g.xf4 + j);
-                const float dx = ax - xj.x, dy = ay - xj.y, dz = az - xj.z;
-                const bool hit = dx * dx + dy * dy + dz * dz < rb2;
-                const int sj = L::renumbered ? j : (hit ? S.slot[j] : 0);
-                const int e = (int)((unsigned)sj | ((unsigned)code << SLOT_BITS));
-                buf.x = hit ? buf.y : buf.x;
-                buf.y = hit ? buf.z : buf.y;
-                buf.z = hit ? buf.w : buf.z;
-                buf.w = hit ? e : buf.w;
-                cnt += hit;
-                if (hit && (cnt & 3) == 0 && cnt <= maxnb) row[(size_t)((cnt >> 2) - 1) * cap] = buf;
-            };
+            int4 buf = make_int4(0, 0, 0, 0);
             const int center = home_code(g);
             for_each_build_cell(g, so, cell_xyz(g, S.cell_of[i]), xi, [&](int code, int c, float ax, float ay, float az) {
                 const int jb = S.cell_start[c], je = S.cell_start[c + 1];
-                if (code == center)
+                auto near = [&](int j) {
+                    const float4 xj = __ldg(g.xf4 + j);
+                    return norm2(make_float3(ax - xj.x, ay - xj.y, az - xj.z)) < rb2;
+                };
+                for (int j0 = jb; j0 < je; j0 += 32)
                 {
-                    for (int j = jb; j < i; j++) take(j, code, ax, ay, az);
-                    for (int j = i + 1; j < je; j++) take(j, code, ax, ay, az);
+                    const int n = min(je - j0, 32);
+                    unsigned m = 0;
+                    int k = 0;
+                    for (; k + 4 <= n; k += 4)
+                    {
+                        const bool h0 = near(j0 + k), h1 = near(j0 + k + 1), h2 = near(j0 + k + 2), h3 = near(j0 + k + 3);
+                        m |= ((h0 ? 1u : 0u) | (h1 ? 2u : 0u) | (h2 ? 4u : 0u) | (h3 ? 8u : 0u)) << k;
+                    }
+                    for (; k < n; k++) m |= near(j0 + k) ? 1u << k : 0u;
+                    // (not the atom itself, in its own cell)
+                    if (code == center && (unsigned)(i - j0) < 32u) m &= ~(1u << (i - j0));
+                    for (; m; m &= m - 1)
+                    {
+                        const int j = j0 + __ffs(m) - 1;
+                        const int sj = L::renumbered ? j : S.slot[j];
+                        buf = make_int4(buf.y, buf.z, buf.w, (int)((unsigned)sj | ((unsigned)code << SLOT_BITS)));
+                        cnt++;
+                        if ((cnt & 3) == 0 && cnt <= maxnb) row[(size_t)((cnt >> 2) - 1) * cap] = buf;
+                    }
                 }
-                else
-                    for (int j = jb; j < je; j++) take(j, code, ax, ay, az);
             });
             const int rem = cnt & 3;
             if (rem && cnt <= maxnb)
