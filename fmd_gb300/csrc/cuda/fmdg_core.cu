@@ -1,7 +1,7 @@
 // Device engine: system lifetime, uploads/downloads, step orchestration.
 //
 // A system owns one CUDA stream.  fmdg_vv_steps captures one
-// velocity-Verlet step (refresh + forces + reductions, ~9 kernels) into a
+// velocity-Verlet step (refresh, list, EAM density, forces: 3 to 8 kernels) into a
 // CUDA graph on first use and replays it once per step, so the host issues
 // one graph launch per step and never waits inside the loop; it synchronises
 // only when the caller reads results (thermo, errors, atoms).

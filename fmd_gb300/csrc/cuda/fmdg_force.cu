@@ -18,7 +18,8 @@
 // atom's energy takes half of each pair term.
 //
 // Per step, after the refresh:
-//   k_prep_local  cell-local binary32 coordinates of every atom (float4)
+//   (the refresh has written the cell-local binary32 coordinates of every
+//   atom; k_prep_local does where no refresh comes before)
 //   k_nlist       27-cell stencil scan in binary32 against the largest
 //                 cutoff plus a margin; stores (j, stencil offset) per atom
 //   k_density     EAM pass 1 + embedding over the list
@@ -26,8 +27,8 @@
 // An atom with more candidates than the list holds falls back to scanning
 // the stencil directly, so the list size is a performance knob only.
 // These kernels serve single systems on the exact per-step list (binary64
-// by default, and boxes too small for a skin list); packed systems and
-// mixed-precision single systems use the skin-list kernels (fmdg_skin.cu).
+// systems of several kinds, boxes too small for a skin list, a skin of
+// zero); the others use the skin-list kernels (fmdg_skin.cu).
 //
 // Precision modes.  FMDG_PREC_FP64: every pair quantity to binary64
 // accuracy, the binary32 list only prunes (its margin keeps every pair

@@ -25,9 +25,10 @@
 //    a small autotuner: the first chunks of each pack try 64, 128 and 256
 //    threads and keep the one with the lowest device time per atom-step.
 //
-// Each member's arithmetic is the single-system arithmetic (one thread per
-// atom, fixed list order), so an atom's trajectory does not depend on the
-// other members of its pack nor on the tuned block size; only the block
+// Each member's arithmetic is its own (fixed list order, shares of the list
+// walks by its size and summed in a fixed tree), so an atom's trajectory does
+// not depend on the other members of its pack, the lanes a pack gives a slot
+// or the tuned block size; only the block
 // partial sums of the thermo record are grouped differently.
 #include "fmdg_internal.cuh"
 

@@ -1,5 +1,5 @@
 // Pair kernels over a Verlet-skin neighbour list: packed (served) systems,
-// and single systems in mixed precision whose box allows it.
+// and single systems whose box allows it (in binary64 those of one kind).
 //
 // Systems on the per-step path rebuild their list every step in the
 // current (reference cell) order.  Skin-list systems keep a list of radius
@@ -17,14 +17,14 @@
 // Packed step:
 //   k_skin_start    velocity-Verlet start step, per-step slot positions,
 //                   displacement test -> rebuild flag
-//   (rebuild steps only) reference-order cell refresh (fmdg_bin.cu),
-//   k_prep_skin     slot tables (renumbered), k_nlist_skin stencil scan of
-//                   the cells within the list radius
-//   k_density_skin  EAM pass 1 + embedding, one thread per slot
+//   (rebuild steps only) k_refresh_cluster (fmdg_bin.cu): reference-order
+//                   cell refresh and slot tables (renumbered);
+//   k_nlist_skin    stencil scan of the cells within the list radius
+//   k_density_skin  EAM pass 1 + embedding
 //   k_force_skin    pair forces + velocity-Verlet finish step + thermo
-//                   record, one thread per slot
-// Single-system step: the reference-order refresh every step, then
-// k_prep_skin (stable slots), k_nlist_skin (when flagged), density, forces.
+//                   record; 2^lane_log lanes per slot in both
+// Single-system step: the reference-order refresh with the slot tables
+// (stable slots) every step, k_nlist_skin (when flagged), density, forces.
 //
 // Geometry.  An atom's binary32 position is kept relative to the cell it
 // had at the last build (unwrapped across periodic faces: it moves less
@@ -466,7 +466,7 @@ __global__ void k_skin_start(__grid_constant__ const L loc)
     slot_rel_build(g, dyn, t, x, __int_as_float(kind));
 }
 
-// The per-atom tables of the current positions (prep_atom), one thread per
+// The per-atom tables of the current positions (prep_skin_atom), one thread per
 // atom, for a force evaluation without a refresh before it
 __global__ void __launch_bounds__(128) k_prep_skin(__grid_constant__ const LocOne loc)
 {
@@ -1138,8 +1138,9 @@ __global__ void __launch_bounds__(L::max_threads, !MIXED ? L::df_min_blocks : (L
                     else
                     {
                         const float inv_r = rsqrt_approx(r2);
-                        const float r = __fmul_rn(r2, inv_r);
-                        const float e1 = ex2_approx(__fmul_rn(__fsub_rn(pq.z, r), m_c1));
+                        // (r0 - r in one rounding: a rounded r would cost
+                        // up to 3e-7 of the exponential)
+                        const float e1 = ex2_approx(__fmul_rn(__fmaf_rn(-r2, inv_r, pq.z), m_c1));
                         fa = __fmul_rn(__fmul_rn(m_c2, inv_r), __fmaf_rn(e1, e1, -e1));
                         e = 0.5f * (pq.x * (e1 * e1 - 2.f * e1));
                     }
