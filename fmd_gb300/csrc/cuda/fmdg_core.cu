@@ -629,7 +629,11 @@ int fmdg_list_capacity(const fmdg_sys_t *s, const int *cell_count, int ncell)
     }
     const double rlist = sqrt(rc2max) + (s->skin_used > 0.0 ? s->skin_used : 1e-2);
     if (s->list_capacity > 0) return s->list_capacity;
-    return fmdg_capacity_estimate(cell_count, ncell, g.cellh[0] * g.cellh[1] * g.cellh[2], rlist);
+    const int est = fmdg_capacity_estimate(cell_count, ncell, g.cellh[0] * g.cellh[1] * g.cellh[2], rlist);
+    // A single system that grows denser (melting, ablation) outlives its list
+    // by far at twice the entries; below 2 GB of lists that is cheap.
+    const int twice = est < 512 ? 2 * est : 1024;
+    return (!s->served && s->skin_used > 0.0 && (size_t)g.cap * twice * 4 < ((size_t)2 << 30)) ? twice : est;
 }
 
 // Neighbour-list entries per atom (before fmdg_upload); 0: the estimate.

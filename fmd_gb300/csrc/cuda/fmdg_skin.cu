@@ -264,20 +264,31 @@ struct NoRound
 // atom has moved less than skin/2 since, so the stencil still covers the
 // list radius), and of the occurrences of a neighbour (a cell recurs in the
 // stencil when an axis has fewer than 2R + 1 cells) only the image within
-// the list radius is passed on.
-template <typename F, bool DF>
+// the list radius is passed on.  Share v of V takes every V-th candidate.
+// ONE: a single system, whose refresh has just written every atom's binary32
+// position in its current cell (xf4): the same numbers without binary64 work
+// for each of some thousand candidates.  A laser-heated slab of 10 000 atoms
+// whose density outgrew its lists took 26 ms for 25 steps with one lane and
+// binary64 positions, 5 now.
+template <bool ONE, typename F, bool DF>
 __device__ __forceinline__ void for_each_slot_overflow(const Geo &g, const Side &S, const SkinOffT<DF> &so, int t,
-                                                       int i, float4 &xi, F &&f)
+                                                       int i, int v, int V, float4 &xi, F &&f)
 {
     const double4_32a xdi = g.xd[t], oi = g.corig[S.cell_of[i]];
     const double xs = g.xs;
     xi = make_float4((float)((xdi.x - oi.x) * xs), (float)((xdi.y - oi.y) * xs), (float)((xdi.z - oi.z) * xs), xi.w);
     const float lim2 = g.rskin2 * 1.0001f;
+    int turn = 0;
     for_each_candidate(g, S, i, xi, [&](int j, int code) {
+        if ((turn++ & (V - 1)) != v) return;
+        float4 xj = g.xf4[j];
         const int js = S.slot[j];
-        const double4_32a xdj = g.xd[js], oj = g.corig[S.cell_of[j]];
-        const float4 xj = make_float4((float)((xdj.x - oj.x) * xs), (float)((xdj.y - oj.y) * xs),
-                                      (float)((xdj.z - oj.z) * xs), g.xf4[j].w);
+        if (!ONE)
+        {
+            const double4_32a xdj = g.xd[js], oj = g.corig[S.cell_of[j]];
+            xj = make_float4((float)((xdj.x - oj.x) * xs), (float)((xdj.y - oj.y) * xs),
+                             (float)((xdj.z - oj.z) * xs), xj.w);
+        }
         float4 o = so.off[code];
         const float3 d = rv_of(xi, xj, o);
         if (d.x * d.x + d.y * d.y + d.z * d.z > lim2) return;
@@ -291,8 +302,8 @@ __device__ __forceinline__ void for_each_slot_overflow(const Geo &g, const Side 
 // image offset); r(k) after every k entries visited (a round of four, or
 // one).  PF: the next round's list rows are prefetched into L1 while this
 // round is processed (the rows stream from DRAM).
-// An atom whose list overflowed is share 0's alone (for_each_slot_overflow).
-template <bool PF = false, typename F, typename R, bool DF>
+// An atom whose list overflowed: for_each_slot_overflow.
+template <bool ONE, bool PF = false, typename F, typename R, bool DF>
 __device__ __forceinline__ void for_each_slot_pair(const Geo &g, const Side &S, const SkinOffT<DF> &so, int t, int i,
                                                    int v, int V, float4 &xi, F &&f, R &&r)
 {
@@ -329,18 +340,18 @@ __device__ __forceinline__ void for_each_slot_pair(const Geo &g, const Side &S, 
             }
         }
     }
-    else if (v == 0)
-        for_each_slot_overflow(g, S, so, t, i, xi, [&](int js, float4 xj, float4 o) {
+    else
+        for_each_slot_overflow<ONE>(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
             f(js, xj, o);
             r(1);
         });
 }
 
-template <typename F, bool DF>
+template <bool ONE, typename F, bool DF>
 __device__ __forceinline__ void for_each_slot_pair(const Geo &g, const Side &S, const SkinOffT<DF> &so, int t, int i,
                                                    int v, int V, float4 &xi, F &&f)
 {
-    for_each_slot_pair(g, S, so, t, i, v, V, xi, f, NoRound{});
+    for_each_slot_pair<ONE>(g, S, so, t, i, v, V, xi, f, NoRound{});
 }
 
 // The double-float kernels' walk.  Their pair arithmetic costs hundreds of
@@ -832,8 +843,8 @@ __global__ void __launch_bounds__(L::max_threads, MIXED ? L::min_blocks : L::df_
                 for_each_pruned(g, so, m_in, t, v, V, [&](int js, float4 jh, float4 jl, unsigned w) {
                     pair(js, jh.w, [&]() { return skin_geom_df(ih, il, jh, jl, w, h3, hl3); });
                 });
-                if (cnt > g.maxnb && v == 0)
-                    for_each_slot_overflow(g, S, so, t, i, xi, [&](int js, float4 xj, float4) {
+                if (cnt > g.maxnb)
+                    for_each_slot_overflow<L::one_system>(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4) {
                         pair(js, xj.w, [&]() { return geom_df_of64(geom64_mi(g, g.xd[t], g.xd[js])); });
                     });
             }
@@ -900,8 +911,8 @@ __global__ void __launch_bounds__(L::max_threads, MIXED ? L::min_blocks : L::df_
                     }
                     if (k < cnt) round(__ldg(col + (size_t)(k >> 2) * cap), cnt - k, std::true_type{});
                 }
-                else if (v == 0)
-                    for_each_slot_overflow(g, S, so, t, i, xi, [&](int js, float4 xj, float4 o) {
+                else
+                    for_each_slot_overflow<L::one_system>(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
                         const float r2 = norm2(rv_of(xi, xj, o));
                         bool in = r2 < rc2f;
                         if (fabsf(r2 - rc2f) <= band) in = geom64_mi(g, g.xd[t], g.xd[js]).r2 < rc2;
@@ -916,7 +927,7 @@ __global__ void __launch_bounds__(L::max_threads, MIXED ? L::min_blocks : L::df_
                 const float inv_h = g.inv_hi_f;   // (scaled r^2: index only)
                 const float kmax = (float)(nint - 1);
                 Acc32<1> ac;
-                for_each_slot_pair(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
+                for_each_slot_pair<L::one_system>(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
                     if (group >= 0 && g.gslot[js] != group) return;
                     const int pidx = ki * nk + __float_as_int(xj.w);
                     const fmdg_pair_t &pp = sp.pairs[pidx];
@@ -1094,8 +1105,8 @@ __global__ void __launch_bounds__(L::max_threads, !MIXED ? L::df_min_blocks : (L
                                                   : prune_share(g, so, cnt <= g.maxnb ? cnt : 0, t, v, V, ih);
                 if (thermo) for_each_pruned(g, so, m_in, t, v, V, listed(std::true_type{}));
                 else for_each_pruned(g, so, m_in, t, v, V, listed(std::false_type{}));
-                if (cnt > g.maxnb && v == 0)
-                    for_each_slot_overflow(g, S, so, t, i, xi, [&](int js, float4 xj, float4) {
+                if (cnt > g.maxnb)
+                    for_each_slot_overflow<L::one_system>(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4) {
                         pair(std::true_type{}, js, xj.w, [&]() { return geom_df_of64(geom64_mi(g, g.xd[t], g.xd[js])); },
                              [&]() {
                                  const float4 *r = g.xr + 2 * (size_t)js;
@@ -1251,8 +1262,8 @@ __global__ void __launch_bounds__(L::max_threads, !MIXED ? L::df_min_blocks : (L
                         }
                         if (k < cnt) round(__ldg(col + (size_t)(k >> 2) * cap), cnt - k, std::true_type{});
                     }
-                    else if (v == 0)
-                        for_each_slot_overflow(g, S, so, t, i, xi, [&](int js, float4 xj, float4 o) {
+                    else
+                        for_each_slot_overflow<L::one_system>(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
                             const float3 rv = rv_of(xi, xj, o);
                             const float r2 = norm2(rv);
                             bool in = r2 < rc2f;
@@ -1279,7 +1290,7 @@ __global__ void __launch_bounds__(L::max_threads, !MIXED ? L::df_min_blocks : (L
                 const float kmax = (float)(nint - 1);
                 const float xs2 = g.xs2_f;
                 Acc32<5> ac;
-                for_each_slot_pair(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
+                for_each_slot_pair<L::one_system>(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
                     if (group >= 0 && g.gslot[js] != group) return;
                     const int pidx = ki * nk + __float_as_int(xj.w);
                     const fmdg_pair_t &pp = sp.pairs[pidx];
