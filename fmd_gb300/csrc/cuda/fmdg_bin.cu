@@ -148,9 +148,19 @@ __device__ __forceinline__ void classify_atom(const Geo &g, Dyn *dyn, const Side
         g.bdest[i] = -1;
         if (g.skin_on)
         {
-            // the slot is gone: its list entries must go too
-            g.pos[S.slot[i]] = -1;
-            dyn->rebuild = 1;
+            // the slot is gone: out of reach of the lists that hold it (a
+            // position beyond every cutoff, finite in all pair arithmetic)
+            // until the next build leaves it out
+            const int t = S.slot[i];
+            const float far = 1e8f;
+            g.pos[t] = -1;
+            g.xl[t] = make_float4(far, far, far, 0.f);
+            g.xd[t] = make_double4_32a(1e8, 1e8, 1e8, 0.0);
+            if (g.prec == FMDG_PREC_FP64)
+            {
+                g.xr[2 * (size_t)t] = make_float4(far, far, far, 0.f);
+                g.xr[2 * (size_t)t + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
         }
         return;
     }
