@@ -79,7 +79,7 @@ __device__ __forceinline__ void for_each_pair(const Geo &g, const Side &S, int i
         const int *col = g.nbr + i;
         for (int k = 0; k < cnt; k++)
         {
-            const int e = __ldg(col + (size_t)k * cap);
+            const int e = col[(size_t)k * cap];
             f(e & 0x3ffffff, e >> 26);
         }
     }
@@ -206,8 +206,8 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_nlist(__grid_
             // four candidates per round, their loads in flight together
             for (; j + 4 <= je; j += 4)
             {
-                const float4 a0 = __ldg(g.xf4 + j), a1 = __ldg(g.xf4 + j + 1);
-                const float4 a2 = __ldg(g.xf4 + j + 2), a3 = __ldg(g.xf4 + j + 3);
+                const float4 a0 = g.xf4[j], a1 = g.xf4[j + 1];
+                const float4 a2 = g.xf4[j + 2], a3 = g.xf4[j + 3];
                 test(j, a0);
                 test(j + 1, a1);
                 test(j + 2, a2);
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_nlist(__grid_
             }
         }
         for (; j < je; j++)
-            if (j != i) test(j, __ldg(g.xf4 + j));
+            if (j != i) test(j, g.xf4[j]);
     }
     g.nbr_count[i] = cnt;
 }
@@ -252,14 +252,14 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_density(__gri
             {
                 // double-float pair arithmetic (fmdg_df.cuh)
                 float4 ih, il;
-                ld_row32(g.xdf + 2 * (size_t)i, ih, il);
+                ld_slot32(g.xdf + 2 * (size_t)i, ih, il);
                 const dfl inv_h = df_of(g.inv_h_df);
                 const float kmax = (float)(nint - 1);
                 dfl acc_rho = {0.f, 0.f};
                 for_each_pair(g, S, i, ci, [&](int j, int code) {
                     if (group >= 0 && S.group[j] != group) return;
                     float4 jh, jl;
-                    ld_row32(g.xdf + 2 * (size_t)j, jh, jl);
+                    ld_slot32(g.xdf + 2 * (size_t)j, jh, jl);
                     const int pidx = ki * nk + __float_as_int(jh.w);
                     const fmdg_pair_t &pp = sp.pairs[pidx];
                     if (HYBRID && pp.cat != FMDG_POT_EAM) return;
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_force(__grid_
                 // src/morse.h:35-56, EAM src/eam.h:186-226 -- the category
                 // chosen per pair for hybrid tables (src/forces.c:33-290)
                 float4 ih, il;
-                ld_row32(g.xdf + 2 * (size_t)i, ih, il);
+                ld_slot32(g.xdf + 2 * (size_t)i, ih, il);
                 const dfl fpi = (CAT == CAT_EAM || CAT == CAT_HYBRID) ? df_of(g.fpdf[i]) : dfl{0.f, 0.f};
                 const dfl inv_h = df_of(g.inv_h_df);
                 const float kmax = (float)(nint - 1);
@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_force(__grid_
                 for_each_pair(g, S, i, ci, [&](int j, int code) {
                     if (group >= 0 && S.group[j] != group) return;
                     float4 jh, jl;
-                    ld_row32(g.xdf + 2 * (size_t)j, jh, jl);
+                    ld_slot32(g.xdf + 2 * (size_t)j, jh, jl);
                     const int pidx = ki * nk + __float_as_int(jh.w);
                     const fmdg_pair_t &pp = sp.pairs[pidx];
                     const int cat = (CAT == CAT_HYBRID) ? pp.cat : CAT;

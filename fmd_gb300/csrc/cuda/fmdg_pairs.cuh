@@ -35,7 +35,11 @@ struct SmemPotT
 
 // one 32-byte table row (two float4) in a single 256-bit load; p must be
 // 32-byte aligned (the row tables are whole allocations, checked when they
-// are built)
+// are built).  For tables set up before any step only: the read-only path
+// (this, __ldg) is defined for data that nobody writes while the kernel
+// lives, and a step kernel launched with overlap (fmdg_launch) lives from
+// before the kernels ahead of it have finished; step_wait() orders ordinary
+// loads, not these.
 __device__ __forceinline__ void ld_row32(const float4 *p, float4 &a, float4 &b)
 {
     asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -43,7 +47,7 @@ __device__ __forceinline__ void ld_row32(const float4 *p, float4 &a, float4 &b)
         : "l"(p));
 }
 
-// the same of a row that kernels of this step wrote
+// the same of a row that kernels of this step wrote (an ordinary load)
 __device__ __forceinline__ void ld_slot32(const float4 *p, float4 &a, float4 &b)
 {
     asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"

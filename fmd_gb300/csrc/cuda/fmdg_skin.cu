@@ -317,7 +317,7 @@ __device__ __forceinline__ void for_each_slot_pair(const Geo &g, const Side &S, 
         {
             if (PF && k + step + 4 <= cnt)
                 asm volatile("prefetch.global.L1 [%0];" ::"l"(col + (size_t)((k + step) >> 2) * cap));
-            const int4 e4 = __ldg(col + (size_t)(k >> 2) * cap);
+            const int4 e4 = col[(size_t)(k >> 2) * cap];
             const int e0 = e4.x, e1 = e4.y, e2 = e4.z, e3 = e4.w;
             const float4 x0 = g.xl[e0 & SLOT_MASK], x1 = g.xl[e1 & SLOT_MASK];
             const float4 x2 = g.xl[e2 & SLOT_MASK], x3 = g.xl[e3 & SLOT_MASK];
@@ -330,7 +330,7 @@ __device__ __forceinline__ void for_each_slot_pair(const Geo &g, const Side &S, 
         if (k < cnt)
         {
             // the last, partial round (1-3 entries)
-            const int4 e4 = __ldg(col + (size_t)(k >> 2) * cap);
+            const int4 e4 = col[(size_t)(k >> 2) * cap];
             const int ee[3] = {e4.x, e4.y, e4.z};
             for (int q = 0; q < 3 && k + q < cnt; q++)
             {
@@ -375,7 +375,7 @@ __device__ __forceinline__ int prune_share(const Geo &g, const SkinOffT<false> &
     int m = 0;
     for (int k = 4 * v; k < cnt; k += 4 * V)
     {
-        const int4 e4 = __ldg(col + (size_t)(k >> 2) * cap);
+        const int4 e4 = col[(size_t)(k >> 2) * cap];
         const int left = cnt - k;
         // (the words behind a list's last entry are not defined)
         const unsigned e[4] = {(unsigned)e4.x, left > 1 ? (unsigned)e4.y : (unsigned)e4.x,
@@ -580,7 +580,7 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_nlist_skin(__
             for_each_build_cell(g, so, cell_xyz(g, S.cell_of[i]), xi, [&](int code, int c, float ax, float ay, float az) {
                 const int jb = S.cell_start[c], je = S.cell_start[c + 1];
                 auto near = [&](int j) {
-                    const float4 xj = __ldg(g.xf4 + j);
+                    const float4 xj = g.xf4[j];
                     return norm2(make_float3(ax - xj.x, ay - xj.y, az - xj.z)) < rb2;
                 };
                 for (int j0 = jb; j0 < je; j0 += 32)
@@ -654,7 +654,7 @@ __device__ __forceinline__ void build_slot_grouped(const Geo &g, const Side &S, 
                 bool hit = false;
                 if (j < je && !(self && j == i))
                 {
-                    const float4 xj = __ldg(g.xf4 + j);
+                    const float4 xj = g.xf4[j];
                     const float dx = ax - xj.x, dy = ay - xj.y, dz = az - xj.z;
                     hit = dx * dx + dy * dy + dz * dz < rb2;
                 }
@@ -907,9 +907,9 @@ __global__ void __launch_bounds__(L::max_threads, MIXED ? L::min_blocks : L::df_
                     {
                         if (k + step + 4 <= cnt)
                             asm volatile("prefetch.global.L1 [%0];" ::"l"(col + (size_t)((k + step) >> 2) * cap));
-                        round(__ldg(col + (size_t)(k >> 2) * cap), 4, std::false_type{});
+                        round(col[(size_t)(k >> 2) * cap], 4, std::false_type{});
                     }
-                    if (k < cnt) round(__ldg(col + (size_t)(k >> 2) * cap), cnt - k, std::true_type{});
+                    if (k < cnt) round(col[(size_t)(k >> 2) * cap], cnt - k, std::true_type{});
                 }
                 else
                     for_each_slot_overflow<L::one_system>(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
@@ -1258,9 +1258,9 @@ __global__ void __launch_bounds__(L::max_threads, !MIXED ? L::df_min_blocks : (L
                         {
                             if (PF && k + step + 4 <= cnt)
                                 asm volatile("prefetch.global.L1 [%0];" ::"l"(col + (size_t)((k + step) >> 2) * cap));
-                            round(__ldg(col + (size_t)(k >> 2) * cap), 4, std::false_type{});
+                            round(col[(size_t)(k >> 2) * cap], 4, std::false_type{});
                         }
-                        if (k < cnt) round(__ldg(col + (size_t)(k >> 2) * cap), cnt - k, std::true_type{});
+                        if (k < cnt) round(col[(size_t)(k >> 2) * cap], cnt - k, std::true_type{});
                     }
                     else
                         for_each_slot_overflow<L::one_system>(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
