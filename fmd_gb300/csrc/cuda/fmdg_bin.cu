@@ -38,6 +38,7 @@
 // launches and their gaps were most of a small system's step.
 #include <cooperative_groups.h>
 
+#include "fmdg_perdev.h"
 #include "fmdg_prep.cuh"
 
 namespace cg = cooperative_groups;
@@ -624,11 +625,18 @@ int refresh_threads(int n, int blocks)
     return t < 64 ? 64 : (t > 512 ? 512 : t);
 }
 
-// A single system takes sixteen, where the device has room for such a
-// cluster: 4000 atoms refresh in 11.6 us against 14.0 with eight.
-int single_refresh_blocks()
+// A single system takes sixteen, where its device has room for such a
+// cluster: 4000 atoms refresh in 11.6 us against 14.0 with eight.  Both the
+// permission for a cluster of more than eight and the answer belong to the
+// device.
+int single_refresh_blocks(const fmdg_sys_t *s)
 {
-    static const int blocks = [] {
+    static PerDevice kept;
+    if (s->refresh_blocks) return s->refresh_blocks;
+    return kept.get(s->device, [s] {
+        int current = s->device;
+        cudaGetDevice(&current);
+        if (current != s->device) cudaSetDevice(s->device);
         const auto kernel = k_refresh_cluster<LocOne>;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(16);
@@ -639,16 +647,16 @@ int single_refresh_blocks()
         at.val.clusterDim.y = at.val.clusterDim.z = 1;
         cfg.attrs = &at;
         cfg.numAttrs = 1;
-        int room = 0;
+        int room = 0, blocks = 16;
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
             cudaOccupancyMaxActiveClusters(&room, kernel, &cfg) != cudaSuccess || room < 1)
         {
             cudaGetLastError();
-            return REFRESH_BLOCKS;
+            blocks = REFRESH_BLOCKS;
         }
-        return 16;
-    }();
-    return blocks;
+        if (current != s->device) cudaSetDevice(current);
+        return blocks;
+    });
 }
 
 } // namespace
@@ -666,7 +674,7 @@ int fmdg_launch_refresh(fmdg_sys_t *s, int mode, double dt, int group, int therm
     const LocOne L{g};
     if (g.cap <= CLUSTER_ATOMS)
     {
-        const int nb = single_refresh_blocks();
+        const int nb = single_refresh_blocks(s);
         FMDG_CK(fmdg_launch(k_refresh_cluster<LocOne>, nb, refresh_threads(g.cap, nb), 0, st, s->overlap, nb, L, mode));
         s->launches++;
         return FMDG_OK;

@@ -645,6 +645,14 @@ extern "C" int fmdg_set_build_lanes(fmdg_sys_t *s, int lanes)
     return FMDG_OK;
 }
 
+extern "C" int fmdg_set_refresh_blocks(fmdg_sys_t *s, int blocks)
+{
+    if (blocks != 0 && blocks != 8) return fmdg_set_error("fmdg_set_refresh_blocks: 0 or 8");
+    s->refresh_blocks = blocks;
+    invalidate_graph(s);
+    return FMDG_OK;
+}
+
 extern "C" int fmdg_set_list_capacity(fmdg_sys_t *s, int entries)
 {
     if (entries < 0 || entries > 1024 || (entries % 8) != 0)

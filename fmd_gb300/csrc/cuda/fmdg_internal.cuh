@@ -212,6 +212,7 @@ struct fmdg_sys
     bool skin_set;                // skin chosen by the caller (any precision)
     int list_capacity;            // neighbour-list entries per atom; 0: estimated at upload
     int build_lanes;              // threads per atom of a skin-list build; 0: by size
+    int refresh_blocks;           // blocks of a small system's refresh; 0: what the device has room for
     double rsk;                   // skin-list radius (largest cutoff + skin), real units
     double skin;                  // Verlet skin asked for (A), 0: exact per-step list
     double skin_used;             // the skin of the list in use, 0: exact per-step list

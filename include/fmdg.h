@@ -122,6 +122,10 @@ int fmdg_set_list_capacity(fmdg_sys_t *s, int entries);
    16 or 32 fix them.
    Every choice builds the same list, entry for entry. */
 int fmdg_set_build_lanes(fmdg_sys_t *s, int lanes);
+/* Blocks of the refresh of this system where one cluster does it (up to 8192
+   atoms): 0 (default) takes sixteen where the device has room for them, else
+   eight; 8 fixes eight.  Every choice gives the same bits. */
+int fmdg_set_refresh_blocks(fmdg_sys_t *s, int blocks);
 
 /* --- atoms (replaces the distribution of the global grid to the local grid,
        src/matter.c:329-447, and the state gathers of src/misc.c:310-422) -- */
