@@ -287,7 +287,14 @@ __device__ double spline_adv(const double *xs, const double *ys, const double *d
     return a * ys[klo] + b * ys[khi] + ((a * a * a - a) * dd[klo] + (b * b * b - b) * dd[khi]) * (h * h) / 6.0;
 }
 
-// 1/x to a few ulps for positive normal x: the hardware approximation (PTX
+// x < 0 (false for -0 and NaN) by one integer comparison: those of binary64
+// numbers issue at the binary64 rate
+__device__ __forceinline__ bool below_zero(double x)
+{
+    return (unsigned long long)__double_as_longlong(x) - 0x8000000000000001ull < 0x7ff0000000000000ull;
+}
+
+// 1/x to a few ulps for normal x: the hardware approximation (PTX
 // rcp.approx.ftz.f64, about 2^-20; no conversion to binary32 and back, which
 // would issue at the binary64 rate) refined by two Newton-Raphson steps
 // r <- r + r (1 - x r), each of which squares the relative error (2^-20 ->
@@ -431,38 +438,46 @@ __global__ void k_ttm_solve(Geo g, DTuri t, double dt, int staged)
         a.srcz[i] = calc_source ? exp(p.laser_m_absdepth_inv * (z - p.frontsurf)) : 0.0;
     }
     __syncthreads();
-    // Type 1 with a thread per cell (every staged grid up to 1024 cells): the
-    // cell's state in registers, the neighbours that take part found once
-    // (activity does not change between substeps; a comparison of binary64
-    // numbers issues at the binary64 rate), one store and one barrier per
+    // Type 1 with a thread per cell (every staged grid: staging ends near 700
+    // cells): the cell's state in registers, one store and one barrier per
     // substep.  A substep is a chain of dependent binary64 operations; a
-    // launch of 100 substeps on the 50-cell grid 104 -> 62 us.
+    // launch of 100 substeps on the 50-cell grid 104 -> 62 us.  Which cells
+    // take part is asked in every substep, by integers: a cell that an
+    // overshooting substep took below zero stands still, and the swap of the
+    // buffers (te and other here) gives it back its value of the substep
+    // before, as in the loop below.
     const bool own = staged && p.type == 1 && hi - lo <= (int)blockDim.x;
     if (own)
     {
-        const int i = lo + threadIdx.x;
-        const bool mine = i < hi && Te[i] >= 0.0;
-        double te = 0.0, ti = 0.0, xi = 0.0, sz = 0.0;
-        int ilo = 0, ihi = 0;
+        const int i = lo + threadIdx.x, im1 = (i == lo) ? 0 : i - 1;
+        const bool mine = i < hi;
+        double te = 0.0, other = 0.0, ti = 0.0, xi = 0.0, sz = 0.0;
         if (mine)
         {
-            const int im1 = (i == lo) ? 0 : i - 1;
             te = Te[i];
+            other = Te2[i];
             ti = a.Ti[i];
             sz = a.srcz[i];
-            ilo = (Te[im1] < 0) ? i : im1;
-            ihi = (Te[i + 1] < 0) ? i : i + 1;
         }
         for (int j = 0; j < p.ratio; j++)
         {
-            if (mine)
+            if (mine && below_zero(te))
             {
+                const double t2 = other;
+                other = te;
+                te = t2;
+            }
+            else if (mine)
+            {
+                const double tl = Te[im1], th = Te[i + 1];
+                const double tlo = below_zero(tl) ? te : tl, thi = below_zero(th) ? te : th;
                 // dte / (C_gamma te) * (K lap / dz2 - G (te - Ti) + source)
                 // with the constant quotients formed once per launch and one
                 // reciprocal instead of two IEEE divisions
                 const double q = dte_C * recip_newton(te);
                 const double source = calc_source ? a.spc[j] * sz : 0.0;
-                te = te + q * (K_dz2 * (Te[ihi] - 2 * te + Te[ilo]) - p.G * (te - ti) + source);
+                other = te;
+                te = te + q * (K_dz2 * (thi - 2 * te + tlo) - p.G * (te - ti) + source);
                 Te2[i] = te;
                 xi += te;
             }
