@@ -336,13 +336,16 @@ __host__ __device__ inline size_t ttm_stage_bytes(int nz, int ratio)
     return (size_t)nz * (8 * sizeof(double) + sizeof(unsigned)) + (size_t)ratio * sizeof(double);
 }
 
+// largest block of the electron solver (a thread per cell up to it)
+constexpr int TTM_THREADS = 1024;
+
 // One thread block: cell activation, timestep_ratio FTCS substeps of the
 // electron temperature with Neumann reflection at inactive neighbours,
 // time-averaged Te and the friction coefficient xi.  staged: the cell
 // arrays live in shared memory for the launch (the substeps are a chain of
 // dependent reads of neighbouring cells), and the laser's time factor of
 // every substep is formed up front, in parallel.
-__global__ void k_ttm_solve(Geo g, DTuri t, double dt, int staged)
+__global__ void __launch_bounds__(TTM_THREADS) k_ttm_solve(Geo g, DTuri t, double dt, int staged)
 {
     extern __shared__ double sm[];
     Dyn *dyn = g.dyn;
@@ -638,7 +641,7 @@ int fmdg_launch_ttm_solve(fmdg_sys_t *s, int k, double dt, cudaStream_t st)
     const size_t bytes = ttm_stage_bytes(t.dims[2], t.p.ratio);
     const int staged = bytes <= 48 * 1024;
     // a thread per cell where a block can (fewer idle warps at its barriers)
-    const int threads = std::min(1024, std::max(64, (t.itc_hi - t.itc_lo + 31) / 32 * 32));
+    const int threads = std::min(TTM_THREADS, std::max(64, (t.itc_hi - t.itc_lo + 31) / 32 * 32));
     k_ttm_solve<<<1, threads, staged ? bytes : 0, st>>>(s->g, t, dt, staged);
     s->launches++;
     FMDG_CK(cudaGetLastError());
