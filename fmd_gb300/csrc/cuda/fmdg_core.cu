@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(256) k_limits(Geo g, int group, unsigned long 
     unsigned long long lo[3] = {~0ull, ~0ull, ~0ull}, hi[3] = {0ull, 0ull, 0ull};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     {
-        if (group >= 0 && S.group[i] != group) continue;
+        if (group != -1 && S.group[i] != group) continue;
         for (int d = 0; d < 3; d++)
         {
             const unsigned long long b = (unsigned long long)__double_as_longlong(S.x[(size_t)d * g.cap + i]);

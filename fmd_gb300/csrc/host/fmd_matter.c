@@ -444,7 +444,7 @@ void fmd_matt_findLimits(fmd_t *md, int GroupID, fmd_rtriple_t LowerLimit, fmd_r
     }
     if (md->ParticlesDistributed)
     {
-        _fmdh_dev_ok(md, fmdg_find_limits(md->dev, GroupID == FMD_GROUP_ALL ? -1 : GroupID, LowerLimit, UpperLimit), "fmdg_find_limits");
+        _fmdh_dev_ok(md, fmdg_find_limits(md->dev, GroupID, LowerLimit, UpperLimit), "fmdg_find_limits");
         return;
     }
     if (_fmdh_current_atoms(md, &n, &x, &v, &kind, &group, &id) == 0)

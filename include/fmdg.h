@@ -241,7 +241,7 @@ int fmdg_pair_forces_noalloc(int n, const int nc[3], const int pbc[3], const dou
                              const fmdg_pair_t *pairs, const double *x, const unsigned *kind,
                              const int *cell_start, const int *cell_of, double *F, double *pe, void *stream);
 
-/* smallest and largest coordinates of a group's atoms (group < 0: all), on
+/* smallest and largest coordinates of a group's atoms (group -1: all), on
    the device: lower and upper hold starting values on entry, which stay
    where no atom lies beyond them (src/matter.c:211-240) */
 int fmdg_find_limits(fmdg_sys_t *s, int group, double lower[3], double upper[3]);
