@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(TTM_THREADS) k_ttm_solve(Geo g, DTuri t, doubl
     const bool own = staged && p.type == 1 && hi - lo <= (int)blockDim.x;
     if (own)
     {
-        const int i = lo + threadIdx.x, im1 = (i == lo) ? 0 : i - 1;
+        const int i = lo + threadIdx.x;
         const bool mine = i < hi;
         double te = 0.0, other = 0.0, ti = 0.0, xi = 0.0, sz = 0.0;
         if (mine)
@@ -462,27 +462,26 @@ __global__ void __launch_bounds__(TTM_THREADS) k_ttm_solve(Geo g, DTuri t, doubl
             ti = a.Ti[i];
             sz = a.srcz[i];
         }
+        const int im1 = (i == lo) ? 0 : i - 1;
         for (int j = 0; j < p.ratio; j++)
         {
-            if (mine && below_zero(te))
+            if (mine)
             {
-                const double t2 = other;
-                other = te;
-                te = t2;
-            }
-            else if (mine)
-            {
+                // (the tests beside the chain te -> 1/te -> te, not in it)
                 const double tl = Te[im1], th = Te[i + 1];
                 const double tlo = below_zero(tl) ? te : tl, thi = below_zero(th) ? te : th;
+                const bool still = below_zero(te);
                 // dte / (C_gamma te) * (K lap / dz2 - G (te - Ti) + source)
                 // with the constant quotients formed once per launch and one
                 // reciprocal instead of two IEEE divisions
                 const double q = dte_C * recip_newton(te);
                 const double source = calc_source ? a.spc[j] * sz : 0.0;
+                const double nv = te + q * (K_dz2 * (thi - 2 * te + tlo) - p.G * (te - ti) + source);
+                const double next = still ? other : nv;
                 other = te;
-                te = te + q * (K_dz2 * (thi - 2 * te + tlo) - p.G * (te - ti) + source);
-                Te2[i] = te;
-                xi += te;
+                te = next;
+                Te2[i] = te;        // (of a cell that stands still: what is there)
+                xi += still ? 0.0 : nv;
             }
             __syncthreads();
             double *tmp = Te2;
