@@ -32,10 +32,11 @@
 //
 // Kernels.  A single system of more than CLUSTER_ATOMS atoms runs the phases
 // as grid kernels (k_bin_classify, k_bin_scan, k_bin_cells, k_bin_arrivals,
-// k_bin_place).  A smaller one, and every packed system on the steps that
-// rebuild its list, runs all of them in one kernel: one cluster of blocks
-// per system, a cluster barrier between the phases (k_refresh_cluster) --
-// launches and their gaps were most of a small system's step.
+// k_bin_place).  A smaller one runs all of them in one kernel: one cluster of
+// blocks, a cluster barrier between the phases (k_refresh_cluster) -- launches
+// and their gaps were most of a small system's step.  Packed systems refresh
+// on the steps that rebuild their list only, on a cluster each, or, in packs
+// of systems above PACK_CLUSTER_ATOMS, by grid kernels (k_pack_*).
 #include <cooperative_groups.h>
 
 #include "fmdg_perdev.h"
@@ -48,6 +49,17 @@ namespace {
 // largest system of the cluster kernel: 4000 atoms refresh in 12 us against
 // 24 for the separate kernels, 32 000 atoms in 61 (eight blocks) against 21
 constexpr int CLUSTER_ATOMS = 1 << 13;
+// Largest packed system of the cluster kernel.  Its eight SMs a system refresh
+// 186 624 LJ atoms in 390 us, the grid kernels in 150, but each of their five
+// launches costs a little on every step, also the nine in ten that refresh
+// nothing: fleets of 186 624-atom jobs, us a step with the cluster -> grid
+// kernels, LJ 479 -> 438, EAM 939 -> 911, Morse 734 -> 706; sixteen LJ jobs of
+// 32 000 atoms 285 -> 279 but Morse 393 -> 400; 2048 jobs of 500 to 200 000
+// atoms (1.762e9 atom-steps/s on clusters alone) 1.750e9 with the line at
+// 2^14, 1.758e9 at 2^16.
+constexpr int PACK_CLUSTER_ATOMS = 1 << 16;
+// blocks of a pack's grid kernels: one per SM (two: 0.2 % less in that fleet)
+constexpr int PACK_GRID = 152;
 
 __device__ __forceinline__ int cell_flat(const Geo &g, int x, int y, int z)
 {
@@ -510,6 +522,7 @@ __global__ void __launch_bounds__(256) k_bin_classify(__grid_constant__ const Lo
 constexpr int WARP_CELLS = 8;
 
 // (one cluster)
+constexpr int SCAN_BLOCKS = 8;
 __global__ void __launch_bounds__(1024) k_bin_scan(__grid_constant__ const LocOne loc)
 {
     step_wait();
@@ -559,6 +572,122 @@ __global__ void __launch_bounds__(256) k_bin_place(__grid_constant__ const LocOn
         {
             dyn->place_done = 0;
             flip_sides(g, dyn, mode);
+        }
+    }
+}
+
+// --------------------------------------------- grid kernels (large, packed)
+//
+// The same phases for a pack of large systems, on the steps that rebuild a
+// member's skin list.  A bounded grid goes from one due member to the next,
+// so on the other steps a launch is a block per SM that reads the members'
+// flags and leaves (a block per 128 atoms, idle on most steps, cost 1.2 % of
+// the 2048-job fleet's rate).
+
+// the members (bits) that rebuild their list this step; every lane of the
+// warp takes part
+__device__ __forceinline__ unsigned due_members(const LocPack &L)
+{
+    const int s = threadIdx.x & 31;
+    bool due = false;
+    if (s < L.nsys)
+    {
+        const Dyn *d = L.geos[s].dyn;
+        due = d->steps_left > 0 && d->rebuild != 0;
+    }
+    return __ballot_sync(0xffffffffu, due);
+}
+
+__global__ void __launch_bounds__(256) k_pack_classify(__grid_constant__ const LocPack loc)
+{
+    step_wait();
+    __shared__ double hk[FMDG_MAXK];
+    for (unsigned m = due_members(loc); m; m &= m - 1)
+    {
+        const Geo &g = loc.geos[__ffs(m) - 1];
+        __syncthreads();
+        load_half_kicks(g, hk);
+        Dyn *dyn = g.dyn;
+        const int n = dyn->n;
+        const Side S = g.side[dyn->cur];
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+            classify_atom(g, dyn, S, i, FMDG_REFRESH_ONLY, hk);
+    }
+}
+
+// (one cluster of SCAN_BLOCKS per system)
+__global__ void __launch_bounds__(512) k_pack_scan(__grid_constant__ const LocPack loc)
+{
+    step_wait();
+    const Geo &g = loc.geos[blockIdx.x / SCAN_BLOCKS];
+    Dyn *dyn = g.dyn;
+    if (dyn->steps_left <= 0 || !dyn->rebuild || !dyn->any_move) return;
+    __shared__ ScanSmem sm;
+    cg::cluster_group cl = cg::this_cluster();
+    scan_cells(g, dyn, g.side[dyn->cur], g.side[dyn->cur ^ 1], sm, cl);
+}
+
+__global__ void __launch_bounds__(256) k_pack_cells(__grid_constant__ const LocPack loc)
+{
+    step_wait();
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+    for (unsigned m = due_members(loc); m; m &= m - 1)
+    {
+        const Geo &g = loc.geos[__ffs(m) - 1];
+        const Dyn *dyn = g.dyn;
+        if (!dyn->any_move) continue;
+        const Side S = g.side[dyn->cur];
+        for (int c = warp * WARP_CELLS; c < g.ncell; c += nw * WARP_CELLS) replay_cells(g, S, c, WARP_CELLS, threadIdx.x & 31);
+    }
+}
+
+__global__ void __launch_bounds__(128) k_pack_arrivals(__grid_constant__ const LocPack loc)
+{
+    step_wait();
+    for (unsigned m = due_members(loc); m; m &= m - 1)
+    {
+        const Geo &g = loc.geos[__ffs(m) - 1];
+        const Dyn *dyn = g.dyn;
+        if (!dyn->any_move) continue;
+        const Side S = g.side[dyn->cur], T = g.side[dyn->cur ^ 1];
+        for (int D = blockIdx.x * blockDim.x + threadIdx.x; D < g.ncell; D += gridDim.x * blockDim.x) order_arrivals(g, S, T, D);
+    }
+}
+
+// The last block to finish a member swaps its sides and leaves the cells'
+// counters at zero for its next refresh.
+__global__ void __launch_bounds__(256) k_pack_place(__grid_constant__ const LocPack loc)
+{
+    step_wait();
+    __shared__ unsigned ticket;
+    for (unsigned m = due_members(loc); m; m &= m - 1)
+    {
+        const Geo &g = loc.geos[__ffs(m) - 1];
+        Dyn *dyn = g.dyn;
+        const int cur = dyn->cur, n = dyn->n;
+        const bool moved = dyn->any_move != 0;
+        const int n_next = moved ? dyn->n_next : n;
+        const Side S = g.side[cur], T = g.side[cur ^ 1];
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < g.cap; i += gridDim.x * blockDim.x)
+        {
+            if (i < n) place_atom<true>(g, dyn, S, T, i, moved, n_next);
+            if (i >= n_next) g.pos[i] = -1;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+        {
+            __threadfence();
+            ticket = atomicAdd(&dyn->place_done, 1u);
+        }
+        __syncthreads();
+        if (ticket != gridDim.x - 1) continue;
+        // (dep_count, arr_lower, arr_total, bucket_fill are contiguous)
+        if (moved)
+            for (int c = threadIdx.x; c < 4 * g.ncell; c += blockDim.x) g.dep_count[c] = 0;
+        if (threadIdx.x == 0)
+        {
+            dyn->place_done = 0;
+            flip_sides(g, dyn, FMDG_REFRESH_ONLY);
         }
     }
 }
@@ -617,7 +746,8 @@ __global__ void __launch_bounds__(512) k_refresh_cluster(__grid_constant__ const
 
 // Blocks of as few threads as give every atom one: the phases are binary64
 // work, which an SM issues for one warp at a time, so few warps on many SMs.
-// A pack's systems take eight blocks each (the portable cluster size).
+// A pack's systems (up to PACK_CLUSTER_ATOMS) take eight blocks each (the
+// portable cluster size).
 constexpr int REFRESH_BLOCKS = 8;
 int refresh_threads(int n, int blocks)
 {
@@ -683,7 +813,7 @@ int fmdg_launch_refresh(fmdg_sys_t *s, int mode, double dt, int group, int therm
     FMDG_CK(cudaMemsetAsync(g.dep_count, 0, sizeof(int) * 4 * (size_t)g.ncell, st));
     const bool ov = s->overlap;
     FMDG_CK(fmdg_launch(k_bin_classify, fmdg_grid(g.cap, 256), 256, 0, st, false, 1, L, mode));
-    FMDG_CK(fmdg_launch(k_bin_scan, 8, 1024, 0, st, ov, 8, L));
+    FMDG_CK(fmdg_launch(k_bin_scan, SCAN_BLOCKS, 1024, 0, st, ov, SCAN_BLOCKS, L));
     FMDG_CK(fmdg_launch(k_bin_cells, fmdg_grid(g.ncell, 4 * WARP_CELLS), 128, 0, st, ov, 1, L));
     FMDG_CK(fmdg_launch(k_bin_arrivals, fmdg_grid(g.ncell, 128), 128, 0, st, ov, 1, L));
     FMDG_CK(fmdg_launch(k_bin_place, fmdg_grid(g.cap, 256), 256, 0, st, ov, 1, L, mode));
@@ -691,19 +821,39 @@ int fmdg_launch_refresh(fmdg_sys_t *s, int mode, double dt, int group, int therm
     return FMDG_OK;
 }
 
+bool fmdg_pack_large(int n) { return n > PACK_CLUSTER_ATOMS; }
+
 // Step start of every system of a pack: velocity-Verlet start step, slot
 // tables and displacement test (k_skin_start), then the cell refresh of the
-// systems that rebuild their skin list this step.  Returns the kernels
-// launched, or minus a status.
+// systems that rebuild their skin list this step: a cluster each, or, in a
+// pack of large systems, the grid kernels.  Returns the kernels launched, or
+// minus a status.
 int fmdg_pack_launch_refresh(const fmdg_pack_launch &P)
 {
     cudaStream_t st = P.stream;
+    const bool ov = P.overlap;
+    const int mode = FMDG_REFRESH_ONLY;
     int n = fmdg_pack_launch_start(P);
     if (n < 0) return n;
-    int most = 1;
-    for (int k = 0; k < P.nsys; k++) most = P.la.geos[k].cap > most ? P.la.geos[k].cap : most;
-    const cudaError_t e = fmdg_launch(k_refresh_cluster<LocPack>, REFRESH_BLOCKS * P.nsys, refresh_threads(most, REFRESH_BLOCKS), 0, st,
-                                      P.overlap, REFRESH_BLOCKS, P.la, FMDG_REFRESH_ONLY);
+    if (P.large)
+    {
+        const int grid = PACK_GRID;
+        fmdg_launch(k_pack_classify, grid, 256, 0, st, ov, 1, P.la);
+        fmdg_launch(k_pack_scan, SCAN_BLOCKS * P.nsys, 512, 0, st, ov, SCAN_BLOCKS, P.la);
+        fmdg_launch(k_pack_cells, grid, 256, 0, st, ov, 1, P.la);
+        fmdg_launch(k_pack_arrivals, grid, 128, 0, st, ov, 1, P.la);
+        fmdg_launch(k_pack_place, grid, 256, 0, st, ov, 1, P.la);
+        n += 5;
+    }
+    else
+    {
+        int most = 1;
+        for (int k = 0; k < P.nsys; k++) most = P.la.geos[k].cap > most ? P.la.geos[k].cap : most;
+        fmdg_launch(k_refresh_cluster<LocPack>, REFRESH_BLOCKS * P.nsys, refresh_threads(most, REFRESH_BLOCKS), 0, st, ov,
+                    REFRESH_BLOCKS, P.la, mode);
+        n++;
+    }
+    const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return -fmdg_fail("pack refresh", e);
-    return n + 1;
+    return n;
 }

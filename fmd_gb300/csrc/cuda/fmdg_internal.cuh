@@ -335,6 +335,7 @@ struct fmdg_pack_launch
     int mixed;
     int lean;                   // every member has one kind (lean kernels)
     int shares;                 // the members' list walks are split into shares (small systems)
+    int large;                  // the members refresh by grid kernels (fmdg_pack_large)
     int fblk;                   // threads per block of the list/density/force kernels
     bool overlap;               // the launches are a captured step's (fmdg_launch)
     LocPack la;                 // 128-thread atom blocks
@@ -343,6 +344,8 @@ struct fmdg_pack_launch
 // all three return the number of kernels launched, or minus a status
 int fmdg_pack_launch_start(const fmdg_pack_launch &P);
 int fmdg_pack_launch_refresh(const fmdg_pack_launch &P);
+// does a packed system of n atoms refresh by grid kernels, not by a cluster?
+bool fmdg_pack_large(int n);
 int fmdg_pack_launch_forces(const fmdg_pack_launch &P, int phases);
 
 // ---- helpers shared by the translation units --------------------------------

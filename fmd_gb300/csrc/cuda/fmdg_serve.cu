@@ -104,6 +104,7 @@ struct Pack
     int cls = 0, mixed = 0;
     int lean = 0;       // one-kind jobs (lean kernels); a job's variant never depends on the mix
     int shares = 0;     // small jobs, whose list walks are split into shares (Geo::share_log > 0)
+    int large = 0;      // large jobs, whose cells are refreshed by grid kernels (fmdg_pack_large)
     cudaStream_t stream = nullptr;
     std::vector<Job *> members;
     bool dirty = true;
@@ -227,16 +228,17 @@ int want_fblk(const fmdg_server_t *S, const Pack &p)
 
 int pack_class(int cats) { return __builtin_popcount(cats) > 1 ? 0 : __builtin_ctz(cats); }
 
-// a pack of (class, mixed, lean, shares) with room for one more system
-Pack *pack_for(fmdg_server_t *S, int cls, int mixed, int lean, int shares)
+// a pack of (class, mixed, lean, shares, large) with room for one more system
+Pack *pack_for(fmdg_server_t *S, int cls, int mixed, int lean, int shares, int large)
 {
     for (Pack *p : S->packs[cls][mixed])
-        if (p->lean == lean && p->shares == shares && p->active() < FMDG_PACK_MAX) return p;
+        if (p->lean == lean && p->shares == shares && p->large == large && p->active() < FMDG_PACK_MAX) return p;
     Pack *p = new Pack();
     p->cls = cls;
     p->mixed = mixed;
     p->lean = lean;
     p->shares = shares;
+    p->large = large;
     if (cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking) != cudaSuccess)
     {
         delete p;
@@ -366,7 +368,7 @@ int admit(fmdg_server_t *S, double budget_s)
             continue;
         }
         Pack *p = pack_for(S, pack_class(j->cats), j->prec == FMDG_PREC_MIXED, j->nkinds == 1,
-                           j->sys->g.share_log > 0);
+                           j->sys->g.share_log > 0, fmdg_pack_large(j->n));
         if (!p)
         {
             fail_job(S, j, fmdg_set_error("fmdg_srv: cannot create a pack stream"), true);
@@ -422,6 +424,7 @@ int rebuild(fmdg_server_t *S, Pack &p)
     P.shares = p.shares;
     P.mixed = p.mixed;
     P.fblk = fblk;
+    P.large = p.large;
     LocPack *locs[2] = {&P.la, &P.lf};
     for (LocPack *L : locs)
     {
@@ -444,7 +447,7 @@ int rebuild(fmdg_server_t *S, Pack &p)
     cudaGraph_t graph;
     FMDG_CK(cudaStreamBeginCapture(p.stream, cudaStreamCaptureModeThreadLocal));
     // one step per graph, replayed chunk_steps times: a membership change
-    // re-captures 10-11 kernels, not chunk_steps times as many
+    // re-captures 4 to 9 kernels, not chunk_steps times as many
     int rc = FMDG_OK, nk = 0;
     {
         P.overlap = true;
