@@ -706,7 +706,7 @@ template <class L>
 __global__ void __launch_bounds__(512) k_refresh_cluster(__grid_constant__ const L loc, int mode)
 {
     step_wait();
-    constexpr bool PACK = L::renumbered;
+    constexpr bool PACK = !L::one_system;
     cg::cluster_group cl = cg::this_cluster();
     const int nblk = cl.num_blocks(), rank = cl.block_rank();
     const Geo &g = cluster_geo(loc, blockIdx.x / nblk);

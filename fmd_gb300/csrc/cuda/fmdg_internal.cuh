@@ -48,7 +48,7 @@ struct Side
     unsigned *atomid;
     int *cell_of;
     int *cell_start;
-    int *slot;          // skin-list systems: stable slot number of the atom
+    int *slot;          // skin-list systems: the atom's slot (its index at the last list build)
 };
 
 // integrator arguments of the step in flight (set by the host before a
@@ -126,10 +126,10 @@ struct Geo   // passed by value to kernels
     double *partials;             // per block: 8 doubles
     fmdg_thermo_t *thermo;
     Dyn *dyn;
-    // Verlet-skin neighbour list of packed (served) systems, indexed by a
-    // stable slot number: the reference's binning renumbers atoms every step,
-    // the slots do not, so the list (radius largest cutoff + skin) is reused
-    // until an atom has moved more than skin/2 since its build.  List entries
+    // Verlet-skin neighbour list (fmdg_skin.cu), indexed by a slot number that
+    // every build forms anew (the index): the reference's binning renumbers
+    // atoms every step, the slots stay, so the list (radius largest cutoff +
+    // skin) is reused until an atom has moved more than skin/2 since.  List entries
     // hold the neighbour's slot and the stencil offset between the two
     // atoms' cells at the build; positions are kept relative to the cell an
     // atom had at the build (unwrapped across periodic faces), so the offset
@@ -264,7 +264,6 @@ struct LocOne
     static constexpr int lean_min_blocks = 7; // lean force kernels: 7 blocks of 128 (72 registers), measured best
     static constexpr bool one_lane = false;     // lanes by Geo::lane_log
     static constexpr bool split_shares = false; // every share has its lane
-    static constexpr bool renumbered = false;  // skin-list slots stay the upload positions
     Geo g;
 };
 
@@ -277,7 +276,6 @@ struct LocPack
     static constexpr int lean_min_blocks = 0; // packed lean force kernels: compiler's choice, measured best
     static constexpr bool one_lane = true;      // one share, one lane per slot
     static constexpr bool split_shares = false;
-    static constexpr bool renumbered = true;   // slot = index whenever a list is built
     int nsys;
     int bstart[FMDG_PACK_MAX + 1];
     Geo geos[FMDG_PACK_MAX];

@@ -9,22 +9,26 @@
 // list.  Pairs are still tested against the exact cutoff at every
 // evaluation, so the list only prunes.
 //
-// Slots.  A slot starts as the atom's upload position and travels with the
-// atom through every re-binning.  Packed systems renumber the slots in the
-// current cell order at each rebuild (slot = index), and refresh their
-// cells only on rebuild steps, so between rebuilds slot and index coincide.
+// Slots.  Every list build numbers the slots in the current cell order (slot
+// = index), so the lists and gathers of a warp stay in one part of the box
+// however far the atoms have diffused; between builds a slot travels with its
+// atom through the re-binnings.  (Slots that stayed the upload positions: a
+// fluid of 192 000 LJ atoms at 3000 K went from 277 to 335 us a step in
+// 30 000 steps, in mixed precision 152 to 216; 268 and 144 throughout now.)  Packed systems refresh their cells only on rebuild
+// steps, so between rebuilds slot and index coincide.
 //
 // Packed step:
 //   k_skin_start    velocity-Verlet start step, per-step slot positions,
 //                   displacement test -> rebuild flag
 //   (rebuild steps only) k_refresh_cluster (fmdg_bin.cu): reference-order
-//                   cell refresh and slot tables (renumbered);
+//                   cell refresh and slot tables (renumbered; k_pack_* for
+//                   large systems);
 //   k_nlist_skin    stencil scan of the cells within the list radius
 //   k_density_skin  EAM pass 1 + embedding
 //   k_force_skin    pair forces + velocity-Verlet finish step + thermo
 //                   record; 2^lane_log lanes per slot in both
-// Single-system step: the reference-order refresh with the slot tables
-// (stable slots) every step, k_nlist_skin (when flagged), density, forces.
+// Single-system step: the reference-order refresh with the slot tables every
+// step, k_nlist_skin (when flagged; renumbers the slots), density, forces.
 //
 // Geometry.  An atom's binary32 position is kept relative to the cell it
 // had at the last build (unwrapped across periodic faces: it moves less
@@ -504,17 +508,32 @@ __device__ __forceinline__ void for_each_build_cell(const Geo &g, const SkinOffT
     });
 }
 
-// per-slot state recorded with a new list: build cell and build-frame
-// position (+ its double-float remainder in binary64 mode)
-__device__ __forceinline__ void record_build(const Geo &g, const Side &S, int t, int i, float4 xi)
+// Per-slot state recorded with a new list: build cell and build-frame
+// position (+ its double-float remainder in binary64 mode).  Slot = index:
+// packed systems were renumbered by the refresh, a single system is here --
+// nothing in a build reads a slot table of another atom, so every thread
+// rewrites its own row of them.
+template <class L>
+__device__ __forceinline__ void record_build(const Geo &g, const Side &S, int t, float4 xi)
 {
-    g.cb[t] = S.cell_of[i];
+    const int c = S.cell_of[t];
+    g.cb[t] = c;
     g.xl[t] = xi;
     g.xb[t] = xi;
+    if (!L::one_system && g.prec != FMDG_PREC_FP64) return;
+    const size_t cap = g.cap;
+    const double4_32a x = L::one_system ? make_double4_32a(S.x[t], S.x[cap + t], S.x[2 * cap + t], 0.0) : g.xd[t];
+    if (L::one_system)
+    {
+        S.slot[t] = t;
+        g.pos[t] = t;
+        g.xd[t] = x;
+        g.gslot[t] = S.group[t];
+    }
     if (g.prec == FMDG_PREC_FP64)
     {
         // (xs is 1 in binary64 mode)
-        const double4_32a x = g.xd[t], o = g.corig[S.cell_of[i]];
+        const double4_32a o = g.corig[c];
         g.xr[2 * (size_t)t] = xi;
         g.xr[2 * (size_t)t + 1] = make_float4((float)(x.x - o.x - (double)xi.x), (float)(x.y - o.y - (double)xi.y),
                                               (float)(x.z - o.z - (double)xi.z), 0.f);
@@ -556,8 +575,8 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_nlist_skin(__
     if (t < cap)
     {
         int cnt = 0;
-        const int i = g.pos[t];
-        if (i >= 0)
+        const int i = t;        // (slot = index: record_build)
+        if (i < dyn->n)
         {
             const Side S = g.side[dyn->cur];
             const float4 xi = g.xf4[i];
@@ -599,8 +618,7 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_nlist_skin(__
                     for (; m; m &= m - 1)
                     {
                         const int j = j0 + __ffs(m) - 1;
-                        const int sj = L::renumbered ? j : S.slot[j];
-                        buf = make_int4(buf.y, buf.z, buf.w, (int)((unsigned)sj | ((unsigned)code << SLOT_BITS)));
+                        buf = make_int4(buf.y, buf.z, buf.w, (int)((unsigned)j | ((unsigned)code << SLOT_BITS)));
                         cnt++;
                         if ((cnt & 3) == 0 && cnt <= maxnb) row[(size_t)((cnt >> 2) - 1) * cap] = buf;
                     }
@@ -613,33 +631,29 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_nlist_skin(__
                                 : (rem == 2) ? make_int4(buf.z, buf.w, 0, 0) : make_int4(buf.y, buf.z, buf.w, 0);
                 row[(size_t)(cnt >> 2) * cap] = last;
             }
-            record_build(g, S, t, i, xi);
+            record_build<L>(g, S, t, xi);
         }
+        else
+            g.pos[t] = -1;
         g.nbr_count[t] = cnt;
     }
     finish_build(dyn, nb);
 }
 
-// Single-system build (a served job's admission, the fmd.h path) with G
-// lanes per slot: a system of 10^4-10^5 atoms gives one thread per slot too
-// few warps to hide the gather latency of its long candidate walk.  The G
-// lanes of a slot test G consecutive candidates of a cell together and
-// place their hits in candidate order (ballot + prefix count), so the list
-// is the one-thread build's, entry for entry.
 // The list of slot t built by the G lanes of a group (gl: this lane's
 // index in it, gbase: the group's first lane in the warp): the lanes test
 // G consecutive candidates of a cell together and place their hits in
 // candidate order (ballot + prefix count), so the list is the one-thread
 // build's, entry for entry.  Every lane of the group must call it (its
 // control flow depends on the slot only).
-__device__ __forceinline__ void build_slot_grouped(const Geo &g, const Side &S, const SkinOffT<false> &so, int t,
+__device__ __forceinline__ void build_slot_grouped(const Geo &g, const Side &S, const SkinOffT<false> &so, int t, int n,
                                                    int G, int gl, int gbase)
 {
     const int cap = g.cap, maxnb = g.maxnb;
     const unsigned gmask = (G == 32) ? 0xffffffffu : ((1u << G) - 1u) << gbase;
     int cnt = 0;
-    const int i = g.pos[t];
-    if (i >= 0)
+    const int i = t;        // (slot = index: record_build)
+    if (i < n)
     {
         const float4 xi = g.xf4[i];
         const float rb2 = g.rskin2 * 1.00001f;   // as in k_nlist_skin
@@ -664,13 +678,15 @@ __device__ __forceinline__ void build_slot_grouped(const Geo &g, const Side &S, 
                     const int k = cnt + __popc(m & ((1u << gl) - 1u));
                     if (k < maxnb)
                         ent[((size_t)(k >> 2) * cap + t) * 4 + (k & 3)] =
-                            (int)((unsigned)S.slot[j] | ((unsigned)code << SLOT_BITS));
+                            (int)((unsigned)j | ((unsigned)code << SLOT_BITS));
                 }
                 cnt += __popc(m);
             }
         });
-        if (gl == 0) record_build(g, S, t, i, xi);
+        if (gl == 0) record_build<LocOne>(g, S, t, xi);
     }
+    else if (gl == 0)
+        g.pos[t] = -1;
     if (gl == 0) g.nbr_count[t] = cnt;
 }
 
@@ -688,7 +704,7 @@ __global__ void __launch_bounds__(128) k_nlist_skin_grp(__grid_constant__ const 
     __shared__ SkinOffT<false> so;
     load_offsets(g, so);
     const int t = (blockIdx.x * blockDim.x + threadIdx.x) / G;   // uniform over a group
-    if (t < g.cap) build_slot_grouped(g, g.side[dyn->cur], so, t, G, threadIdx.x & (G - 1), threadIdx.x & 31 & ~(G - 1));
+    if (t < g.cap) build_slot_grouped(g, g.side[dyn->cur], so, t, dyn->n, G, threadIdx.x & (G - 1), threadIdx.x & 31 & ~(G - 1));
     finish_build(dyn, gridDim.x);
 }
 
