@@ -995,12 +995,15 @@ extern "C" int fmdg_set_state(fmdg_sys_t *s, const double *x, const double *v)
     };
     if (x && (rc = put3(x, S.x))) return rc;
     if (v && (rc = put3(v, S.v))) return rc;
-    if (x)
-    {
-        // positions set from outside: the skin list is rebuilt first
-        const int one = 1;
-        FMDG_CK(cudaMemcpyAsync((char *)s->g.dyn + offsetof(Dyn, rebuild), &one, sizeof one, cudaMemcpyHostToDevice, s->stream));
-    }
+    // positions set from outside: the skin list is rebuilt first
+    return x ? fmdg_renew_list(s) : FMDG_OK;
+}
+
+extern "C" int fmdg_renew_list(fmdg_sys_t *s)
+{
+    if (!s->atoms) return FMDG_E_STATE;
+    const int one = 1;
+    FMDG_CK(cudaMemcpyAsync((char *)s->g.dyn + offsetof(Dyn, rebuild), &one, sizeof one, cudaMemcpyHostToDevice, s->stream));
     return FMDG_OK;
 }
 

@@ -98,8 +98,18 @@ static bool initial_forces(fmd_t *md)
     return true;
 }
 
+/* After a state was saved the run goes on as one that starts from the saved
+   state does, bit for bit: from a neighbour list of the current positions
+   (its age shows in the last bits of the forces), and inside a run from
+   forces over it. */
+void _fmdh_state_saved(fmd_t *md)
+{
+    if (!_fmdh_dev_ok(md, fmdg_renew_list(md->dev), "fmdg_renew_list")) return;
+    if (md->vv_running) initial_forces(md);
+}
+
 /* velocity Verlet with optional Berendsen scaling (src/integrators.c:227-264) */
-static void vv_integrate(fmd_t *md, double duration, bool thermostat)
+static void vv_steps(fmd_t *md, double duration, bool thermostat)
 {
     const double start = md->time;
     const double dt = md->timestep;
@@ -147,6 +157,14 @@ static void vv_integrate(fmd_t *md, double duration, bool thermostat)
         _fmdh_check_device_errors(md);
         if (md->EventHandler != NULL) _fmdh_send_timer_events(md);
     }
+}
+
+static void vv_integrate(fmd_t *md, double duration, bool thermostat)
+{
+    const bool outer = md->vv_running;
+    md->vv_running = true;
+    vv_steps(md, duration, thermostat);
+    md->vv_running = outer;
 }
 
 void fmd_dync_integrate(fmd_t *md, int GroupID, fmd_real_t duration, fmd_real_t timestep)

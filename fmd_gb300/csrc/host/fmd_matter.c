@@ -755,6 +755,7 @@ void fmd_io_saveState(fmd_t *md, fmd_string_t filename)
             fprintf(fp, fmt3, v[3 * i], v[3 * i + 1], v[3 * i + 2]);
         }
         fclose(fp);
+        if (md->ParticlesDistributed) _fmdh_state_saved(md);
     }
     free(x); free(v); free(kind); free(group); free(id);
 }

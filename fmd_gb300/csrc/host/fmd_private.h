@@ -126,6 +126,7 @@ struct _fmd
     double GroupVirial;    /* pair virial of the last force evaluation (no reference counterpart) */
     double GroupMomentum[3];
     unsigned GroupParticlesNum;
+    bool vv_running;          /* inside a velocity-Verlet run (an event handler may call in) */
     bool thermo_pending;      /* device thermo record newer than the cache */
     /* events */
     fmd_EventHandler_t EventHandler;
@@ -187,6 +188,7 @@ void _fmdh_turies_updated(fmd_t *md, unsigned mask, bool with_ttm);
 /* fmd_dync.c */
 void _fmdh_send_timer_events(fmd_t *md);
 void _fmdh_check_device_errors(fmd_t *md);
+void _fmdh_state_saved(fmd_t *md);
 
 /* rng (fmd_matter.c) */
 double _fmdh_rng_uniform(fmd_t *md, unsigned long long *state);

@@ -139,6 +139,10 @@ int fmdg_download(fmdg_sys_t *s, int *cell_of, double *x, double *v, double *F, 
                   unsigned *kind, int *group, unsigned *atomid);
 /* overwrite positions and/or velocities (cell order, n*3 interleaved) */
 int fmdg_set_state(fmdg_sys_t *s, const double *x, const double *v);
+/* build the neighbour list anew before the next forces: they are then those
+   of the same state uploaded afresh, bit for bit (a list's age shows in the
+   order and rounding of the pair sums) */
+int fmdg_renew_list(fmdg_sys_t *s);
 
 /* --- per-timestep work ---------------------------------------------- */
 /* cell-list refresh with the reference's cell assignment and in-cell order
