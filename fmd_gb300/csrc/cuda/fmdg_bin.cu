@@ -162,8 +162,10 @@ __device__ __forceinline__ void classify_atom(const Geo &g, Dyn *dyn, const Side
         if (g.skin_on)
         {
             // the slot is gone: out of reach of the lists that hold it (a
-            // position beyond every cutoff, finite in all pair arithmetic)
-            // until the next build leaves it out
+            // position beyond every cutoff) until the next build leaves it
+            // out.  What the branch-free walks form from so large an r^2 may
+            // be infinite or not a number (the cubic of a table's interval):
+            // they select zero instead of it, and must not multiply by a mask.
             const int t = S.slot[i];
             const float far = 1e8f;
             g.pos[t] = -1;
