@@ -696,9 +696,9 @@ def plain_sample(L, eam, jobs, every=PLAIN_EVERY, nsteps=PLAIN_STEPS):
     single-system binary64 path (the path libfmd.so's fmd_dync_integrate
     drives).  Every `every`-th job: set-up plus its first step timed as a
     fixed cost, then up to `nsteps` steps timed; the job's time is the fixed
-    cost plus the per-step time times its remaining steps (the plain path
-    rebuilds its exact neighbour list every step, so a step costs the same
-    all along).  Returns (atom-steps/s, details)."""
+    cost plus the per-step time times its remaining steps (the timed steps
+    hold several list builds, and a step costs the same all along: the slots
+    are renumbered at each).  Returns (atom-steps/s, details)."""
     from fmd_gb300 import serve
     t_total, as_total, timed_s = 0.0, 0.0, 0.0
     drifts = []

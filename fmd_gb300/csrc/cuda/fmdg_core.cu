@@ -316,8 +316,8 @@ extern "C" int fmdg_create(fmdg_sys_t **out, int device)
     s->ttm_turi = -1;
     s->fblk = 128;
     s->rec = REC_FULL;
-    // Verlet skin of the neighbour list (A) of mixed-precision systems;
-    // FMD_SKIN=0 keeps the exact per-step stencil list
+    // default Verlet skin of the neighbour list (A); 0 (FMD_SKIN=0) keeps
+    // the exact per-step stencil list
     s->skin = 0.5;
     if (const char *e = getenv("FMD_SKIN")) s->skin = atof(e);
     s->g.xs = s->g.inv_xs = 1.0;
@@ -611,7 +611,8 @@ extern "C" int fmdg_set_precision(fmdg_sys_t *s, int mode)
 }
 
 // Neighbour-list entries per atom: 1.3x the pairs an atom of the densest
-// cell has within the list radius (largest cutoff + 0.01), at least 32.
+// cell has within the list radius (largest cutoff + the skin, or + 0.01 on
+// the exact list), at least 32; a caller's number as it is.
 int fmdg_list_capacity(const fmdg_sys_t *s, const int *cell_count, int ncell)
 {
     const Geo &g = s->g;
@@ -636,7 +637,6 @@ int fmdg_list_capacity(const fmdg_sys_t *s, const int *cell_count, int ncell)
     return (!s->served && s->skin_used > 0.0 && (size_t)g.cap * twice * 4 < ((size_t)2 << 30)) ? twice : est;
 }
 
-// Neighbour-list entries per atom (before fmdg_upload); 0: the estimate.
 extern "C" int fmdg_set_build_lanes(fmdg_sys_t *s, int lanes)
 {
     if (lanes != 0 && lanes != 1 && lanes != 2 && lanes != 4 && lanes != 8 && lanes != 16 && lanes != 32)
@@ -653,6 +653,7 @@ extern "C" int fmdg_set_refresh_blocks(fmdg_sys_t *s, int blocks)
     return FMDG_OK;
 }
 
+// Neighbour-list entries per atom (before fmdg_upload); 0: the estimate.
 extern "C" int fmdg_set_list_capacity(fmdg_sys_t *s, int entries)
 {
     if (entries < 0 || entries > 1024 || (entries % 8) != 0)
@@ -696,8 +697,11 @@ int fmdg_share_log(const fmdg_sys_t *s, int n)
     int target = s->g.prec == FMDG_PREC_FP64 ? 400000 : 1 << 16;
     if (s->served) target = s->g.prec == FMDG_PREC_FP64 ? 1 << 14 : 1 << 13;
     int l = 0;
-    // (32 shares: argon 256 atoms 32.6 -> 30.9 us, EAM 2048 50 -> 46.6, but
-    // argon 4000 36.0 -> 38.6)
+    // (32 shares against 16 in binary64, us a step: 2048 atoms, LJ 21.9 ->
+    // 19.9, EAM 34.0 -> 30.6, Morse 30.4 -> 28.2; 2916, 26.0 -> 25.6, 35.0 ->
+    // 33.9, 43.3 -> 41.0; 4000, 25.8 -> 25.7, 36.5 -> 34.4, 39.0 -> 37.0, but
+    // argon 36.0 -> 38.6 when the line was drawn; in mixed precision the
+    // target leaves 16 above 2048)
     const int most = (!s->served && n <= 2048) ? 5 : 4;
     while (l < most && ((long long)n << (l + 1)) <= target) l++;
     return l;

@@ -667,9 +667,6 @@ int fmdg_launch_forces(fmdg_sys_t *s, int group, int finish, double dt, int ther
     return fmdg_launch_pair_forces(s, group, finish, dt, thermostat, tau, T0);
 }
 
-// Neighbour lists, EAM density and pair forces + finish step for every
-// system of a pack (one launch per kernel).
-
 // thermo-only reduction (no force evaluation); keeps the potential energy
 int fmdg_launch_thermo(fmdg_sys_t *s, int group, int thermostat, double dt, double tau, double T0)
 {

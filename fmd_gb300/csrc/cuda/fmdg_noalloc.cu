@@ -206,7 +206,9 @@ __global__ void __launch_bounds__(32 * NOALLOC_WARPS) k_pair_noalloc(
                         const float dx = px - trunc_f(x[j]), dy = py - trunc_f(x[n + j]);
                         const float dz = pz - trunc_f(x[2 * (size_t)n + j]);
                         bad = bad || kind[j] >= (unsigned)a.nkinds;     // outside the pair table: no table read
-                        hit = !bad && !(dx * dx + dy * dy + dz * dz >= lim2);     // (NaN passes)
+                        // (a coordinate that is not a number is infinity here and
+                        // dropped, as the exact test drops it)
+                        hit = !bad && !(dx * dx + dy * dy + dz * dz >= lim2);
                     }
                     const unsigned m = __ballot_sync(FULL, hit);
                     if (hit) q[qn + __popc(m & ((1u << lane) - 1u))] = j | (code << 20);

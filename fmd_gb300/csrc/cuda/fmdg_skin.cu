@@ -401,12 +401,12 @@ __device__ __forceinline__ int prune_share(const Geo &g, const SkinOffT<false> &
 }
 
 // f(neighbour slot, its double-float row, the entry's cell steps) for the m
-// entries of a share's compact list.  L1 wavefronts bound the walk (80 % of
-// their peak, the FMA pipe at 38 to 50 %), so a neighbour is one 32-byte row
-// and its offset one shared word (rv_steps), F'(rho_j) rides in the row
-// (LEAN) and the EAM slopes come from one 64-byte row (eam_pair_row): 256k
-// EAM density 187 -> 166 us, force 230 -> 175; 300 jobs of 600 to 3000
-// atoms 1464 -> 1160 us a step.
+// entries of a share's compact list.  L1 wavefronts bound the walk, so a
+// neighbour is one 32-byte row and its offset one shared word (rv_steps),
+// F'(rho_j) rides in the row (LEAN) and the EAM slopes come from one 64-byte
+// row (eam_pair_row): 256k EAM density 187 -> 166 us, force 230 -> 177, L1
+// wavefronts from 80 % of their peak (the FMA pipe at 38 to 50 %) to 68 and
+// 73 % (44 and 62 %); 300 jobs of 600 to 3000 atoms 1464 -> 1160 us a step.
 template <typename F>
 __device__ __forceinline__ void for_each_pruned(const Geo &g, const SkinOffT<false> &so, int m, int t, int v, int V, F &&f)
 {

@@ -103,8 +103,9 @@ int fmdg_set_eam(fmdg_sys_t *s, int nelem, int Nrho, double drho, int Nr2, doubl
                  const double *phi, const double *phiDD);
 int fmdg_set_precision(fmdg_sys_t *s, int mode);
 /* Verlet skin (A) of the neighbour list, before fmdg_upload: the list holds
-   the pairs within the largest cutoff + skin, indexed by stable atom slots,
-   and is rebuilt on the device once an atom has moved more than skin/2.
+   the pairs within the largest cutoff + skin, indexed by atom slots (the
+   storage order of the build), and is rebuilt on the device once an atom
+   has moved more than skin/2.
    Used when every periodic box length exceeds twice the list radius and
    the radius spans at most two cells; otherwise (and with skin 0) the
    exact stencil list is rebuilt every step.  Default: 0.5 A (environment
@@ -112,10 +113,11 @@ int fmdg_set_precision(fmdg_sys_t *s, int mode);
    for binary64 systems of several kinds. */
 int fmdg_set_skin(fmdg_sys_t *s, double skin);
 /* Neighbour-list entries per atom (before fmdg_upload; 0, the default:
-   1.3 x the count at the fullest cell's density + 16).  A multiple of 8 up
-   to 1024.  An atom with more neighbours than the list holds scans its
-   stencil directly (same results, slower), so this bounds list memory
-   only. */
+   1.3 x the count at the fullest cell's density + 16, in single systems
+   with a skin list twice that while the lists stay below 2 GB).  A multiple
+   of 8 up to 1024.  An atom with more neighbours than the list holds scans
+   its stencil directly: the same pairs, several times slower, on a skin
+   list with other roundings in the last bits. */
 int fmdg_set_list_capacity(fmdg_sys_t *s, int entries);
 /* Threads per atom of this system's skin-list builds: 0 (default) picks
    them by size (16 up to 2^14 atoms, 8 up to 2^16, else 1); 1, 2, 4, 8,
@@ -275,8 +277,8 @@ int fmdg_measure_fma_peak(fmdg_sys_t *s, int fp64, double *tflops);
    kernels (d2f_rn): for n inputs, its results and the conversion
    instruction's */
 int fmdg_check_d2f(fmdg_sys_t *s, const double *x, int n, float *ours, float *ref);
-/* self-check of the TTM solver's binary64 reciprocal (a binary32 seed and
-   two Newton-Raphson steps): for n inputs, its results and 1.0 / x */
+/* self-check of the TTM solver's binary64 reciprocal (the hardware
+   approximation, about 2^-20, and two Newton-Raphson steps): for n inputs, its results and 1.0 / x */
 int fmdg_check_recip(fmdg_sys_t *s, const double *x, int n, double *ours, double *ref);
 /* write a buffer larger than L2 so the next kernel starts cold */
 int fmdg_flush_l2(fmdg_sys_t *s);
