@@ -264,6 +264,7 @@ struct LocOne
     static constexpr int lean_min_blocks = 7; // lean force kernels: 7 blocks of 128 (72 registers), measured best
     static constexpr bool one_lane = false;     // lanes by Geo::lane_log
     static constexpr bool split_shares = false; // every share has its lane
+    static constexpr bool free_loads = false;   // ld_step (fmdg_pairs.cuh)
     Geo g;
 };
 
@@ -276,6 +277,7 @@ struct LocPack
     static constexpr int lean_min_blocks = 0; // packed lean force kernels: compiler's choice, measured best
     static constexpr bool one_lane = true;      // one share, one lane per slot
     static constexpr bool split_shares = false;
+    static constexpr bool free_loads = true;
     int nsys;
     int bstart[FMDG_PACK_MAX + 1];
     Geo geos[FMDG_PACK_MAX];
@@ -287,6 +289,7 @@ struct LocPackShares : LocPack
     static constexpr int df_min_blocks = 0;     // (bounded: 300 small binary64 jobs 3.4e8 -> 3.0e8)
     static constexpr bool one_lane = false;
     static constexpr bool split_shares = true;  // a lane may walk several shares
+    static constexpr bool free_loads = false;
 };
 static_assert(sizeof(LocPack) <= 32704, "a packed launch's parameters exceed the 32 KB limit");
 

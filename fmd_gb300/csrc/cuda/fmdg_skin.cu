@@ -579,7 +579,8 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_nlist_skin(__
         if (i < dyn->n)
         {
             const Side S = g.side[dyn->cur];
-            const float4 xi = g.xf4[i];
+            const float4 *xf = after_wait<true>(g.xf4);
+            const float4 xi = xf[i];
             const float rl2 = g.rskin2;
             int4 *row = reinterpret_cast<int4 *>(g.nbr) + t;
             // Up to 32 candidates of a cell give a mask of hits first, then
@@ -599,7 +600,7 @@ __global__ void __launch_bounds__(L::max_threads, L::min_blocks) k_nlist_skin(__
             for_each_build_cell(g, so, cell_xyz(g, S.cell_of[i]), xi, [&](int code, int c, float ax, float ay, float az) {
                 const int jb = S.cell_start[c], je = S.cell_start[c + 1];
                 auto near = [&](int j) {
-                    const float4 xj = g.xf4[j];
+                    const float4 xj = ld_step<L::free_loads>(xf + j);
                     return norm2(make_float3(ax - xj.x, ay - xj.y, az - xj.z)) < rb2;
                 };
                 for (int j0 = jb; j0 < je; j0 += 32)
@@ -917,15 +918,15 @@ __global__ void __launch_bounds__(L::max_threads, MIXED ? L::min_blocks : L::df_
                 {
                     const int step = 4 * V;
                     const size_t cap = g.cap;
-                    const int4 *col = reinterpret_cast<const int4 *>(g.nbr) + t;
+                    const int4 *col = after_wait<L::free_loads>(reinterpret_cast<const int4 *>(g.nbr)) + t;
                     int k = 4 * v;
                     for (; k + 4 <= cnt; k += step)
                     {
                         if (k + step + 4 <= cnt)
                             asm volatile("prefetch.global.L1 [%0];" ::"l"(col + (size_t)((k + step) >> 2) * cap));
-                        round(col[(size_t)(k >> 2) * cap], 4, std::false_type{});
+                        round(ld_step<L::free_loads>(col + (size_t)(k >> 2) * cap), 4, std::false_type{});
                     }
-                    if (k < cnt) round(col[(size_t)(k >> 2) * cap], cnt - k, std::true_type{});
+                    if (k < cnt) round(ld_step<L::free_loads>(col + (size_t)(k >> 2) * cap), cnt - k, std::true_type{});
                 }
                 else
                     for_each_slot_overflow<L::one_system>(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
@@ -1268,15 +1269,15 @@ __global__ void __launch_bounds__(L::max_threads, !MIXED ? L::df_min_blocks : (L
                     {
                         constexpr bool PF = CAT != CAT_EAM;      // prefetch of the next list row
                         const int step = 4 * V;
-                        const int4 *col = reinterpret_cast<const int4 *>(g.nbr) + t;
+                        const int4 *col = after_wait<L::free_loads>(reinterpret_cast<const int4 *>(g.nbr)) + t;
                         int k = 4 * v;
                         for (; k + 4 <= cnt; k += step)
                         {
                             if (PF && k + step + 4 <= cnt)
                                 asm volatile("prefetch.global.L1 [%0];" ::"l"(col + (size_t)((k + step) >> 2) * cap));
-                            round(col[(size_t)(k >> 2) * cap], 4, std::false_type{});
+                            round(ld_step<L::free_loads>(col + (size_t)(k >> 2) * cap), 4, std::false_type{});
                         }
-                        if (k < cnt) round(col[(size_t)(k >> 2) * cap], cnt - k, std::true_type{});
+                        if (k < cnt) round(ld_step<L::free_loads>(col + (size_t)(k >> 2) * cap), cnt - k, std::true_type{});
                     }
                     else
                         for_each_slot_overflow<L::one_system>(g, S, so, t, i, v, V, xi, [&](int js, float4 xj, float4 o) {
